@@ -101,16 +101,11 @@ int pf_ctx_set_stream(pf_ctx *ctx, void *cuda_stream);
  * bit; only the speed differs.  The autotuner (pipeflow.tune) sets them by
  * timing the candidates per pipe shape.  A zero struct is the built-in
  * choice.  Setting them drops the context's captured step graphs. */
-#define PF_LD_AUTO     0  /* the built-in choice (streamed factors) */
-#define PF_LD_STREAMED 1  /* Helmholtz factors streamed from HBM */
-#define PF_LD_REBUILT  2  /* Helmholtz factors rebuilt on chip (factorisations
-                             that did not pivot, N >= 10; else streamed) */
-#define PF_LD_PAIRED   3  /* streamed factors, modes k and -k paired on one
-                             factor stream (pressure and Helmholtz solves) */
-#define PF_LD_WARPRING 4  /* streamed Helmholtz factors, one shared-memory ring
-                             per mode read by its real and imaginary lanes (the
-                             pressure solve does so for every choice but
-                             PF_LD_PAIRED) */
+#define PF_LD_AUTO     0  /* the Helmholtz and pressure solves have one form, */
+#define PF_LD_STREAMED 1  /* inside the one-launch vel_step: every ld_solver  */
+#define PF_LD_REBUILT  2  /* value is accepted and runs it                    */
+#define PF_LD_PAIRED   3
+#define PF_LD_WARPRING 4
 typedef struct {
     int ld_solver; /* PF_LD_* */
     int nl_mc;     /* z-pass columns per block (1..M; 0 = built-in) */
@@ -503,14 +498,13 @@ int pf_serve_batch(pf_server *s, pf_batch **b);
 #define PF_K_THINV    1   /* theta pass (c2r) -> physical                   */
 #define PF_K_THFWD    2   /* theta pass (r2c), fused u x curl(u)            */
 #define PF_K_ZFWD     3   /* z pass -> spectral, truncation                 */
-#define PF_K_LUSOLVE  4   /* banded solves (the Helmholtz u+, u-, uz ones in
-                             the fused step)                                 */
+#define PF_K_LUSOLVE  4   /* banded solves outside the fused step            */
 #define PF_K_STENCIL  5   /* meshmult / curl / grad / div / tim_meshmult    */
 #define PF_K_EW       6   /* elementwise, symmetry, reductions, transfers   */
 #define PF_K_INFL     7   /* influence correction, flux, addHPF             */
 #define PF_K_FACTOR   8   /* banded LU factorisation (vel_matrices)          */
-#define PF_K_STEP     9   /* fused per-mode step kernels                     */
-#define PF_K_PPE     10   /* pressure-Poisson banded solve of the fused step */
+#define PF_K_STEP     9   /* the fused vel_step, its solves included         */
+#define PF_K_PPE     10   /* unused (the pressure solve is part of the step) */
 #define PF_K_NCAT    11
 /* Count of this library's kernel launches on the context since creation. */
 int pf_ctx_launches(const pf_ctx *ctx, unsigned long long *n);

@@ -77,6 +77,7 @@ struct pf_batch {
     bool fresh;                      // built, no step run yet (the first runs uncaptured)
     pf_nl_batch *nlb;
     pf_step_batch *stb;
+    pf_aux aux;                      // streams of the step's concurrent launches
     int par0;                        // pipe 0's pointer parity when nlb/stb were built
     SymArgs *d_sym[2];               // [pointer state]
     DevScalars **d_scp;              // each pipe's device scalars
@@ -136,6 +137,7 @@ static void batch_graphs_reset(pf_batch *b) {
 static void batch_free(pf_batch *b) {
     batch_graphs_reset(b);
     batch_io_free(b);
+    b->aux.free();
     for (cudaEvent_t e : b->join) cudaEventDestroy(e);
     if (b->fork) cudaEventDestroy(b->fork);
     if (b->master) cudaStreamDestroy(b->master);
@@ -309,7 +311,7 @@ static bool batch_stageable(const pf_batch *b) {
 static int staged_build(pf_batch *b) {
     staged_free(b);
     PF_TRY(pf_nl_batch_build(b->pipes.data(), b->n, b->worklist, &b->nlb));
-    PF_TRY(pf_step_batch_build(b->pipes.data(), b->n, &b->stb));
+    PF_TRY(pf_step_batch_build(b->pipes.data(), b->n, &b->aux, &b->stb));
     std::vector<SymArgs> sym(b->n);
     std::vector<DevScalars *> scp(b->n);
     for (int s = 0; s < 2; ++s) {
@@ -470,6 +472,7 @@ static long long batch_after_step(pf_batch *b, int orbit, int *status) {
     for (int i = 0; i < b->n; ++i) {
         pf_ctx *c = b->pipes[i];
         const double err2 = bits_to_double(b->hsc[i].dterr2_bits);
+        if (pf_step_status(b->hsc[i]) != PF_OK) *status = PF_ERR_CUDA;
         c->tim.dterr = std::max(c->tim.dterr, std::sqrt(err2));
         c->tim.it = 1;
         c->last_status = PF_OK;

@@ -69,14 +69,25 @@ __host__ __device__ inline void mode_km(int nh, int K, int &k, int &m) {
     }
 }
 
-// Compact index of the modes with k >= 0 (c = m*K + |k|, M*K of them), the
-// layout of the factor copies the streamed solves read, and its padded size.
-__host__ __device__ inline int mode_compact(int nh, int K) {
-    int k = 0, m = 0;
-    mode_km(nh, K, k, m);
-    return m * K + (k < 0 ? -k : k);
-}
-inline int pf_compact_modes_padded(const Geo &g) { return (g.M * g.K + 31) / 32 * 32; }
+// Factor tiles of the fused step.  A block of it takes 16 modes: k and -k of
+// 8 consecutive (m, k >= 0) with m >= 1, whose matrices are bitwise equal (k
+// enters as alpha*k*alpha*k only, timestep.f90:76), or 16 consecutive k of
+// m = 0.  A factor set is stored in that order, the m = 0 tiles first, with
+// W = 8 distinct matrices per paired tile and 16 per m = 0 tile.  A tile holds
+// what the forward sweep reads, [col][FR][W] (L(1..KL) of each column, then
+// its pivot offset as a bit pattern if any matrix of the set pivots), then
+// what the back substitution reads, [col descending][BR][W] (1/U(0) as the
+// sum of two doubles, then U(1..KU)): each sweep is one contiguous stream.
+// FT_ROWS rows a column are kept, the pivoting form.
+constexpr int FT_ROWS = 3 * PF_KL + 3;
+__host__ __device__ constexpr int ft_fwd_rows(bool piv) { return PF_KL + (piv ? 1 : 0); }
+__host__ __device__ constexpr int ft_back_rows(bool piv) { return (piv ? 2 : 1) * PF_KL + 2; }
+__host__ __device__ inline int pf_mean_tiles(const Geo &g) { return (g.K + 15) / 16; }
+__host__ __device__ inline int pf_paired_tiles(const Geo &g) { return ((g.M - 1) * g.K + 7) / 8; }
+__host__ __device__ inline int pf_step_tiles(const Geo &g) { return pf_mean_tiles(g) + pf_paired_tiles(g); }
+// matrices of a set's tiles, padding included, and doubles of its storage
+inline size_t pf_tile_modes(const Geo &g) { return (size_t)16 * pf_mean_tiles(g) + (size_t)8 * pf_paired_tiles(g); }
+inline size_t pf_tile_elems(const Geo &g) { return pf_tile_modes(g) * g.N * FT_ROWS; }
 
 // Radial mesh on the device (meshs.f90:48-55).
 struct DevMesh {
@@ -128,8 +139,18 @@ struct DevScalars {
     double flux_d1;                  // vel_adjustFlux d1
     unsigned long long dterr2_bits;  // max |corr|^2 as ordered bits
     int info;                        // first singular pivot (1-based col), 0 = ok
-    int pad;
+    int tiles_done;                  // fused corrector: blocks that have added to dterr2_acc
+    unsigned long long dterr2_acc;   // their maximum so far (0 between launches)
 };
+
+// DevScalars::info of a fused step whose factor copies never arrived
+#define PF_STEP_STUCK (-1000000)
+
+inline int pf_step_status(const DevScalars &s) {
+    if (s.info != PF_STEP_STUCK) return PF_OK;
+    pf_set_error("fused step: a factor copy into shared memory did not complete");
+    return PF_ERR_CUDA;
+}
 
 // Mixed-radix FFT plan of length L: radices in application order.
 struct FFTPlan {
@@ -156,18 +177,11 @@ struct pf_mesh {
 struct pf_lumesh {
     pf_ctx *ctx;
     int PM, BC;
-    int pivoted;         // host copy: any row interchange in the factorisation
-    double *pivd;        // pivot offsets as doubles [col*Hp + nh] (context sets only)
+    int pivoted;         // host copy: bit 0 any row interchange, bit 1 U wider than KL columns
     double c1, c2;
     double *lu;
     unsigned char *piv;
-    // context sets only: the factors and pivots (as doubles) of the modes
-    // with k >= 0, [(row*N + col)*Hcp + c] and [col*Hcp + c] with
-    // c = m*K + |k|.  The matrix of mode (-k, m) is bitwise that of (k, m)
-    // (k enters as alpha*k*alpha*k only, timestep.f90:76), so its factors are
-    // too; the streamed solves read this copy and fetch half the factor bytes.
-    double *luc;
-    double *pivdc;
+    double *tiles;       // context sets of fused-step sizes: the factor tiles (above)
 };
 
 struct pf_ctx {
@@ -414,8 +428,38 @@ bool pf_nl_batch_supported(pf_ctx *const *pipes, int n);
 int pf_nl_batch_build(pf_ctx *const *pipes, int n, bool worklist, pf_nl_batch **out);
 int pf_nl_batch_launch(pf_nl_batch *b, int state, cudaStream_t st, pf_stage_prof *prof, unsigned long long *nk);
 void pf_nl_batch_free(pf_nl_batch *b);
+// Streams onto which a batch forks the concurrent launches of a stage, and
+// their events; they live with the batch, whose launches are rebuilt at every
+// change of membership.
+struct pf_aux {
+    std::vector<cudaStream_t> st;
+    std::vector<cudaEvent_t> join;
+    cudaEvent_t fork = nullptr;
+    int reserve(size_t n) {
+        if (!fork) PF_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+        while (st.size() < n) {
+            cudaStream_t s = nullptr;
+            PF_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+            st.push_back(s);
+        }
+        while (join.size() < n) {
+            cudaEvent_t e = nullptr;
+            PF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+            join.push_back(e);
+        }
+        return PF_OK;
+    }
+    void free() {
+        for (cudaStream_t s : st) cudaStreamDestroy(s);
+        for (cudaEvent_t e : join) cudaEventDestroy(e);
+        if (fork) cudaEventDestroy(fork);
+        st.clear();
+        join.clear();
+        fork = nullptr;
+    }
+};
 struct pf_step_batch;
-int pf_step_batch_build(pf_ctx *const *pipes, int n, pf_step_batch **out);
+int pf_step_batch_build(pf_ctx *const *pipes, int n, pf_aux *aux, pf_step_batch **out);
 int pf_step_batch_launch(pf_step_batch *b, int state, int corrector, cudaStream_t st, pf_stage_prof *prof,
                          unsigned long long *nk);
 void pf_step_batch_free(pf_step_batch *b);

@@ -49,6 +49,7 @@ __global__ void k_lu_factor(double *__restrict__ lu, unsigned char *__restrict__
         if (jp != 0) atomicOr(anypiv, 1);
         if (LU(KV + jp, j) != 0.0) {
             ju = max(ju, min(j + KL + jp, N - 1));
+            if (jp != 0 && ju > j + KL) atomicOr(anypiv, 2);  // row j of U reaches beyond KL columns
             if (jp != 0)
                 for (int c = j; c <= ju; ++c) {
                     const double t = LU(KV + jp - (c - j), c);
@@ -355,29 +356,31 @@ int pf_launch_flux1(pf_ctx *ctx) {
 }
 
 // ---------------------------------------------------------- vel_matrices
-__global__ void k_piv_to_double(const unsigned char *__restrict__ piv, double *__restrict__ pivd, size_t n) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        pivd[i] = (double)piv[i];
-}
-
-// The compact copy of a factor set: the band and pivots of the modes with
-// k >= 0 only, at c = m*K + k (padding columns zero).
-__global__ void k_lu_compact(const double *__restrict__ lu, const double *__restrict__ pivd, double *__restrict__ luc,
-                             double *__restrict__ pivdc, int N, int Hp, int Hcp, int K, int M) {
-    const size_t rows = (size_t)NLU * N + N;  // band entries, then the pivot row of each column
-    const size_t total = rows * Hcp;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t r = i / Hcp;
-        const int c = (int)(i - r * Hcp);
-        double v = 0.0;
-        if (c < M * K) {
-            const int m = c / K, k = c - m * K;
-            const int nh = m == 0 ? k : m * (2 * K - 1) + k;
-            v = r < (size_t)NLU * N ? lu[r * Hp + nh] : pivd[(r - (size_t)NLU * N) * Hp + nh];
-        }
-        if (r < (size_t)NLU * N) luc[r * Hcp + c] = v;
-        else pivdc[(r - (size_t)NLU * N) * Hcp + c] = v;
-    }
+// The factor tiles of a set (pf_internal.cuh): thread per (tile matrix,
+// column), 8 consecutive matrices of a tile on consecutive threads.  A matrix
+// that is not factored (BC=1 at k=m=0) and padding are zeros, which solve to 0.
+template <bool PIV, bool WIDE>
+__global__ void k_lu_tiles(const double *__restrict__ lu, const unsigned char *__restrict__ piv,
+                           double *__restrict__ tiles, Geo g, int BC) {
+    constexpr int FR = ft_fwd_rows(PIV), BR = ft_back_rows(WIDE);
+    const int N = g.N, Hp = g.Hp, nz = 16 * pf_mean_tiles(g), nt = nz + 8 * pf_paired_tiles(g);
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (long long)nt * N) return;
+    const int e = (int)(t % 8), j = (int)(t / 8 % N), c = (int)(t / 8 / N) * 8 + e;
+    const int W = c < nz ? 16 : 8;
+    const int m = c < nz ? 0 : 1 + (c - nz) / g.K, k = c < nz ? c : (c - nz) % g.K;
+    const bool live = (c < nz ? k < g.K : m < g.M) && !(BC == 1 && c == 0);
+    const int nh = m * (2 * g.K - 1) + k;
+    double *o = tiles + (size_t)(c / W * W) * N * FT_ROWS + c % W;
+    double *f = o + (size_t)j * FR * W, *b = o + ((size_t)N * FR + (size_t)(N - 1 - j) * BR) * W;
+#pragma unroll
+    for (int r = 1; r <= KL; ++r) f[(r - 1) * W] = live && j + r < N ? LU(KV + r, j) : 0.0;
+    if (PIV) f[KL * W] = __hiloint2double(0, live && j < N - 1 ? piv[(size_t)j * Hp + nh] : 0);
+    const double u = live ? LU(KV, j) : 0.0, hi = live ? 1.0 / u : 0.0;
+    b[0] = hi;
+    b[W] = fma(-u, hi, 1.0) * hi;
+#pragma unroll
+    for (int r = 1; r <= BR - 2; ++r) b[(r + 1) * W] = live && j - r >= 0 ? LU(KV - r, j) : 0.0;
 }
 
 static int lumesh_init(pf_ctx *ctx, pf_lumesh *A, int PM, int BC, double c1, double c2) {
@@ -386,24 +389,16 @@ static int lumesh_init(pf_ctx *ctx, pf_lumesh *A, int PM, int BC, double c1, dou
     A->c1 = c1;
     A->c2 = c2;
     PF_TRY(pf_launch_lu_factor(ctx, A));
-    if (A->pivd) {  // pivots as doubles, staged by the fused solves with 8-byte copies
-        const Geo &g = ctx->g;
-        const size_t np = (size_t)g.N * g.Hp;
+    if (A->tiles) {
         {
             ProfScope ps_(ctx, PF_K_FACTOR);
-            k_piv_to_double<<<grid1(np, 256), 256, 0, ctx->stream>>>(A->piv, A->pivd, np);
+            const unsigned grid = grid1((long long)pf_tile_modes(ctx->g) * ctx->g.N, 128);
+            const auto k = BC == 1 || A->pivoted > 1 ? k_lu_tiles<true, true>  // the pressure set always in the full form
+                           : A->pivoted ? k_lu_tiles<true, false>
+                                        : k_lu_tiles<false, false>;
+            k<<<grid, 128, 0, ctx->stream>>>(A->lu, A->piv, A->tiles, ctx->g, BC);
         }
         PF_LAUNCHED(ctx);
-        if (A->luc) {
-            const int Hcp = pf_compact_modes_padded(g);
-            const size_t nc = ((size_t)NLU * g.N + g.N) * Hcp;
-            {
-                ProfScope ps_(ctx, PF_K_FACTOR);
-                k_lu_compact<<<grid1(nc, 256), 256, 0, ctx->stream>>>(A->lu, A->pivd, A->luc, A->pivdc, g.N, g.Hp, Hcp,
-                                                                      g.K, g.M);
-            }
-            PF_LAUNCHED(ctx);
-        }
     }
     return PF_OK;
 }

@@ -1,48 +1,32 @@
-// Fused vel_step (velocity.f90:367-394) in five launches:
-//   S1 k_step_rhs  : tile of 16 modes x all radial points: optional
-//                    nlincorr (timestep.f90:174-184) or N_ := N copy,
-//                    rhs = Lt u_ + N in the u+-/uz variables (velocity.f90:369-373,
-//                    tim_meshmult with the per-mode band rebuilt in registers),
-//                    then the PPE right-hand side div(pm2rt(rhs)) with zero
-//                    boundary rows (velocity.f90:228-230)
-//   S2 k_solve_pnpw: pressure Poisson solve with LNp (pivoting band LU,
-//                    BC=1, mean mode zeroed; timestep.f90:102-123), the
-//                    factor ring of a mode shared by its re and im lanes
-//   S3 k_step_proj : the projection rhs - rt2pm(grad p) with zero boundary
-//                    rows (velocity.f90:232-236, 376-378)
-//   S4 k_solve_ld  : the u+, u-, uz Helmholtz solves (LDp, LDm, LDz; the
-//                    pivot-free sweep unless that factorisation pivoted)
-//   S5 k_step_final: influence-matrix correction (velocity.f90:238-256),
-//                    pm2rt, constant-flux adjustment for k=m=0
-//                    (velocity.f90:170-175), mean-mode symmetry zeros, and the
-//                    corrector error max |u_old - u_new|^2 (timestep.f90:190-207)
-// Scratch: v (3 coll) holds rhs then the solutions, prhs/p the pressure
-// right-hand side and solution, rl (3 coll) the Helmholtz right-hand sides.
+// Fused vel_step (velocity.f90:367-394): one launch per predictor or corrector.
+//
+// Every stage of the step is independent between Fourier modes, so a block
+// takes a tile of 16 modes through all of them with the tile's fields in
+// shared memory:
+//   rhs    : optional nlincorr (timestep.f90:174-184) or N_ := N copy, rhs =
+//            Lt u_ + N in the u+-/uz variables (velocity.f90:369-373)
+//   div    : PPE right-hand side div(pm2rt(rhs)), zero boundary rows
+//            (velocity.f90:228-230)
+//   PPE    : pressure Poisson solve with LNp (timestep.f90:102-123)
+//   proj   : rhs - rt2pm(grad p), zero boundary rows (velocity.f90:232-236)
+//   solves : the u+, u-, uz Helmholtz systems (LDp, LDm, LDz)
+//   final  : influence-matrix correction (velocity.f90:238-256), pm2rt,
+//            constant-flux adjustment of k=m=0 (velocity.f90:170-175),
+//            mean-mode symmetry zeros, and the corrector error
+//            max |u_old - u_new|^2 (timestep.f90:190-207)
+// From HBM it reads u_, N (and N_, the old u in the corrector), the factors
+// and the influence vectors, and writes N (or N_) and u: no stage's result
+// leaves the SM.
 #include <cmath>
 #include "pf_internal.cuh"
-
-static constexpr int TM = 32;  // modes per tile
-static constexpr int TR = 8;   // radial row groups per tile
 
 struct StepArgs {
     const double2 *u_[3];  // previous state (ur_, ut_, uz_)
     double2 *Nl[3];        // vel_N (read; rewritten by nlincorr)
     double2 *N_[3];        // saved N_ (read in the corrector, written in the predictor)
-    double2 *v[3];         // scratch: rhs / solutions in u+, u-, uz
-    double2 *prhs;         // scratch: pressure right-hand side
-    double2 *p;            // scratch: pressure
-    double2 *rl[3];        // scratch: Helmholtz right-hand sides
     double2 *u[3];         // vel_u (read as u_old by the corrector, written)
-    const double *lnp, *ldp, *ldm, *ldz;
-    const double *pivd;    // LNp pivots as doubles [col*Hp + nh]
-    const double *pivld[3];  // LDp/LDm/LDz pivots as doubles
+    const double *lnp, *ld[3];  // factor tiles of LNp, LDp, LDm, LDz
     int ldpiv[3];          // 1 if that Helmholtz factorisation pivoted
-    // compact copies (modes k >= 0, c = m*K + |k|, stride Hcp) the streamed
-    // pressure and Helmholtz solves read: LNp, LDp, LDm, LDz and their pivots
-    const double *lnpc, *ldc[3];
-    const double *pivdc, *pivldc[3];
-    int Hcp;
-    double ldc1, ldc2;     // Helmholtz coefficients (LDp/LDm/LDz: 1/dt, -implicit nu/Re)
     const double *U, *Ainv, *Ui;
     DevMesh dm;
     Geo g;
@@ -53,1279 +37,655 @@ struct StepArgs {
     DevScalars *sc;
 };
 
-__device__ __forceinline__ double lap_diag(const DevMesh &dm, const Geo &g, int PM, int n, int k, int m) {
-    const double r2 = dm.rp[1 * g.N + n];
-    double d = -(r2 * g.Mp * m * g.Mp * m) - g.alpha * k * g.alpha * k;
-    if (PM != 0) d = d - r2 - 2.0 * PM * g.Mp * m * r2;
-    return d;
-}
-
-// ------------------------------------------------------------------- S1
-// Block = 16 modes x 16 radial row groups; each thread owns RPT rows
-// n = ty + 16 r (RPT = 4 for N <= 64, 8 for N <= 128), so the values it
-// keeps between the two phases stay in registers.  Pointers are held as
-// __restrict__ locals so loads of later rows can be issued before the stores
-// of earlier ones.
-static constexpr int HM = 16;  // modes per S1 block
-static constexpr int HR = 16;  // row groups per S1 block
-
-template <int RPT>
-__device__ __forceinline__ void step_rhs_body(const StepArgs &a, int hb) {
-    extern __shared__ double2 rsm[];  // [N][HM]: radial component of pm2rt(rhs)
-    const Geo &g = a.g;
-    const int N = g.N;
-    const size_t Hp = g.Hp;
-    const int tx = threadIdx.x % HM, ty = threadIdx.x / HM;
-    const int nh = hb * HM + tx;
-    // the corrector's error max (timestep.f90:190-207) restarts here; S5
-    // accumulates it after every block of this launch has finished
-    if (a.mode == 1 && hb == 0 && threadIdx.x == 0) a.sc->dterr2_bits = 0ull;
-    const bool live = nh < g.H;
-    const int nhc = live ? nh : 0;
-    int k = 0, m = 0;
-    if (live) mode_km(nh, g.K, k, m);
-    const double c1 = a.c1, c2 = a.c2;
-    const double2 *__restrict__ ur_ = a.u_[0] + nhc;
-    const double2 *__restrict__ ut_ = a.u_[1] + nhc;
-    const double2 *__restrict__ uz_ = a.u_[2] + nhc;
-    double2 *__restrict__ N0 = a.Nl[0] + nhc;
-    double2 *__restrict__ N1 = a.Nl[1] + nhc;
-    double2 *__restrict__ N2 = a.Nl[2] + nhc;
-    double2 *__restrict__ P0 = a.N_[0] + nhc;
-    double2 *__restrict__ P1 = a.N_[1] + nhc;
-    double2 *__restrict__ P2 = a.N_[2] + nhc;
-    double2 *__restrict__ v0 = a.v[0] + nhc;
-    double2 *__restrict__ v1 = a.v[1] + nhc;
-    double2 *__restrict__ v2 = a.v[2] + nhc;
-    double2 *__restrict__ prhs = a.prhs + nhc;
-    const double *__restrict__ radLap = a.dm.radLap;
-    const double *__restrict__ drb = a.dm.dr;
-    const double *__restrict__ rp = a.dm.rp;
-    double2 tkeep[RPT], zkeep[RPT];
-#pragma unroll
-    for (int r = 0; r < RPT; ++r) {
-        const int n = ty + HR * r;
-        double2 vp = make_double2(0, 0), vm = vp, vz = vp;
-        if (live && n < N) {
-            const size_t at = (size_t)n * Hp;
-            // read once (and in the corrector overwritten): stream past L1
-            double2 Nr = __ldcs(N0 + at), Nt = __ldcs(N1 + at), Nz = __ldcs(N2 + at);
-            if (a.mode == 1) {  // N = c N + (1-c) N_
-                const double d1 = a.implicit, d2 = 1.0 - a.implicit;
-                const double2 Pr = __ldcs(P0 + at), Pt = __ldcs(P1 + at), Pz = __ldcs(P2 + at);
-                Nr = make_double2(d1 * Nr.x + d2 * Pr.x, d1 * Nr.y + d2 * Pr.y);
-                Nt = make_double2(d1 * Nt.x + d2 * Pt.x, d1 * Nt.y + d2 * Pt.y);
-                Nz = make_double2(d1 * Nz.x + d2 * Pz.x, d1 * Nz.y + d2 * Pz.y);
-                N0[at] = Nr;
-                N1[at] = Nt;
-                N2[at] = Nz;
-            } else {  // N_ := N
-                P0[at] = Nr;
-                P1[at] = Nt;
-                P2[at] = Nz;
-            }
-            // rhs = Lt u_ + N, accumulated from N in increasing column order
-            vp = make_double2(Nr.x - Nt.y, Nr.y + Nt.x);
-            vm = make_double2(Nr.x + Nt.y, Nr.y - Nt.x);
-            vz = Nz;
-            const int lo = max(0, n - KL), hi = min(N - 1, n + KL);
-            for (int j = lo; j <= hi; ++j) {
-                const size_t aj = (size_t)j * Hp;
-                const double2 rr = ur_[aj], t = ut_[aj], z = uz_[aj];
-                const double off = c2 * radLap[(KL + n - j) * N + j];
-                double wp = off, wm = off, wz = off;
-                if (j == n) {
-                    wp = (off + c2 * lap_diag(a.dm, g, 1, j, k, m)) + c1;
-                    wm = (off + c2 * lap_diag(a.dm, g, -1, j, k, m)) + c1;
-                    wz = (off + c2 * lap_diag(a.dm, g, 0, j, k, m)) + c1;
-                }
-                vp.x = fma(wp, rr.x - t.y, vp.x);
-                vp.y = fma(wp, rr.y + t.x, vp.y);
-                vm.x = fma(wm, rr.x + t.y, vm.x);
-                vm.y = fma(wm, rr.y - t.x, vm.y);
-                vz.x = fma(wz, z.x, vz.x);
-                vz.y = fma(wz, z.y, vz.y);
-            }
-            v0[at] = vp;
-            v1[at] = vm;
-            v2[at] = vz;
-        }
-        // pm2rt (velocity.f90:98-114)
-        if (n < N) rsm[n * HM + tx] = make_double2(0.5 * (vp.x + vm.x), 0.5 * (vp.y + vm.y));
-        tkeep[r] = make_double2(0.5 * (vp.y - vm.y), -0.5 * (vp.x - vm.x));
-        zkeep[r] = vz;
-    }
-    __syncthreads();
-    if (!live) return;
-    const double kal = g.alpha * k;
-#pragma unroll
-    for (int r = 0; r < RPT; ++r) {
-        const int n = ty + HR * r;
-        if (n >= N) break;
-        double2 dv = make_double2(0, 0);
-        if (n != 0 && n != N - 1) {  // tim_zerobc
-            const double rm1 = rp[2 * N + n];
-            const double m1r1 = rm1 * g.Mp * m;
-            double2 dr = make_double2(0, 0);
-            const int lo = max(0, n - KL), hi = min(N - 1, n + KL);
-            for (int j = lo; j <= hi; ++j) {
-                const double w = drb[(KL + n - j) * N + j];
-                const double2 x = rsm[j * HM + tx];
-                dr.x = fma(w, x.x, dr.x);
-                dr.y = fma(w, x.y, dr.y);
-            }
-            const double2 rr = rsm[n * HM + tx], t = tkeep[r], z = zkeep[r];
-            dv.x = rr.x * rm1 + dr.x - t.y * m1r1 - z.y * kal;  // variables.f90:472-477
-            dv.y = rr.y * rm1 + dr.y + t.x * m1r1 + z.x * kal;
-        }
-        prhs[(size_t)n * Hp] = dv;
-    }
-}
-
-// --------------------------------------------------- banded solves (S2, S4)
-// One thread per (mode, system, re/im) chain.  The factor values of a
-// column and the right-hand side entering the elimination window are staged
-// D columns ahead into a per-thread shared-memory ring with cp.async (8-byte
-// copies, one commit group per column), so each step of the sequential
-// sweep reads shared memory instead of waiting on DRAM.  The ring is laid out
-// [slot][value][thread] so consecutive threads hit consecutive banks.  Six
-// columns ahead, with the register budgets the launch bounds below set (four
-// Helmholtz blocks and eight pressure blocks per SM), measured fastest: deeper
-// rings or register queues cost more in resident warps than they hide.
-static constexpr int RING = 6;
-
-__device__ __forceinline__ void cp_async8(double *smem, const double *gmem) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
-__device__ __forceinline__ void cp_async8s(unsigned saddr, const double *gmem) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(saddr), "l"(gmem) : "memory");
-}
-
-// dgbtrs ('N', one right-hand side) followed by dtbsv: rhs(n) = rhs[n*rs],
-// solution to out[n*os] (out must not alias rhs).  PIV: LAPACK band with
-// KL+KU superdiagonals in U and pivots pivd[col*Hp+nh] (as doubles); else
-// the pivot-free band with KU = KL.  The ring is strided by the block's TS
-// threads; the column loop is unrolled by RING so every ring slot is a
-// constant shared-memory offset, and the global addresses step by one
-// column per iteration instead of being recomputed.
-template <bool PIV, int TS>
-__device__ __forceinline__ void solve_async(const double *__restrict__ lu, const double *__restrict__ pivd, int N,
-                                            int Hp, int nh, const double *__restrict__ rhs, size_t rs, double *out,
-                                            size_t os, double *ring) {
-    constexpr int KU = PIV ? KV : KL;
-    constexpr int SWF = KL + 1 + (PIV ? 1 : 0);  // forward slot: L column, rhs ahead, pivot
-    constexpr int SWB = KU + 1;                  // backward slot: U column
-    constexpr int SW = SWF > SWB ? SWF : SWB;
-    constexpr unsigned QB = 8u * TS, SB = 8u * TS * SW;  // bytes between values / slots
-    const size_t rowst = (size_t)N * Hp;                 // doubles between band rows
-    const unsigned sbase = (unsigned)__cvta_generic_to_shared(ring);
-#define RSLOT(s, q) ring[((s) * SW + (q)) * TS]
-    // forward: column j needs L(KV+1+i, j), i < KL, rhs(j+KL+1) and its pivot
-    const double *Lj = lu + (size_t)(KV + 1) * rowst + nh;
-    const double *Pj = PIV ? pivd + nh : nullptr;
-    const double *Rj = rhs + (size_t)(KL + 1) * rs;
-    int jj = 0;  // next column to stage
-    auto issue_fwd = [&](int s) {
-        if (jj < N) {
-            if (jj < N - 1) {
-#pragma unroll
-                for (int i = 0; i < KL; ++i) cp_async8s(sbase + s * SB + i * QB, Lj + i * rowst);
-                if (PIV) cp_async8s(sbase + s * SB + (KL + 1) * QB, Pj);
-            }
-            if (jj + KL + 1 < N) cp_async8s(sbase + s * SB + KL * QB, Rj);
-        }
-        cp_async_commit();
-        ++jj;
-        Lj += Hp;
-        if (PIV) Pj += Hp;
-        Rj += rs;
-    };
-    double w[KL + 1];
-#pragma unroll
-    for (int i = 0; i <= KL; ++i) w[i] = (i < N) ? rhs[(size_t)i * rs] : 0.0;
-#pragma unroll
-    for (int s = 0; s < RING; ++s) issue_fwd(s);
-    double *Oj = out;
-    for (int j0 = 0; j0 < N; j0 += RING) {
-#pragma unroll
-        for (int s = 0; s < RING; ++s) {
-            const int j = j0 + s;
-            if (j < N) {
-                cp_async_wait<RING - 1>();
-                const double ahead = (j + KL + 1 < N) ? RSLOT(s, KL) : 0.0;
-                if (j < N - 1) {
-                    if (PIV) {
-                        const int p = (int)RSLOT(s, KL + 1);
-#pragma unroll
-                        for (int i = 1; i <= KL; ++i)
-                            if (p == i) {
-                                const double t = w[0];
-                                w[0] = w[i];
-                                w[i] = t;
-                            }
-                    }
-                    const double bj = w[0];
-#pragma unroll
-                    for (int i = 1; i <= KL; ++i)
-                        if (j + i < N) w[i] = fma(-RSLOT(s, i - 1), bj, w[i]);
-                }
-                *Oj = w[0];
-                Oj += os;
-#pragma unroll
-                for (int i = 0; i < KL; ++i) w[i] = w[i + 1];
-                w[KL] = ahead;
-                issue_fwd(s);
-            }
-        }
-    }
-    cp_async_wait<0>();
-    // back substitution: column j needs U(KV-i, j), i <= KU; y (this thread's
-    // forward output) is read through a four-deep register queue, with
-    // streaming loads: each value is read once and then overwritten
-    const double *Uj = lu + (size_t)KV * rowst + (size_t)(N - 1) * Hp + nh;
-    int tt = 0;  // next step to stage (step t handles column N-1-t)
-    auto issue_bwd = [&](int s) {
-        if (tt < N) {
-#pragma unroll
-            for (int i = 0; i <= KU; ++i) cp_async8s(sbase + s * SB + i * QB, Uj - i * rowst);
-        }
-        cp_async_commit();
-        ++tt;
-        Uj -= Hp;
-    };
-#pragma unroll
-    for (int s = 0; s < RING; ++s) issue_bwd(s);
-    double v[KU + 1];
-#pragma unroll
-    for (int i = 0; i <= KU; ++i) v[i] = (N - 1 - i >= 0) ? __ldcs(out + (size_t)(N - 1 - i) * os) : 0.0;
-    constexpr int QY = 4;
-    double yq[QY];
-#pragma unroll
-    for (int q = 0; q < QY; ++q) {
-        const int r = N - 1 - KU - 1 - q;
-        yq[q] = (r >= 0) ? __ldcs(out + (size_t)r * os) : 0.0;
-    }
-    double *Xj = out + (size_t)(N - 1) * os;
-    for (int t0 = 0; t0 < N; t0 += RING) {
-#pragma unroll
-        for (int s = 0; s < RING; ++s) {
-            const int t = t0 + s;
-            if (t < N) {
-                const int j = N - 1 - t;
-                cp_async_wait<RING - 1>();
-                const double ahead = yq[0];
-#pragma unroll
-                for (int q = 0; q < QY - 1; ++q) yq[q] = yq[q + 1];
-                {
-                    const int r = j - KU - 1 - QY;
-                    yq[QY - 1] = (r >= 0) ? __ldcs(out + (size_t)r * os) : 0.0;
-                }
-                double x = v[0];
-                if (x != 0.0) {
-                    x = x / RSLOT(s, 0);
-#pragma unroll
-                    for (int i = 1; i <= KU; ++i)
-                        if (j - i >= 0) v[i] = fma(-x, RSLOT(s, i), v[i]);
-                }
-                *Xj = x;
-                Xj -= os;
-#pragma unroll
-                for (int i = 0; i < KU; ++i) v[i] = v[i + 1];
-                v[KU] = (j - KU - 1 >= 0) ? ahead : 0.0;
-                issue_bwd(s);
-            }
-        }
-    }
-    cp_async_wait<0>();
-#undef RSLOT
-}
-
-// The same solve with the factor ring of a mode shared by its real and
-// imaginary chains, which sit in one warp: lanes 0-15 are the real parts of
-// 16 modes, lanes 16-31 their imaginary parts.  Each factor value of a
-// column is copied once (the two lanes of a mode split the values), both
-// read it from shared memory after a __syncwarp; each lane stages its own
-// right-hand-side value.  A slot is refilled only after the next
-// __syncwarp, once both lanes have read it, so RING-1 columns are in
-// flight.  Every arithmetic operation is solve_async's, so the solutions are
-// bitwise the same.  `mask` holds the lanes that run (a mode's two lanes are
-// both in it or both out); all of them take the same number of steps.
-// Warp ring: RING slots of [FV values][16 modes] + [32 lanes] doubles.
-template <bool PIV> __host__ __device__ constexpr int rw_fv() {
-    return (KL + (PIV ? 1 : 0)) > ((PIV ? KV : KL) + 1) ? (KL + (PIV ? 1 : 0)) : ((PIV ? KV : KL) + 1);
-}
-template <bool PIV> __host__ __device__ constexpr int rw_slot() { return rw_fv<PIV>() * 16 + 32; }
-
-template <bool PIV>
-__device__ __forceinline__ void solve_async_rw(const double *__restrict__ lu, const double *__restrict__ pivd, int N,
-                                               int Hp, int nh, const double *__restrict__ rhs, size_t rs, double *out,
-                                               size_t os, double *wring, unsigned mask) {
-    constexpr int KU = PIV ? KV : KL;
-    constexpr int FQ = KL + (PIV ? 1 : 0);  // forward values: L(KV+1+i, j), i < KL, then the pivot
-    constexpr int BQ = KU + 1;              // backward values: U(KV-i, j), i <= KU
-    constexpr int SLOT = rw_slot<PIV>(), RQ = rw_fv<PIV>() * 16;
-    const int lane = threadIdx.x & 31, ml = lane & 15, part = lane >> 4;
-    const size_t rowst = (size_t)N * Hp;
-    const unsigned sbase = (unsigned)__cvta_generic_to_shared(wring);
-#define WSLOT(s, q) wring[(s) * SLOT + (q) * 16 + ml]
-#define WRHS(s) wring[(s) * SLOT + RQ + lane]
-    const double *Lj = lu + (size_t)(KV + 1) * rowst + nh;
-    const double *Pj = PIV ? pivd + nh : nullptr;
-    const double *Rj = rhs + (size_t)(KL + 1) * rs;
-    int jj = 0;
-    auto issue_fwd = [&](int s) {
-        if (jj < N) {
-            if (jj < N - 1) {
-#pragma unroll
-                for (int q = 0; q < FQ; ++q) {
-                    if ((q & 1) != part) continue;
-                    const unsigned d = sbase + (unsigned)(((s) * SLOT + q * 16 + ml) * 8);
-                    if (q < KL) cp_async8s(d, Lj + q * rowst);
-                    else cp_async8s(d, Pj);
-                }
-            }
-            if (jj + KL + 1 < N) cp_async8s(sbase + (unsigned)(((s) * SLOT + RQ + lane) * 8), Rj);
-        }
-        cp_async_commit();
-        ++jj;
-        Lj += Hp;
-        if (PIV) Pj += Hp;
-        Rj += rs;
-    };
-    double w[KL + 1];
-#pragma unroll
-    for (int i = 0; i <= KL; ++i) w[i] = (i < N) ? rhs[(size_t)i * rs] : 0.0;
-#pragma unroll
-    for (int s = 0; s < RING - 1; ++s) issue_fwd(s);
-    double *Oj = out;
-    for (int j0 = 0; j0 < N; j0 += RING) {
-#pragma unroll
-        for (int s = 0; s < RING; ++s) {
-            const int j = j0 + s;
-            if (j < N) {
-                cp_async_wait<RING - 2>();
-                __syncwarp(mask);
-                const double ahead = (j + KL + 1 < N) ? WRHS(s) : 0.0;
-                if (j < N - 1) {
-                    if (PIV) {
-                        const int p = (int)WSLOT(s, KL);
-#pragma unroll
-                        for (int i = 1; i <= KL; ++i)
-                            if (p == i) {
-                                const double t = w[0];
-                                w[0] = w[i];
-                                w[i] = t;
-                            }
-                    }
-                    const double bj = w[0];
-#pragma unroll
-                    for (int i = 1; i <= KL; ++i)
-                        if (j + i < N) w[i] = fma(-WSLOT(s, i - 1), bj, w[i]);
-                }
-                *Oj = w[0];
-                Oj += os;
-#pragma unroll
-                for (int i = 0; i < KL; ++i) w[i] = w[i + 1];
-                w[KL] = ahead;
-                issue_fwd((s + RING - 1) % RING);  // the slot both lanes finished at j-1
-            }
-        }
-    }
-    cp_async_wait<0>();
-    __syncwarp(mask);  // the partner has read the last forward slots
-    const double *Uj = lu + (size_t)KV * rowst + (size_t)(N - 1) * Hp + nh;
-    int tt = 0;
-    auto issue_bwd = [&](int s) {
-        if (tt < N) {
-#pragma unroll
-            for (int q = 0; q < BQ; ++q)
-                if ((q & 1) == part) cp_async8s(sbase + (unsigned)(((s) * SLOT + q * 16 + ml) * 8), Uj - q * rowst);
-        }
-        cp_async_commit();
-        ++tt;
-        Uj -= Hp;
-    };
-#pragma unroll
-    for (int s = 0; s < RING - 1; ++s) issue_bwd(s);
-    double v[KU + 1];
-#pragma unroll
-    for (int i = 0; i <= KU; ++i) v[i] = (N - 1 - i >= 0) ? __ldcs(out + (size_t)(N - 1 - i) * os) : 0.0;
-    constexpr int QY = 4;
-    double yq[QY];
-#pragma unroll
-    for (int q = 0; q < QY; ++q) {
-        const int r = N - 1 - KU - 1 - q;
-        yq[q] = (r >= 0) ? __ldcs(out + (size_t)r * os) : 0.0;
-    }
-    double *Xj = out + (size_t)(N - 1) * os;
-    for (int t0 = 0; t0 < N; t0 += RING) {
-#pragma unroll
-        for (int s = 0; s < RING; ++s) {
-            const int t = t0 + s;
-            if (t < N) {
-                const int j = N - 1 - t;
-                cp_async_wait<RING - 2>();
-                __syncwarp(mask);
-                const double ahead = yq[0];
-#pragma unroll
-                for (int q = 0; q < QY - 1; ++q) yq[q] = yq[q + 1];
-                {
-                    const int r = j - KU - 1 - QY;
-                    yq[QY - 1] = (r >= 0) ? __ldcs(out + (size_t)r * os) : 0.0;
-                }
-                double x = v[0];
-                if (x != 0.0) {
-                    x = x / WSLOT(s, 0);
-#pragma unroll
-                    for (int i = 1; i <= KU; ++i)
-                        if (j - i >= 0) v[i] = fma(-x, WSLOT(s, i), v[i]);
-                }
-                *Xj = x;
-                Xj -= os;
-#pragma unroll
-                for (int i = 0; i < KU; ++i) v[i] = v[i + 1];
-                v[KU] = (j - KU - 1 >= 0) ? ahead : 0.0;
-                issue_bwd((s + RING - 1) % RING);
-            }
-        }
-    }
-    cp_async_wait<0>();
-#undef WSLOT
-#undef WRHS
-}
-
-// The same banded solve for two right-hand sides through one factor
-// stream: modes (k, m) and (-k, m) have the same matrix (bitwise, see
-// lumesh_entry) and therefore the same factors and pivots, so one thread
-// solves the real (or imaginary) parts of both and every factor value is
-// fetched once for the two.  rhsB/outB belong to the mirror mode; with
-// twin false the second chain is idle.  Each chain's operations are those of
-// solve_async, so the solutions are bitwise the same.
-template <bool PIV, int TS>
-__device__ __forceinline__ void solve_async2(const double *__restrict__ lu, const double *__restrict__ pivd, int N,
-                                             int Hp, int nh, const double *__restrict__ rhsA,
-                                             const double *__restrict__ rhsB, size_t rs, double *outA, double *outB,
-                                             size_t os, bool twin, double *ring) {
-    constexpr int KU = PIV ? KV : KL;
-    constexpr int SWF = KL + 2 + (PIV ? 1 : 0);  // forward slot: L column, two rhs ahead, pivot
-    constexpr int SWB = KU + 1;                  // backward slot: U column
-    constexpr int SW = SWF > SWB ? SWF : SWB;
-    constexpr unsigned QB = 8u * TS, SB = 8u * TS * SW;
-    const size_t rowst = (size_t)N * Hp;
-    const unsigned sbase = (unsigned)__cvta_generic_to_shared(ring);
-#define RSLOT(s, q) ring[((s) * SW + (q)) * TS]
-    const double *Lj = lu + (size_t)(KV + 1) * rowst + nh;
-    const double *Pj = PIV ? pivd + nh : nullptr;
-    const double *RAj = rhsA + (size_t)(KL + 1) * rs;
-    const double *RBj = rhsB + (size_t)(KL + 1) * rs;
-    int jj = 0;
-    auto issue_fwd = [&](int s) {
-        if (jj < N) {
-            if (jj < N - 1) {
-#pragma unroll
-                for (int i = 0; i < KL; ++i) cp_async8s(sbase + s * SB + i * QB, Lj + i * rowst);
-                if (PIV) cp_async8s(sbase + s * SB + (KL + 2) * QB, Pj);
-            }
-            if (jj + KL + 1 < N) {
-                cp_async8s(sbase + s * SB + KL * QB, RAj);
-                if (twin) cp_async8s(sbase + s * SB + (KL + 1) * QB, RBj);
-            }
-        }
-        cp_async_commit();
-        ++jj;
-        Lj += Hp;
-        if (PIV) Pj += Hp;
-        RAj += rs;
-        RBj += rs;
-    };
-    double wa[KL + 1], wb[KL + 1];
-#pragma unroll
-    for (int i = 0; i <= KL; ++i) {
-        wa[i] = (i < N) ? rhsA[(size_t)i * rs] : 0.0;
-        wb[i] = (i < N && twin) ? rhsB[(size_t)i * rs] : 0.0;
-    }
-#pragma unroll
-    for (int s = 0; s < RING; ++s) issue_fwd(s);
-    double *OAj = outA, *OBj = outB;
-    for (int j0 = 0; j0 < N; j0 += RING) {
-#pragma unroll
-        for (int s = 0; s < RING; ++s) {
-            const int j = j0 + s;
-            if (j < N) {
-                cp_async_wait<RING - 1>();
-                const double aheadA = (j + KL + 1 < N) ? RSLOT(s, KL) : 0.0;
-                const double aheadB = (j + KL + 1 < N && twin) ? RSLOT(s, KL + 1) : 0.0;
-                if (j < N - 1) {
-                    if (PIV) {
-                        const int p = (int)RSLOT(s, KL + 2);
-#pragma unroll
-                        for (int i = 1; i <= KL; ++i)
-                            if (p == i) {
-                                const double t = wa[0];
-                                wa[0] = wa[i];
-                                wa[i] = t;
-                                const double u = wb[0];
-                                wb[0] = wb[i];
-                                wb[i] = u;
-                            }
-                    }
-                    const double bja = wa[0], bjb = wb[0];
-#pragma unroll
-                    for (int i = 1; i <= KL; ++i)
-                        if (j + i < N) {
-                            const double L = RSLOT(s, i - 1);
-                            wa[i] = fma(-L, bja, wa[i]);
-                            wb[i] = fma(-L, bjb, wb[i]);
-                        }
-                }
-                *OAj = wa[0];
-                if (twin) *OBj = wb[0];
-                OAj += os;
-                OBj += os;
-#pragma unroll
-                for (int i = 0; i < KL; ++i) {
-                    wa[i] = wa[i + 1];
-                    wb[i] = wb[i + 1];
-                }
-                wa[KL] = aheadA;
-                wb[KL] = aheadB;
-                issue_fwd(s);
-            }
-        }
-    }
-    cp_async_wait<0>();
-    // back substitution with the U columns shared by the two chains
-    const double *Uj = lu + (size_t)KV * rowst + (size_t)(N - 1) * Hp + nh;
-    int tt = 0;
-    auto issue_bwd = [&](int s) {
-        if (tt < N) {
-#pragma unroll
-            for (int i = 0; i <= KU; ++i) cp_async8s(sbase + s * SB + i * QB, Uj - i * rowst);
-        }
-        cp_async_commit();
-        ++tt;
-        Uj -= Hp;
-    };
-#pragma unroll
-    for (int s = 0; s < RING; ++s) issue_bwd(s);
-    double va[KU + 1], vb[KU + 1];
-#pragma unroll
-    for (int i = 0; i <= KU; ++i) {
-        va[i] = (N - 1 - i >= 0) ? __ldcs(outA + (size_t)(N - 1 - i) * os) : 0.0;
-        vb[i] = (N - 1 - i >= 0 && twin) ? __ldcs(outB + (size_t)(N - 1 - i) * os) : 0.0;
-    }
-    constexpr int QY = 4;
-    double ya[QY], yb[QY];
-#pragma unroll
-    for (int q = 0; q < QY; ++q) {
-        const int r = N - 1 - KU - 1 - q;
-        ya[q] = (r >= 0) ? __ldcs(outA + (size_t)r * os) : 0.0;
-        yb[q] = (r >= 0 && twin) ? __ldcs(outB + (size_t)r * os) : 0.0;
-    }
-    double *XAj = outA + (size_t)(N - 1) * os, *XBj = outB + (size_t)(N - 1) * os;
-    for (int t0 = 0; t0 < N; t0 += RING) {
-#pragma unroll
-        for (int s = 0; s < RING; ++s) {
-            const int t = t0 + s;
-            if (t < N) {
-                const int j = N - 1 - t;
-                cp_async_wait<RING - 1>();
-                const double aheadA = ya[0], aheadB = yb[0];
-#pragma unroll
-                for (int q = 0; q < QY - 1; ++q) {
-                    ya[q] = ya[q + 1];
-                    yb[q] = yb[q + 1];
-                }
-                {
-                    const int r = j - KU - 1 - QY;
-                    ya[QY - 1] = (r >= 0) ? __ldcs(outA + (size_t)r * os) : 0.0;
-                    yb[QY - 1] = (r >= 0 && twin) ? __ldcs(outB + (size_t)r * os) : 0.0;
-                }
-                double xa = va[0], xb = vb[0];
-                if (xa != 0.0) {
-                    xa = xa / RSLOT(s, 0);
-#pragma unroll
-                    for (int i = 1; i <= KU; ++i)
-                        if (j - i >= 0) va[i] = fma(-xa, RSLOT(s, i), va[i]);
-                }
-                if (xb != 0.0) {
-                    xb = xb / RSLOT(s, 0);
-#pragma unroll
-                    for (int i = 1; i <= KU; ++i)
-                        if (j - i >= 0) vb[i] = fma(-xb, RSLOT(s, i), vb[i]);
-                }
-                *XAj = xa;
-                if (twin) *XBj = xb;
-                XAj -= os;
-                XBj -= os;
-#pragma unroll
-                for (int i = 0; i < KU; ++i) {
-                    va[i] = va[i + 1];
-                    vb[i] = vb[i + 1];
-                }
-                va[KU] = (j - KU - 1 >= 0) ? aheadA : 0.0;
-                vb[KU] = (j - KU - 1 >= 0) ? aheadB : 0.0;
-                issue_bwd(s);
-            }
-        }
-    }
-    cp_async_wait<0>();
-#undef RSLOT
-}
-
-// items of the paired solves: item = m*K + k (k >= 0); the primary mode
-// (k, m) and, for m >= 1 and k >= 1, its mirror (-k, m)
-__device__ __forceinline__ bool pair_item(const Geo &g, int item, int &nh, int &nh2) {
-    if (item >= g.M * g.K) return false;
-    const int m = item / g.K, k = item - m * g.K;
-    const int base = m * (2 * g.K - 1);
-    nh = m == 0 ? k : base + k;
-    nh2 = (m > 0 && k > 0) ? base - k : -1;
-    return true;
-}
-__host__ __device__ inline int pair_tiles(const Geo &g) { return (g.M * g.K + 31) / 32; }
-
-// S2 with the mirror modes paired: warp = (re or im) of 32 items
-__device__ __forceinline__ void solve_pnp2_body(const StepArgs &a, int bx) {
-    extern __shared__ double ring2p[];
-    const Geo &g = a.g;
-    const int part = threadIdx.x >> 5;
-    int nh, nh2;
-    if (!pair_item(g, bx * 32 + (threadIdx.x & 31), nh, nh2)) return;
-    const size_t st = 2 * (size_t)g.Hp;
-    const bool twin = nh2 >= 0;
-    const int nhb = twin ? nh2 : nh;
-    double *outA = reinterpret_cast<double *>(a.p) + 2 * (size_t)nh + part;
-    double *outB = reinterpret_cast<double *>(a.p) + 2 * (size_t)nhb + part;
-    const double *rhsA = reinterpret_cast<const double *>(a.prhs) + 2 * (size_t)nh + part;
-    const double *rhsB = reinterpret_cast<const double *>(a.prhs) + 2 * (size_t)nhb + part;
-    if (nh == 0) {  // BC=1 at k=m=0: zero (timestep.f90:110-113); no mirror
-        for (int n = 0; n < g.N; ++n) outA[n * st] = 0.0;
-        return;
-    }
-    solve_async2<true, 64>(a.lnp, a.pivd, g.N, g.Hp, nh, rhsA, rhsB, st, outA, outB, st, twin, ring2p + threadIdx.x);
-}
-
-// S4 with the mirror modes paired: warp = one (system, re/im) of 32 items
-__device__ __forceinline__ void solve_ld2_body(const StepArgs &a, int bx) {
-    extern __shared__ double ring4p[];
-    const Geo &g = a.g;
-    const int w = threadIdx.x >> 5;
-    const int sys = w >> 1, part = w & 1;
-    int nh, nh2;
-    if (!pair_item(g, bx * 32 + (threadIdx.x & 31), nh, nh2)) return;
-    const size_t st = 2 * (size_t)g.Hp;
-    const bool twin = nh2 >= 0;
-    const int nhb = twin ? nh2 : nh;
-    const double *rl = reinterpret_cast<const double *>(pick3(a.rl, sys));
-    double *v = reinterpret_cast<double *>(pick3(a.v, sys));
-    const double *lu = sys == 0 ? a.ldp : sys == 1 ? a.ldm : a.ldz;
-    if (pick3(a.ldpiv, sys))
-        solve_async2<true, 192>(lu, pick3(a.pivld, sys), g.N, g.Hp, nh, rl + 2 * (size_t)nh + part,
-                                rl + 2 * (size_t)nhb + part, st, v + 2 * (size_t)nh + part, v + 2 * (size_t)nhb + part,
-                                st, twin, ring4p + threadIdx.x);
-    else
-        solve_async2<false, 192>(lu, nullptr, g.N, g.Hp, nh, rl + 2 * (size_t)nh + part, rl + 2 * (size_t)nhb + part,
-                                 st, v + 2 * (size_t)nh + part, v + 2 * (size_t)nhb + part, st, twin,
-                                 ring4p + threadIdx.x);
-}
-
-// S2 with the factor ring of a mode shared by its real and imaginary lanes:
-// warp = 16 consecutive modes x (re, im)
-__device__ __forceinline__ void solve_pnpw_body(const StepArgs &a, int bx) {
-    extern __shared__ double ring2w[];
-    const Geo &g = a.g;
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, part = lane >> 4;
-    const int nh = bx * 32 + w * 16 + (lane & 15);
-    const size_t st = 2 * (size_t)g.Hp;
-    double *out = reinterpret_cast<double *>(a.p) + 2 * (size_t)nh + part;
-    const bool live = nh < g.H && nh != 0;
-    const unsigned mask = __ballot_sync(0xffffffffu, live);
-    if (nh == 0) {  // BC=1 at k=m=0: zero (timestep.f90:110-113)
-        for (int n = 0; n < g.N; ++n) out[n * st] = 0.0;
-        return;
-    }
-    if (!live) return;
-    const double *rhs = reinterpret_cast<const double *>(a.prhs) + 2 * (size_t)nh + part;
-    // factors of the compact copy: mode (-k, m) reads those of (k, m)
-    solve_async_rw<true>(a.lnpc, a.pivdc, g.N, a.Hcp, mode_compact(nh, g.K), rhs, st, out, st,
-                         ring2w + (size_t)w * RING * rw_slot<true>(), mask);
-}
-
-// S4 with the shared rings: warp = one system of 16 consecutive modes x (re,
-// im); WIDE rings hold the pivoting band (launches of pipes any of whose
-// Helmholtz factorisations pivoted), narrow ones the pivot-free band
-template <bool WIDE>
-__device__ __forceinline__ void solve_ldw_body(const StepArgs &a, int bx) {
-    extern __shared__ double ring4w[];
-    const Geo &g = a.g;
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, part = lane >> 4;
-    const int sys = w >> 1;
-    const int nh = bx * 32 + (w & 1) * 16 + (lane & 15);
-    const bool live = nh < g.H;
-    const unsigned mask = __ballot_sync(0xffffffffu, live);
-    if (!live) return;
-    const size_t st = 2 * (size_t)g.Hp;
-    const double *rhs = reinterpret_cast<const double *>(pick3(a.rl, sys)) + 2 * (size_t)nh + part;
-    double *out = reinterpret_cast<double *>(pick3(a.v, sys)) + 2 * (size_t)nh + part;
-    const double *lu = sys == 0 ? a.ldp : sys == 1 ? a.ldm : a.ldz;
-    double *wr = ring4w + (size_t)w * RING * rw_slot<WIDE>();
-    if constexpr (WIDE) {
-        if (pick3(a.ldpiv, sys)) {
-            solve_async_rw<true>(lu, pick3(a.pivld, sys), g.N, g.Hp, nh, rhs, st, out, st, wr, mask);
-            return;
-        }
-    }
-    solve_async_rw<false>(lu, nullptr, g.N, g.Hp, nh, rhs, st, out, st, wr, mask);
-}
-
-// S3: rhs - rt2pm(grad p) (velocity.f90:232-236) with zero boundary rows
-// (velocity.f90:376-378), one thread per (mode, PR consecutive rows)
-static constexpr int PR = 4;  // S3 rows per thread
-
-__device__ __forceinline__ void step_proj_body(const StepArgs &a, int bx, int by) {
-    const Geo &g = a.g;
-    const int nh = bx * blockDim.x + threadIdx.x, n0 = by * PR;
-    const int N = g.N;
-    if (nh >= g.H) return;
-    const size_t Hp = g.Hp;
-    const double2 *__restrict__ p = a.p + nh;
-    const double2 *__restrict__ v0 = a.v[0] + nh;
-    const double2 *__restrict__ v1 = a.v[1] + nh;
-    const double2 *__restrict__ v2 = a.v[2] + nh;
-    double2 *__restrict__ r0 = a.rl[0] + nh;
-    double2 *__restrict__ r1 = a.rl[1] + nh;
-    double2 *__restrict__ r2 = a.rl[2] + nh;
-    const double *__restrict__ drb = a.dm.dr;
-    int k, m;
-    mode_km(nh, g.K, k, m);
-    const double kal = g.alpha * k;
-    // the pressure rows this thread's band products touch, loaded once
-    double2 pw[PR + 2 * KL];
-#pragma unroll
-    for (int i = 0; i < PR + 2 * KL; ++i) {
-        const int j = n0 - KL + i;
-        pw[i] = (j >= 0 && j < N) ? p[(size_t)j * Hp] : make_double2(0.0, 0.0);
-    }
-#pragma unroll
-    for (int q = 0; q < PR; ++q) {
-        const int n = n0 + q;
-        if (n >= N) break;
-        const size_t at = (size_t)n * Hp;
-        if (n == 0 || n == N - 1) {
-            r0[at] = r1[at] = r2[at] = make_double2(0.0, 0.0);
-            continue;
-        }
-        double2 dr2 = make_double2(0, 0);
-        const int lo = max(0, n - KL), hi = min(N - 1, n + KL);
-#pragma unroll
-        for (int d = -KL; d <= KL; ++d) {
-            const int j = n + d;
-            if (j < lo || j > hi) continue;
-            const double w = drb[(KL + n - j) * N + j];
-            const double2 x = pw[q + KL + d];
-            dr2.x = fma(w, x.x, dr2.x);
-            dr2.y = fma(w, x.y, dr2.y);
-        }
-        const double2 pv = pw[q + KL];
-        const double m1r1 = a.dm.rp[2 * N + n] * g.Mp * m;
-        // grad p = (dr p, i m/r p, i alpha k p); rt2pm of its (r, theta) parts
-        const double tRe = -pv.y * m1r1, tIm = pv.x * m1r1;
-        const double2 vp = v0[at], vm = v1[at], vz = v2[at];
-        r0[at] = make_double2(vp.x - (dr2.x - tIm), vp.y - (dr2.y + tRe));
-        r1[at] = make_double2(vm.x - (dr2.x + tIm), vm.y - (dr2.y - tRe));
-        r2[at] = make_double2(vz.x - (-pv.y * kal), vz.y - (pv.x * kal));
-    }
-}
-
-// S4: warp = one (system, re/im) of 32 consecutive modes; the pivot-free
-// sweep is used for the systems whose factorisation did not pivot
-__device__ __forceinline__ void solve_ld_body(const StepArgs &a, int bx) {
-    extern __shared__ double ring4[];
-    const Geo &g = a.g;
-    const int w = threadIdx.x >> 5;
-    const int nh = bx * 32 + (threadIdx.x & 31);
-    const int sys = w >> 1, part = w & 1;
-    if (nh >= g.H) return;
-    const size_t st = 2 * (size_t)g.Hp;
-    const double *rhs = reinterpret_cast<const double *>(pick3(a.rl, sys)) + 2 * (size_t)nh + part;
-    double *out = reinterpret_cast<double *>(pick3(a.v, sys)) + 2 * (size_t)nh + part;
-    // factors of the compact copy: mode (-k, m) reads those of (k, m), so a
-    // warp's factor loads cover about half as many distinct columns
-    const double *lu = pick3(a.ldc, sys);
-    const int c = mode_compact(nh, g.K);
-    if (pick3(a.ldpiv, sys))  // pivoting band (low Re, small dt or very clustered meshes)
-        solve_async<true, 192>(lu, pick3(a.pivldc, sys), g.N, a.Hcp, c, rhs, st, out, st, ring4 + threadIdx.x);
-    else
-        solve_async<false, 192>(lu, nullptr, g.N, a.Hcp, c, rhs, st, out, st, ring4 + threadIdx.x);
-}
-
-// ------------------------- S4 with the factors rebuilt on chip (no pivoting)
-// For a pipe none of whose Helmholtz factorisations pivoted.  One thread per
-// (system, k >= 0, m): it assembles the band of its mode (lumesh_entry, the
-// bits k_lu_factor assembles) and eliminates it column by column in a 5 x 5
-// register window in dgbtf2's order of operations, while the unit-lower
-// sweep of dgbtrs runs on four right-hand sides at once: the real and
-// imaginary parts of mode (k, m) and of its mirror (-k, m), whose matrix is
-// the same.  The rows U(j, j..j+3) of the upper factor go to shared memory
-// for the back substitution (dtbsv); U(j, j+4) is never updated by the
-// elimination, so it is reassembled instead of stored.  Every factor value
-// and every solve operation is the one k_lu_factor + solve_async perform, so
-// the solutions are bitwise those of the streamed-factor path, but the
-// factors never touch HBM: the launch moves the right-hand sides in and the
-// solutions out (plus the forward results, written and read back once).
-//
-// Shared memory per thread: U rows 4*N doubles and a ring of LDR_D
-// right-hand-side rows (two modes, double2) staged ahead by cp.async.
-static constexpr int LDR_BT = 32;  // items per block
-static constexpr int LDR_D = 8;    // right-hand-side rows in flight per item
-
-__device__ __forceinline__ void cp_async16s(unsigned saddr, const void *gmem) {
+// --------------------------------------------------------- banded solves
+// A warp solves one system of its tile's 16 modes: lane = 2*slot + (re, im),
+// and the right-hand side sits in shared memory as rows of 32 doubles, solved
+// in place.  The factors are streamed from the set's tile (pf_internal.cuh)
+// through a ring of chunks that another warp keeps filled with bulk copies:
+// asking for a copy takes some 200 cycles, as long as five columns of the
+// solve.  Modes k and -k of a paired tile (W = 8) read the same factor values.
+// Column j costs one multiply-add on the dependent chain going forward and
+// three going back: the division by U(j, j) is a product with its reciprocal
+// held as a sum of two doubles, as accurate as the division.  With the
+// factors at hand a column takes 42 cycles forward and 54 back, 73 and 83
+// with pivots and wide rows (N = 40, W = 8).
+__device__ __forceinline__ void cp_async16(unsigned saddr, const void *gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(saddr), "l"(gmem) : "memory");
 }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-static __host__ __device__ inline size_t ldr_smem(int N) {
-    return (size_t)LDR_BT * (4 * (size_t)N * sizeof(double) + (size_t)LDR_D * 2 * sizeof(double2));
+// w[0] and w[p] exchanged, p = 0 .. KL
+__device__ __forceinline__ void pivot_swap(double (&w)[KL + 1], int p) {
+    static_assert(KL == 4, "select tree of five entries");
+    const double t = w[0];
+    const double lo = (p & 1) ? w[1] : t, hi = (p & 1) ? w[3] : w[2];
+    const double mid = (p & 2) ? hi : lo;
+    w[0] = (p & 4) ? w[4] : mid;
+#pragma unroll
+    for (int r = 1; r <= KL; ++r) w[r] = p == r ? t : w[r];
 }
-// tiles of one pipe: 3 systems x ceil(M*K / LDR_BT)
-static __host__ __device__ inline int ldr_tiles(const Geo &g) { return 3 * ((g.M * g.K + LDR_BT - 1) / LDR_BT); }
 
-__device__ __forceinline__ void solve_ld_rebuild_body(const StepArgs &a, int tile) {
-    extern __shared__ __align__(16) double ldr_sm[];
-    const Geo &g = a.g;
-    const int N = g.N, K = g.K;
-    const int nitem = g.M * K;
-    const int per = (nitem + LDR_BT - 1) / LDR_BT;
-    const int sys = tile / per;
-    const int item = (tile - sys * per) * LDR_BT + (int)threadIdx.x;
-    if (item >= nitem) return;  // no block barrier below
-    const int m = item / K, k = item - m * K;
-    const int base = m * (2 * K - 1);
-    const bool twin = m > 0 && k > 0;
-    const int nh = m == 0 ? k : base + k;
-    const int nh2 = twin ? base - k : nh;
-    const int PM = sys == 0 ? 1 : (sys == 1 ? -1 : 0);
-    const int S = (m * g.Mp + abs(PM)) % 2;
-    const double c1 = a.ldc1, c2 = a.ldc2;
-    const DevMesh &dm = a.dm;
-    const size_t Hp = g.Hp;
-    const double2 *__restrict__ rhs = pick3(a.rl, sys);
-    double2 *__restrict__ out = pick3(a.v, sys);
-    double *ur = ldr_sm + threadIdx.x;  // U(j, j+c) at ur[(j*4 + c) * LDR_BT]
-    double2 *ring = reinterpret_cast<double2 *>(ldr_sm + (size_t)4 * N * LDR_BT) + threadIdx.x;
-    const unsigned rbase = (unsigned)__cvta_generic_to_shared(ring);
-    constexpr unsigned RSTEP = 16u * LDR_BT;  // bytes between ring entries
-    auto A = [&](int r, int c) { return lumesh_entry(dm, N, g.Mp, g.alpha, PM, 0, c1, c2, k, m, S, r, c); };
-    // right-hand-side rows enter in order 0, 1, 2, ...; row r sits in slot r % LDR_D
-    int rin = 0;
-    auto issue = [&](void) {
-        if (rin < N) {
-            const unsigned sa = rbase + (unsigned)((rin % LDR_D) * 2) * RSTEP;
-            cp_async16s(sa, rhs + (size_t)rin * Hp + nh);
-            cp_async16s(sa + RSTEP, rhs + (size_t)rin * Hp + nh2);
+// Accesses to a lane's own column of a field under a uniform condition, as
+// predicated instructions (a branch each costs the solves a third of their time).
+__device__ __forceinline__ double lds_if(unsigned addr, bool on) {
+    double v;
+    asm volatile("{\n.reg .pred p;\nsetp.ne.s32 p, %2, 0;\nmov.f64 %0, 0d0000000000000000;\n@p ld.shared.f64 %0, [%1];\n}\n"
+                 : "=d"(v) : "r"(addr), "r"((int)on));
+    return v;
+}
+__device__ __forceinline__ void sts_if(unsigned addr, double v, bool on) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.s32 p, %2, 0;\n@p st.shared.f64 [%0], %1;\n}\n" ::"r"(addr), "d"(v), "r"((int)on));
+}
+
+// Bulk copy of `bytes` (a multiple of 16) into shared memory; the mbarrier's
+// phase completes when they have landed.  One lane calls it.
+__device__ __forceinline__ void bulk_copy(unsigned dst, const void *src, unsigned bytes, unsigned mbar) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(mbar), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(mbar) : "memory");
+}
+// Waits for the phase of the given parity, at most a second or so; false if
+// it did not complete.
+__device__ __forceinline__ bool mbar_wait(unsigned mbar, unsigned parity) {
+    unsigned done = 0;
+    for (int t = 0; t < (1 << 20) && !done; ++t)
+        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+                     : "=r"(done) : "r"(mbar), "r"(parity) : "memory");
+    return done != 0;
+}
+__device__ __forceinline__ void mbar_arrive(unsigned mbar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(mbar) : "memory");
+}
+
+// The stream of one system's factors through its ring.  flags bit 0: the set
+// has pivots; bit 1: its U has entries beyond KL columns (pivots in the last
+// KL+1 columns alone, the wall row's, leave U narrow).  A chunk is `g` groups
+// of 1920 bytes (W = 8) or twice that: five columns of the forward sweep, one
+// turn of its register window, then five narrow or three wide columns of the
+// back substitution.
+static constexpr int RING = 4;      // chunks, or two where four of a group each do not fit
+static constexpr int GROUP = 1920;  // bytes for W = 8
+static constexpr int GF = KL + 1;   // forward columns of a group
+__host__ __device__ constexpr int group_back(bool wide) { return wide ? 3 : 5; }
+__host__ __device__ constexpr int group_bytes(int W) { return GROUP / 8 * W; }
+struct FactorStream {
+    const double *ft;   // the tile
+    int N, W, flags;
+    int g, places;      // groups a chunk, chunks of the ring
+    unsigned ring, full, empty;  // shared addresses: the chunks, RING barriers each
+};
+// Ask for chunks from .. to-1 of the stream, each once its place is free; by
+// one lane.  False if a place never was.
+__device__ __noinline__ bool stream_fill(const FactorStream s, int from, int to) {
+    if (s.g < 1) return false;  // a ring too small for a chunk
+    const double *src = s.ft;
+    int q = 0, place = 0, turn = 0;
+#pragma unroll 1
+    for (int back = 0; back < 2; ++back) {
+        const int cols = s.g * (back ? group_back(s.flags & 2) : GF);
+        const int row = (back ? ft_back_rows(s.flags & 2) : ft_fwd_rows(s.flags & 1)) * s.W;
+#pragma unroll 1
+        for (int j0 = 0; j0 < s.N; j0 += cols, ++q) {
+            const int words = min(cols, s.N - j0) * row;
+            if (q >= to) return true;
+            if (q >= from) {
+                if (turn > 0 && !mbar_wait(s.empty + place * 8, (turn - 1) & 1)) return false;
+                bulk_copy(s.ring + place * s.g * group_bytes(s.W), src, words * 8, s.full + place * 8);
+            }
+            src += words;
+            if (++place == s.places) {
+                place = 0;
+                ++turn;
+            }
         }
-        cp_async_commit();
-        ++rin;
+    }
+    return true;
+}
+
+// A group's factors are read into registers before any of its results is
+// stored, which would order the reads behind the chain.  f: the field's byte
+// offset into the block's dynamic shared memory.  Returns false if a copy
+// never came.
+template <bool PIV, bool WIDE, int W>
+__device__ __noinline__ bool tile_solve(const FactorStream s, int f) {
+    extern __shared__ __align__(128) unsigned char step_sm[];
+    constexpr int FR = ft_fwd_rows(PIV), BR = ft_back_rows(WIDE), KU = BR - 2, GB = group_back(WIDE);
+    static_assert(GF * FR * W * 8 <= group_bytes(W) && GB * BR * W * 8 <= group_bytes(W) && (KU + 1) % GB == 0, "group size");
+    const int lane = threadIdx.x & 31, N = s.N;
+    const unsigned base = (unsigned)__cvta_generic_to_shared(step_sm);
+    const double *rd = reinterpret_cast<const double *>(step_sm + (s.ring - base)) + (W == 16 ? lane >> 1 : lane >> 2);
+    const unsigned fl = base + f + lane * 8;
+    int place = 0, left = 0;
+    unsigned par = 0;
+    bool ok = true;
+    if (s.g < 1) return false;
+    const double *col = rd;
+    auto next = [&](int group) {  // the next group's factors
+        if (left == 0) {
+            ok &= mbar_wait(s.full + place * 8, par);
+            col = rd + place * s.g * (group_bytes(W) / 8);
+            left = s.g;
+        } else {
+            col += group;
+        }
     };
+    // they have been used; at a chunk's end its place is handed back to the
+    // asynchronous copies, which only the proxy fence orders after the reads
+    // (handed back with the reads still in flight, a refill overtook them)
+    auto done = [&](bool sweep_over) {
+        if (--left == 0 || sweep_over) {
+            left = 0;
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(s.empty + place * 8);
+            if (++place == s.places) {
+                place = 0;
+                par ^= 1;
+            }
+        }
+    };
+    {
+        double w[KL + 1];
 #pragma unroll
-    for (int q = 0; q < LDR_D; ++q) issue();
-    cp_async_wait<LDR_D - 5>();  // rows 0..4
-    // forward window: W[i][c] = A(j+i, j+c) as eliminated so far, held in
-    // physical slot [(i+j)%5][(c+j)%5]; right-hand sides w[q][(i+j)%5]
-    double W[5][5];
-    double2 w0[5], w1[5];
+        for (int r = 0; r <= KL; ++r) w[r] = lds_if(fl + r * 256, true);
+        unsigned fj = fl;
+#pragma unroll 1
+        for (int j0 = 0; j0 < N; j0 += GF, fj += GF * 256) {
+            next(GF * FR * W);
+            double L[GF][FR];
 #pragma unroll
-    for (int i = 0; i < 5; ++i) {
+            for (int c = 0; c < GF; ++c)
 #pragma unroll
-        for (int c = 0; c < 5; ++c) W[i][c] = (i < N && c < N) ? A(i, c) : 0.0;
-        const bool in = i < N;
-        w0[i] = in ? ring[(size_t)((i % LDR_D) * 2) * LDR_BT] : make_double2(0.0, 0.0);
-        w1[i] = in ? ring[(size_t)((i % LDR_D) * 2 + 1) * LDR_BT] : make_double2(0.0, 0.0);
+                for (int r = 0; r < FR; ++r) L[c][r] = col[(c * FR + r) * W];
+#pragma unroll
+            for (int c = 0; c < GF; ++c) {  // columns past N-1: nothing of them is stored
+                const double ahead = lds_if(fj + (c + KL + 1) * 256, j0 + c + KL + 1 < N);
+                if (PIV) pivot_swap(w, __double2loint(L[c][FR - 1]));
+                const double b = w[0];
+                sts_if(fj + c * 256, b, j0 + c < N);
+#pragma unroll
+                for (int r = 1; r <= KL; ++r) w[r - 1] = fma(-L[c][r - 1], b, w[r]);  // L zero beyond row N-1
+                w[KL] = ahead;
+            }
+            done(j0 + GF >= N);
+        }
     }
+    {
+        double v[KU + 1];
+        unsigned fj = fl + (N - 1) * 256;
 #pragma unroll
-    for (int q = 0; q < 5; ++q) issue();
-    double2 *Yj = out;  // forward results y(j) of mode nh, then of nh2 at +(nh2-nh)
-    const ptrdiff_t d2 = (ptrdiff_t)nh2 - (ptrdiff_t)nh;
-    Yj += nh;
-    for (int j0 = 0; j0 < N; j0 += 5) {
+        for (int r = 0; r <= KU; ++r) v[r] = lds_if(fj - r * 256, true);
+#pragma unroll 1
+        for (int j0 = N - 1; j0 >= 0; j0 -= KU + 1, fj -= (KU + 1) * 256) {
 #pragma unroll
-        for (int s = 0; s < 5; ++s) {
-            const int j = j0 + s;
-            if (j < N) {
-                const int km = min(KL, N - 1 - j);
-                // column j of L and row j of U (dgbtf2, no interchange)
-                double L[5];
-                const double piv = W[s % 5][s % 5];
+            for (int h = 0; h < (KU + 1) / GB; ++h) {
+                if (h > 0 && j0 - h * GB < 0) break;
+                next(GB * BR * W);
+                double U[GB][BR];
 #pragma unroll
-                for (int c = 0; c < 4; ++c) ur[(size_t)(j * 4 + c) * LDR_BT] = W[s % 5][(c + s) % 5];
-                if (km > 0) {
-                    const double rp = 1.0 / piv;
+                for (int c = 0; c < GB; ++c)
 #pragma unroll
-                    for (int i = 1; i <= KL; ++i) L[i] = (i <= km) ? W[(i + s) % 5][s % 5] * rp : 0.0;
+                    for (int r = 0; r < BR; ++r) U[c][r] = col[(c * BR + r) * W];
 #pragma unroll
-                    for (int c = 1; c <= KL; ++c) {
-                        if (c > km) break;
-                        const double y = -W[s % 5][(c + s) % 5];
+                for (int cc = 0; cc < GB; ++cc) {
+                    const int c = h * GB + cc;
+                    const double ahead = lds_if(fj - (c + KU + 1) * 256, j0 - c - KU - 1 >= 0);
+                    const double x = fma(v[0], U[cc][0], v[0] * U[cc][1]);
+                    sts_if(fj - c * 256, x, j0 - c >= 0);
 #pragma unroll
-                        for (int i = 1; i <= KL; ++i)
-                            if (i <= km) W[(i + s) % 5][(c + s) % 5] = fma(L[i], y, W[(i + s) % 5][(c + s) % 5]);
-                    }
-                    // dgbtrs forward sweep on the four right-hand sides
-                    const double2 b0 = w0[s % 5], b1 = w1[s % 5];
-#pragma unroll
-                    for (int i = 1; i <= KL; ++i)
-                        if (i <= km) {
-                            double2 &x0 = w0[(i + s) % 5], &x1 = w1[(i + s) % 5];
-                            x0.x = fma(-L[i], b0.x, x0.x);
-                            x0.y = fma(-L[i], b0.y, x0.y);
-                            x1.x = fma(-L[i], b1.x, x1.x);
-                            x1.y = fma(-L[i], b1.y, x1.y);
-                        }
+                    for (int r = 1; r <= KU; ++r) v[r - 1] = fma(-x, U[cc][r + 1], v[r]);  // U zero above row 0
+                    v[KU] = ahead;
                 }
-                Yj[0] = w0[s % 5];
-                if (twin) Yj[d2] = w1[s % 5];
-                Yj += Hp;
-                // the row entering the right-hand-side window: j + 5
-                cp_async_wait<LDR_D - 1>();
-                const bool more = j + 5 < N;
-                const int sl = ((j + 5) % LDR_D) * 2;
-                w0[s % 5] = more ? ring[(size_t)sl * LDR_BT] : make_double2(0.0, 0.0);
-                w1[s % 5] = more ? ring[(size_t)(sl + 1) * LDR_BT] : make_double2(0.0, 0.0);
-                issue();
-                // the window moves one row down and one column right: row j+5
-                // and column j+5 enter with their assembled values
-#pragma unroll
-                for (int c = 0; c < 5; ++c) W[s % 5][(c + s) % 5] = (more && c >= 1) ? A(j + 5, j + c) : 0.0;
-                if (more) W[s % 5][s % 5] = A(j + 5, j + 5);
-#pragma unroll
-                for (int i = 1; i < 5; ++i) W[(i + s) % 5][s % 5] = more ? A(j + i, j + 5) : 0.0;
+                done(j0 - (h + 1) * GB < 0);
             }
         }
     }
-    cp_async_wait<0>();
-    // back substitution (dtbsv) on the four right-hand sides; y(j) is read
-    // back through a register queue QY rows ahead
-    constexpr int QY = 4;
-    const double2 *Yr = out + nh;
-    double2 v0[5], v1[5], q0[QY], q1[QY];
-#pragma unroll
-    for (int i = 0; i < 5; ++i) {
-        const int r = N - 1 - i;
-        v0[i] = r >= 0 ? __ldcg(Yr + (size_t)r * Hp) : make_double2(0.0, 0.0);
-        v1[i] = (r >= 0 && twin) ? __ldcg(Yr + (size_t)r * Hp + d2) : make_double2(0.0, 0.0);
-    }
-#pragma unroll
-    for (int q = 0; q < QY; ++q) {
-        const int r = N - 1 - 5 - q;
-        q0[q] = r >= 0 ? __ldcg(Yr + (size_t)r * Hp) : make_double2(0.0, 0.0);
-        q1[q] = (r >= 0 && twin) ? __ldcg(Yr + (size_t)r * Hp + d2) : make_double2(0.0, 0.0);
-    }
-    double2 *Xj = out + nh + (size_t)(N - 1) * Hp;
-    for (int t0 = 0; t0 < N; t0 += 5) {
-#pragma unroll
-        for (int s = 0; s < 5; ++s) {
-            const int t = t0 + s;
-            if (t < N) {
-                const int j = N - 1 - t;
-                // U(j-i, j), i = 0..4
-                double Uc[5];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) Uc[i] = (j - i >= 0) ? ur[(size_t)((j - i) * 4 + i) * LDR_BT] : 0.0;
-                Uc[4] = (j - 4 >= 0) ? A(j - 4, j) : 0.0;
-                double2 x0 = v0[s % 5], x1 = v1[s % 5];
-                // dtbsv skips a column whose right-hand side is exactly zero
-                const bool n0x = x0.x != 0.0, n0y = x0.y != 0.0, n1x = x1.x != 0.0, n1y = x1.y != 0.0;
-                const double u = Uc[0];
-                if (n0x) x0.x = x0.x / u;
-                if (n0y) x0.y = x0.y / u;
-                if (n1x) x1.x = x1.x / u;
-                if (n1y) x1.y = x1.y / u;
-#pragma unroll
-                for (int i = 1; i <= KL; ++i)
-                    if (j - i >= 0) {
-                        double2 &a0 = v0[(i + s) % 5], &a1 = v1[(i + s) % 5];
-                        if (n0x) a0.x = fma(-x0.x, Uc[i], a0.x);
-                        if (n0y) a0.y = fma(-x0.y, Uc[i], a0.y);
-                        if (n1x) a1.x = fma(-x1.x, Uc[i], a1.x);
-                        if (n1y) a1.y = fma(-x1.y, Uc[i], a1.y);
-                    }
-                Xj[0] = x0;
-                if (twin) Xj[d2] = x1;
-                Xj -= Hp;
-                const bool more = j - 5 >= 0;
-                v0[s % 5] = more ? q0[0] : make_double2(0.0, 0.0);
-                v1[s % 5] = more ? q1[0] : make_double2(0.0, 0.0);
-#pragma unroll
-                for (int q = 0; q < QY - 1; ++q) {
-                    q0[q] = q0[q + 1];
-                    q1[q] = q1[q + 1];
-                }
-                const int r = j - 5 - QY;
-                q0[QY - 1] = r >= 0 ? __ldcg(Yr + (size_t)r * Hp) : make_double2(0.0, 0.0);
-                q1[QY - 1] = (r >= 0 && twin) ? __ldcg(Yr + (size_t)r * Hp + d2) : make_double2(0.0, 0.0);
-            }
-        }
-    }
+    __syncwarp();
+    return ok;
 }
 
-// ------------------------------------------------------------------- S5
-__device__ __forceinline__ double sq(double2 a) { return a.x * a.x + a.y * a.y; }
+// ------------------------------------------------------------------ tiles
+// The mode of a slot of a tile: the pipe's first tiles (wide) hold 16
+// consecutive k of m = 0, the others k and -k of 8 consecutive (m, k >= 0),
+// m >= 1, in slots 2i and 2i+1.  Returns false for an idle slot.
+__device__ __forceinline__ bool tile_mode(const Geo &g, int tile, int slot, int &nh, int &k, int &m) {
+    const int nz = pf_mean_tiles(g);
+    if (tile < nz) {
+        m = 0;
+        nh = k = tile * 16 + slot;
+        return k < g.K;
+    }
+    const int it = (tile - nz) * 8 + (slot >> 1);
+    m = 1 + it / g.K;
+    k = it - (m - 1) * g.K;
+    const bool twin = slot & 1;
+    if (twin) k = -k;
+    nh = m * (2 * g.K - 1) + k;
+    return m < g.M && !(twin && k == 0);
+}
+
+__device__ __forceinline__ double sq(double2 a) { return fma(a.x, a.x, __dmul_rn(a.y, a.y)); }
 // max that keeps a NaN (fmax drops it): a state gone non-finite shows as a
 // NaN corrector error instead of a converged one
 __device__ __forceinline__ double nanmax(double a, double b) { return (b > a || b != b) ? b : a; }
 
-__device__ __forceinline__ void step_final_body(const StepArgs &a, int bx) {
-    __shared__ double coef[TM][8];        // aR(1..4), aI(1..4) per mode
-    __shared__ double red[TM * TR];
-    __shared__ double m0buf[3][2][128];    // mode 0 after pm2rt (N <= 128)
+// Row n of a radial band, zero beyond the ends (and for n >= N).  Loaded a
+// row ahead of its use: the tables come from L2 more often than not, as the
+// blocks' shared memory leaves little L1.
+struct BandRow {
+    double w[NBAND];
+    __device__ __forceinline__ void load(const double *__restrict__ band, int N, int n) {
+#pragma unroll
+        for (int d = -KL; d <= KL; ++d) {
+            const int j = n + d;
+            w[d + KL] = j >= 0 && j < N && n < N ? __ldg(band + (KL - d) * N + j) : 0.0;
+        }
+    }
+    // sum_j band(n, j) x(j), j ascending, x a field at this thread's slot
+    __device__ __forceinline__ double2 apply(int N, int n, const double2 *x) const {
+        double2 acc = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int d = -KL; d <= KL; ++d) {
+            const int j = n + d;
+            if (j < 0 || j >= N) continue;
+            const double2 v = x[j * 16];
+            acc.x = fma(w[d + KL], v.x, acc.x);
+            acc.y = fma(w[d + KL], v.y, acc.y);
+        }
+        return acc;
+    }
+};
+
+// Dynamic shared memory of a block: StepHead, four fields b0..b3 of [N][16]
+// double2, the pressure ring of `ppe` bytes, then three Helmholtz rings of
+// `ld` bytes each if there is room for them (`apart`); else these share b3
+// and the pressure ring, once both are done with.
+struct StepHead {
+    unsigned long long bars[4][2][RING];  // LNp, LDp, LDm, LDz: full, empty
+    double ainv[16][17];   // 4x4 inverse per slot
+    double coef[8][16];    // aR(1..4), aI(1..4) per slot
+    double flux;           // 2 int uz r dr of the mean mode
+    double wmax[8];
+};
+static constexpr int STEP_HEAD = 3584;
+static_assert(sizeof(StepHead) <= STEP_HEAD, "block header");
+struct StepSmem {
+    int ppe, ld, apart;
+};
+
+// 16 slots by NT/16 row groups; W = 16: a tile of m = 0.  Products that feed
+// sums are written as fma or rounded products, so every instantiation rounds
+// alike and a pipe steps bit for bit the same alone and in a batch.  Each stage reads
+// the rows it needs of other threads from fields nobody writes in that stage,
+// so a stage is one short loop over the thread's rows and one barrier; fully
+// unrolled rows held in registers took twice as long, waiting for instructions.
+template <int NT, int W>
+__device__ __forceinline__ void step_tile(const StepArgs &a, int tile, const StepSmem lay) {
+    extern __shared__ __align__(128) unsigned char step_sm[];
+    StepHead &hd = *reinterpret_cast<StepHead *>(step_sm);
+    constexpr int NR = NT / 16;
     const Geo &g = a.g;
-    const int N = g.N, Hp = g.Hp;
-    const int tx = threadIdx.x % TM, ty = threadIdx.x / TM;
-    const int nh = bx * TM + tx;
-    const bool live = nh < g.H;
-    int k = 0, m = 0;
-    if (live) mode_km(nh, g.K, k, m);
-    if (ty == 0 && live) {
-        double aR[4] = {0, 0, 0, 0}, aI[4] = {0, 0, 0, 0};
-        if (nh != 0) {  // vel_evalBC + a = -A^-1 B (velocity.f90:239-243, 262-298)
-            const size_t at = (size_t)(N - 1) * Hp + nh;
-            const double2 pw = a.v[0][at], qw = a.v[1][at], zw = a.v[2][at];
-            const double urRe = 0.5 * (pw.x + qw.x), urIm = 0.5 * (pw.y + qw.y);
-            const double utRe = 0.5 * (pw.y - qw.y), utIm = -0.5 * (pw.x - qw.x);
-            double drRe = 0.0, drIm = 0.0;
-            for (int j = 0; j <= KL; ++j) {
-                const size_t aj = (size_t)(N - 1 - KL + j) * Hp + nh;
-                const double w = a.dm.dr1[1 * (KL + 1) + j];
-                const double2 x = a.v[0][aj], y = a.v[1][aj];
-                drRe += w * (x.x + y.x);
-                drIm += w * (x.y + y.y);
+    const int N = g.N, nz = pf_mean_tiles(g);
+    const size_t Hp = g.Hp;
+    const int slot = threadIdx.x & 15, ty = threadIdx.x >> 4, warp = threadIdx.x >> 5;
+    // six of the warps take turns, tile by tile, at solving a system (roles 0
+    // to 2, and 0 the pressure) and at filling its ring (3 to 5): a warp's
+    // number decides the scheduler it runs on
+    static_assert(NT >= 192, "a solving and a filling warp for each system");
+    const int role = warp < 6 ? (warp + tile) % 6 : 6;
+    const bool lane0 = (threadIdx.x & 31) == 0;
+    double2 *const b0 = reinterpret_cast<double2 *>(step_sm + STEP_HEAD) + slot;
+    double2 *const b1 = b0 + N * 16, *const b2 = b1 + N * 16, *const b3 = b2 + N * 16;
+    const unsigned sbase = (unsigned)__cvta_generic_to_shared(step_sm);
+    int nh, k, m;
+    const bool live = tile_mode(g, tile, slot, nh, k, m);
+    if (!live) nh = 0;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 8 * RING; ++i)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(sbase + i * 8) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    }
+    // u_r, u_theta, u_z of the tile into b0, b3, b1
+    for (int n = ty; n < N; n += NR) {
+        const int e = n * 16;
+        if (live) {
+            const size_t at = (size_t)n * Hp + nh;
+            cp_async16((unsigned)__cvta_generic_to_shared(b0 + e), a.u_[0] + at);
+            cp_async16((unsigned)__cvta_generic_to_shared(b3 + e), a.u_[1] + at);
+            cp_async16((unsigned)__cvta_generic_to_shared(b1 + e), a.u_[2] + at);
+        } else {
+            b0[e] = b1[e] = b3[e] = make_double2(0.0, 0.0);
+        }
+    }
+    // the factor streams; those whose rings are free now are started
+    const size_t ftile = (size_t)(W == 16 ? 16 * tile : 8 * (tile + nz)) * N * FT_ROWS;
+    auto stream = [&](int sys) {  // 0: LNp, 1..3: LDp, LDm, LDz
+        FactorStream s;
+        s.N = N;
+        s.W = W;
+        s.ft = (sys == 0 ? a.lnp : pick3(a.ld, sys - 1)) + ftile;
+        s.flags = sys == 0 ? 3 : pick3(a.ldpiv, sys - 1);
+        const int bytes = sys == 0 ? lay.ppe : lay.ld;
+        s.ring = sbase + STEP_HEAD + N * 1024;
+        if (sys > 0) s.ring += (lay.apart ? lay.ppe : -N * 256) + (sys - 1) * lay.ld;
+        s.places = bytes >= RING * group_bytes(W) ? RING : 2;
+        s.g = bytes / (s.places * group_bytes(W));
+        s.full = (unsigned)__cvta_generic_to_shared(&hd.bars[sys][0][0]);
+        s.empty = (unsigned)__cvta_generic_to_shared(&hd.bars[sys][1][0]);
+        return s;
+    };
+    bool ok = true;
+    __syncthreads();  // the barriers are there
+    if (lane0 && (role == 0 || (lay.apart && role >= 3 && role < 6))) {
+        const FactorStream s = stream(role == 0 ? 0 : role - 2);
+        ok = stream_fill(s, 0, s.places);
+    }
+    for (int i = threadIdx.x; i < 256; i += NT) {
+        int h, kk, mm;
+        if (tile_mode(g, tile, i & 15, h, kk, mm)) hd.ainv[i & 15][i >> 4] = h != 0 ? a.Ainv[(size_t)(i >> 4) * Hp + h] : 0.0;
+    }
+    const double *__restrict__ radLap = a.dm.radLap;
+    const double *__restrict__ drb = a.dm.dr;
+    const double *__restrict__ rp = a.dm.rp;
+    const double mMp = (double)(m * g.Mp), kal = g.alpha * k, c2 = a.c2;
+    // diagonal of Lt for the uz system at row n: c1 - c2 ((m Mp)^2/r^2 + (alpha k)^2)
+    const double mm2 = __dmul_rn(mMp, mMp), kk2 = __dmul_rn(kal, kal);
+    auto diag0 = [&](double r2) { return fma(-c2, fma(mm2, r2, kk2), a.c1); };
+    // N of one component at one row, and N_ in the corrector: the loads of the
+    // next row (of the next component after the last) are in flight while one
+    // is worked on; each value is read once: streamed past L1
+    double2 vN = make_double2(0.0, 0.0), vP = vN;
+    auto load_N = [&](int c, int n) {
+        if (!live || n >= N) return;
+        const size_t at = (size_t)n * Hp + nh;
+        vN = __ldcs(pick3(a.Nl, c) + at);
+        if (a.mode == 1) vP = __ldcs(pick3(a.N_, c) + at);
+    };
+    load_N(2, ty);
+    BandRow next;
+    next.load(radLap, N, ty);
+    cp_async_wait_all();
+    __syncthreads();
+    // st 0: rhs of uz, b1 -> b2; st 1: the off-diagonal part of Lt u_r plus
+    // N_r, b0 -> b1; st 2: the same of u_theta (b3), then the u+ and u-
+    // right-hand sides b0, b1
+#pragma unroll 1
+    for (int st = 0; st < 3; ++st) {
+        const int comp = st == 0 ? 2 : st - 1;
+        const double2 *src = st == 0 ? b1 : st == 1 ? b0 : b3;
+#pragma unroll 1
+        for (int n = ty; n < N; n += NR) {
+            double2 v = vN;
+            const double2 P = vP;
+            const bool last = n + NR >= N;
+            if (!last || st < 2) load_N(last ? st : comp, last ? ty : n + NR);
+            const BandRow row = next;
+            next.load(last && st == 2 ? drb : radLap, N, last ? ty : n + NR);
+            const double2 s = row.apply(N, n, src);
+            const double r2 = rp[N + n], d = diag0(r2);
+            if (a.mode == 1) {  // N = c N + (1-c) N_
+                const double d1 = a.implicit, d2 = 1.0 - a.implicit;
+                v = make_double2(fma(d1, v.x, __dmul_rn(d2, P.x)), fma(d1, v.y, __dmul_rn(d2, P.y)));
             }
-            drRe = 0.5 * drRe;
-            drIm = 0.5 * drIm;
-            const double d = a.dm.rp[2 * N + (N - 1)];
-            const double m_ = (double)(m * g.Mp), a_ = g.alpha * k;
-            const double BRe[4] = {pw.x, qw.x, -zw.y, urRe * d + drRe - d * m_ * utIm - a_ * zw.y};
-            const double BIm[4] = {pw.y, qw.y, zw.x, urIm * d + drIm + d * m_ * utRe + a_ * zw.x};
-            for (int i = 0; i < 4; ++i) {
-                double sr = 0.0, si = 0.0;
-                for (int j = 0; j < 4; ++j) {
-                    const double A = a.Ainv[(size_t)(i * 4 + j) * Hp + nh];
-                    sr += A * BRe[j];
-                    si += A * BIm[j];
-                }
-                aR[i] = -sr;
-                aI[i] = -si;
+            if (live) (a.mode == 1 ? pick3(a.Nl, comp) : pick3(a.N_, comp))[(size_t)n * Hp + nh] = v;
+            v = make_double2(fma(c2, s.x, v.x), fma(c2, s.y, v.y));
+            if (st == 0) {
+                const double2 x = b1[n * 16];
+                b2[n * 16] = make_double2(fma(d, x.x, v.x), fma(d, x.y, v.y));
+            } else if (st == 1) {
+                b1[n * 16] = v;
+            } else {
+                const double2 ar = b1[n * 16], x = b0[n * 16], y = b3[n * 16];
+                // the u+- systems' diagonals: -1/r^2 -+ 2 m Mp/r^2 beyond that of uz
+                const double t = __dmul_rn(2.0 * mMp, r2);
+                const double dp = fma(-c2, __dadd_rn(r2, t), d), dm = fma(-c2, __dsub_rn(r2, t), d);
+                b0[n * 16] = make_double2(fma(dp, x.x - y.y, ar.x - v.y), fma(dp, x.y + y.x, ar.y + v.x));
+                b1[n * 16] = make_double2(fma(dm, x.x + y.y, ar.x + v.y), fma(dm, x.y - y.x, ar.y - v.x));
             }
         }
+        __syncthreads();
+    }
+    // div(pm2rt(rhs)) (velocity.f90:98-114; variables.f90:472-477) with
+    // tim_zerobc: b0, b1, b2 -> b3
+#pragma unroll 1
+    for (int n = ty; n < N; n += NR) {
+        const BandRow row = next;
+        next.load(drb, N, n + NR);
+        double2 dv = make_double2(0.0, 0.0);
+        if (n != 0 && n != N - 1) {
+            double2 s = make_double2(0.0, 0.0);
+#pragma unroll 1
+            for (int f = 0; f < 2; ++f) {
+                const double2 e = row.apply(N, n, f ? b1 : b0);
+                s.x += e.x;
+                s.y += e.y;
+            }
+            const double rm1 = rp[2 * N + n], m1r1 = rm1 * mMp;
+            const double2 p = b0[n * 16], q = b1[n * 16], z = b2[n * 16];
+            const double tx = 0.5 * (p.y - q.y), ty_ = -0.5 * (p.x - q.x);
+            dv.x = fma(-z.y, kal, fma(-ty_, m1r1, fma(0.5 * (p.x + q.x), rm1, 0.5 * s.x)));
+            dv.y = fma(z.x, kal, fma(tx, m1r1, fma(0.5 * (p.y + q.y), rm1, 0.5 * s.y)));
+        }
+        b3[n * 16] = dv;
+    }
+    __syncthreads();
+    // LNp of k = m = 0 is held as zeros, so its pressure is zero (timestep.f90:110-113)
+    if (role == 0) {
+        ok &= tile_solve<true, true, W>(stream(0), STEP_HEAD + 3 * N * 256);
+    } else if (role == 3 && lane0) {
+        ok &= stream_fill(stream(0), stream(0).places, 1 << 30);
+    }
+    __syncthreads();
+    // rhs - rt2pm(grad p), grad p = (dr p, i m/r p, i alpha k p); zero boundary rows
+    next.load(drb, N, ty);
+#pragma unroll 1
+    for (int n = ty; n < N; n += NR) {
+        const int e = n * 16;
+        const BandRow row = next;
+        next.load(drb, N, n + NR);
+        if (n == 0 || n == N - 1) {
+            b0[e] = b1[e] = b2[e] = make_double2(0.0, 0.0);
+            continue;
+        }
+        const double2 s = row.apply(N, n, b3);
+        const double2 pv = b3[e];
+        const double m1r1 = rp[2 * N + n] * mMp;
+        const double2 vp = b0[e], vm = b1[e], vz = b2[e];
+        b0[e] = make_double2(vp.x - fma(-pv.x, m1r1, s.x), vp.y - fma(-pv.y, m1r1, s.y));
+        b1[e] = make_double2(vm.x - fma(pv.x, m1r1, s.x), vm.y - fma(pv.y, m1r1, s.y));
+        b2[e] = make_double2(fma(pv.y, kal, vz.x), fma(-pv.x, kal, vz.y));
+    }
+    // b3 and the pressure ring, written by ordinary stores and read by loads
+    // so far, may now take asynchronous copies
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    __syncthreads();
+    if (role < 3) {
+        const FactorStream s = stream(1 + role);
+        const int f = STEP_HEAD + role * N * 256;
+        if (s.flags == 0) ok &= tile_solve<false, false, W>(s, f);
+        else if (s.flags == 1) ok &= tile_solve<true, false, W>(s, f);
+        else ok &= tile_solve<true, true, W>(s, f);  // low Re, small dt or very clustered meshes
+    } else if (role < 6 && lane0) {
+        const FactorStream s = stream(role - 2);
+        ok &= stream_fill(s, lay.apart ? s.places : 0, 1 << 30);
+    }
+    if (!ok) atomicCAS(&a.sc->info, 0, PF_STEP_STUCK);
+    __syncthreads();
+    if (threadIdx.x < 16 && live) {
+        // vel_evalBC + a = -A^-1 B (velocity.f90:239-243, 262-298)
+        const int e = (N - 1) * 16;
+        const double2 pw = b0[e], qw = b1[e], zw = b2[e];
+        const double urRe = 0.5 * (pw.x + qw.x), urIm = 0.5 * (pw.y + qw.y);
+        const double utRe = 0.5 * (pw.y - qw.y), utIm = -0.5 * (pw.x - qw.x);
+        double drRe = 0.0, drIm = 0.0;
+#pragma unroll
+        for (int j = 0; j <= KL; ++j) {
+            const int ej = (N - 1 - KL + j) * 16;
+            const double w = a.dm.dr1[1 * (KL + 1) + j];
+            const double2 x = b0[ej], y = b1[ej];
+            drRe = fma(w, x.x + y.x, drRe);
+            drIm = fma(w, x.y + y.y, drIm);
+        }
+        drRe = 0.5 * drRe;
+        drIm = 0.5 * drIm;
+        const double d = rp[2 * N + (N - 1)];
+        const double dm_ = __dmul_rn(d, mMp);
+        const double BRe[4] = {pw.x, qw.x, -zw.y, fma(-kal, zw.y, fma(-dm_, utIm, fma(urRe, d, drRe)))};
+        const double BIm[4] = {pw.y, qw.y, zw.x, fma(kal, zw.x, fma(dm_, utRe, fma(urIm, d, drIm)))};
         for (int i = 0; i < 4; ++i) {
-            coef[tx][i] = aR[i];
-            coef[tx][4 + i] = aI[i];
+            double sr = 0.0, si = 0.0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                sr = fma(hd.ainv[slot][i * 4 + j], BRe[j], sr);
+                si = fma(hd.ainv[slot][i * 4 + j], BIm[j], si);
+            }
+            hd.coef[i][slot] = -sr;
+            hd.coef[4 + i][slot] = -si;
         }
+    }
+    if (W == 16 && tile == 0 && warp == 1) {  // the tile of k = m = 0 (slot 0)
+        const double2 *z = reinterpret_cast<const double2 *>(step_sm + STEP_HEAD) + 2 * N * 16;
+        double s = 0.0;
+        for (int n = threadIdx.x & 31; n < N; n += 32) s = fma(z[n * 16].x, a.dm.intrdr[n], s);
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if ((threadIdx.x & 31) == 0) hd.flux = 2.0 * s;
     }
     __syncthreads();
     double err = 0.0;
     if (live) {
-        const double *cf = coef[tx];
-        const double2 *__restrict__ v0 = a.v[0] + nh;
-        const double2 *__restrict__ v1 = a.v[1] + nh;
-        const double2 *__restrict__ v2 = a.v[2] + nh;
-        const double *__restrict__ Uc = a.U + nh;
+        double cf[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) cf[i] = hd.coef[i][slot];
+        // U of (k, m) and (-k, m): equal but for the sign of the last vector,
+        // which the gradient's i alpha k gives; both read the k >= 0 column
+        const double *__restrict__ Uc = a.U + (k < 0 ? nh - 2 * k : nh);
+        const double sg = k < 0 ? -1.0 : 1.0;
         double2 *__restrict__ u0 = a.u[0] + nh;
         double2 *__restrict__ u1 = a.u[1] + nh;
         double2 *__restrict__ u2 = a.u[2] + nh;
         const size_t NH = (size_t)N * Hp;
-        // rows are taken two at a time and every load of both rows is issued
-        // before either row's stores, so two rows' memory latencies overlap
-        constexpr int RB = 2;
-        for (int n0 = ty; n0 < N; n0 += RB * TR) {
-            double2 r[RB], t[RB], z[RB], o[RB][3];
-            double Uv[RB][6];
-#pragma unroll
-            for (int q = 0; q < RB; ++q) {
-                const int n = n0 + q * TR;
-                if (n >= N) break;
-                const size_t at = (size_t)n * Hp;
-                r[q] = v0[at];
-                t[q] = v1[at];
-                z[q] = v2[at];
-                if (nh != 0) {
-#pragma unroll
-                    for (int i = 0; i < 6; ++i) Uv[q][i] = Uc[i * NH + at];
-                }
-                if (a.mode == 1 && nh != 0) {  // read once, overwritten below: stream past L1
-                    o[q][0] = __ldcs(u0 + at);
-                    o[q][1] = __ldcs(u1 + at);
-                    o[q][2] = __ldcs(u2 + at);
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < RB; ++q) {
-                const int n = n0 + q * TR;
-                if (n >= N) break;
-                const size_t at = (size_t)n * Hp;
-                double2 rr = r[q], tt = t[q], zz = z[q];
-                if (nh != 0) {
-                    const double U1 = Uv[q][0], U2 = Uv[q][1], U3 = Uv[q][2];
-                    const double U4 = Uv[q][3], U5 = Uv[q][4], U6 = Uv[q][5];
-                    rr.x = rr.x + cf[0] * U1; rr.y = rr.y + cf[4] * U1;
-                    tt.x = tt.x + cf[1] * U2; tt.y = tt.y + cf[5] * U2;
-                    zz.x = zz.x - cf[6] * U3; zz.y = zz.y + cf[2] * U3;
-                    rr.x = rr.x + cf[3] * U4; rr.y = rr.y + cf[7] * U4;
-                    tt.x = tt.x + cf[3] * U5; tt.y = tt.y + cf[7] * U5;
-                    zz.x = zz.x - cf[7] * U6; zz.y = zz.y + cf[3] * U6;
-                }
-                // pm2rt
-                const double2 ur = make_double2(0.5 * (rr.x + tt.x), 0.5 * (rr.y + tt.y));
-                const double2 ut = make_double2(0.5 * (rr.y - tt.y), -0.5 * (rr.x - tt.x));
-                if (nh == 0) {
-                    m0buf[0][0][n] = ur.x; m0buf[0][1][n] = ur.y;
-                    m0buf[1][0][n] = ut.x; m0buf[1][1][n] = ut.y;
-                    m0buf[2][0][n] = zz.x; m0buf[2][1][n] = zz.y;
-                    continue;
-                }
-                if (a.mode == 1) {
-                    err = nanmax(err, sq(make_double2(o[q][0].x - ur.x, o[q][0].y - ur.y)));
-                    err = nanmax(err, sq(make_double2(o[q][1].x - ut.x, o[q][1].y - ut.y)));
-                    err = nanmax(err, sq(make_double2(o[q][2].x - zz.x, o[q][2].y - zz.y)));
-                }
-                u0[at] = ur;
-                u1[at] = ut;
-                u2[at] = zz;
-            }
-        }
-    }
-    if (bx == 0) {  // mode 0: flux adjustment and symmetry zeros
-        __syncthreads();
-        double s = 0.0;
-        for (int n = threadIdx.x; n < N; n += blockDim.x) s += m0buf[2][0][n] * a.dm.intrdr[n];
-        red[threadIdx.x] = s;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double tsum = 0.0;
-            for (int i = 0; i < (int)blockDim.x; ++i) tsum += red[i];
-            red[0] = tsum;
-        }
-        __syncthreads();
-        double d3 = 0.0;
-        if (a.const_flux) d3 = -(2.0 * red[0]) / a.sc->flux_d1;
-        for (int n = threadIdx.x; n < N; n += blockDim.x) {
+        const bool zero = nh == 0;
+        const double d3 = (zero && a.const_flux) ? -hd.flux / a.sc->flux_d1 : 0.0;
+#pragma unroll 2
+        for (int n = ty; n < N; n += NR) {
             const size_t at = (size_t)n * Hp;
-            const double2 ur = make_double2(0.0, 0.0);
-            const double2 ut = make_double2(m0buf[1][0][n], 0.0);
-            double zr = m0buf[2][0][n];
-            if (a.const_flux) zr = zr + d3 * a.Ui[n];
-            const double2 uz = make_double2(zr, 0.0);
-            if (a.mode == 1) {
-                const double2 o0 = a.u[0][at], o1 = a.u[1][at], o2 = a.u[2][at];
-                err = nanmax(err, sq(make_double2(o0.x - ur.x, o0.y - ur.y)));
-                err = nanmax(err, sq(make_double2(o1.x - ut.x, o1.y - ut.y)));
-                err = nanmax(err, sq(make_double2(o2.x - uz.x, o2.y - uz.y)));
+            double Uv[6];
+#pragma unroll
+            for (int i = 0; i < 6; ++i) Uv[i] = zero ? 0.0 : Uc[i * NH + at];
+            double2 o[3];
+            if (a.mode == 1) {  // read once, overwritten below: stream past L1
+                o[0] = __ldcs(u0 + at);
+                o[1] = __ldcs(u1 + at);
+                o[2] = __ldcs(u2 + at);
             }
-            a.u[0][at] = ur;
-            a.u[1][at] = ut;
-            a.u[2][at] = uz;
+            double2 rr = b0[n * 16], tt = b1[n * 16], zz = b2[n * 16];
+            Uv[5] = sg * Uv[5];
+            rr.x = fma(cf[0], Uv[0], rr.x); rr.y = fma(cf[4], Uv[0], rr.y);
+            tt.x = fma(cf[1], Uv[1], tt.x); tt.y = fma(cf[5], Uv[1], tt.y);
+            zz.x = fma(-cf[6], Uv[2], zz.x); zz.y = fma(cf[2], Uv[2], zz.y);
+            rr.x = fma(cf[3], Uv[3], rr.x); rr.y = fma(cf[7], Uv[3], rr.y);
+            tt.x = fma(cf[3], Uv[4], tt.x); tt.y = fma(cf[7], Uv[4], tt.y);
+            zz.x = fma(-cf[7], Uv[5], zz.x); zz.y = fma(cf[3], Uv[5], zz.y);
+            double2 ur = make_double2(0.5 * (rr.x + tt.x), 0.5 * (rr.y + tt.y));
+            double2 ut = make_double2(0.5 * (rr.y - tt.y), -0.5 * (rr.x - tt.x));
+            if (zero) {  // flux adjustment and symmetry zeros of the mean mode
+                ur = make_double2(0.0, 0.0);
+                ut.y = 0.0;
+                zz = make_double2(a.const_flux ? fma(d3, a.Ui[n], zz.x) : zz.x, 0.0);
+            }
+            if (a.mode == 1) {
+                err = nanmax(err, sq(make_double2(o[0].x - ur.x, o[0].y - ur.y)));
+                err = nanmax(err, sq(make_double2(o[1].x - ut.x, o[1].y - ut.y)));
+                err = nanmax(err, sq(make_double2(o[2].x - zz.x, o[2].y - zz.y)));
+            }
+            u0[at] = ur;
+            u1[at] = ut;
+            u2[at] = zz;
         }
-        if (threadIdx.x == 0 && a.const_flux) a.sc->Pr0 = a.sc->Pr0 + d3 * g.Re / 4.0;
+        if (zero && ty == 0 && a.const_flux) a.sc->Pr0 = a.sc->Pr0 + d3 * g.Re / 4.0;
     }
-    if (a.mode == 1) {  // one atomic per block: warp maxima, then the block's
-        __shared__ double wmax[TM * TR / 32];
+    if (a.mode == 1) {
+        // one atomic per block; the pipe's last block publishes the maximum
+        // and clears the accumulator for the next corrector
         for (int o = 16; o > 0; o >>= 1) err = nanmax(err, __shfl_xor_sync(0xffffffffu, err, o));
-        if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = err;
+        if ((threadIdx.x & 31) == 0) hd.wmax[warp] = err;
         __syncthreads();
         if (threadIdx.x == 0) {
-            double e = wmax[0];
-            for (int i = 1; i < TM * TR / 32; ++i) e = nanmax(e, wmax[i]);
-            atomicMax(&a.sc->dterr2_bits, (unsigned long long)__double_as_longlong(e));
+            double e = hd.wmax[0];
+            for (int i = 1; i < NT / 32; ++i) e = nanmax(e, hd.wmax[i]);
+            atomicMax(&a.sc->dterr2_acc, (unsigned long long)__double_as_longlong(e));
+            __threadfence();
+            if (atomicAdd(&a.sc->tiles_done, 1) == pf_step_tiles(g) - 1) {
+                a.sc->dterr2_bits = atomicExch(&a.sc->dterr2_acc, 0ull);
+                a.sc->tiles_done = 0;
+            }
         }
     }
 }
 
 // ------------------------------------------------------------- kernels
-// Lone pipe: one launch per stage over that pipe's tiles.  Batch: one launch
-// per stage over the tiles of every pipe, blk[b] = (pipe, tile of that pipe).
-template <int RPT>
-__global__ void __launch_bounds__(HM *HR, 3) k_step_rhs(StepArgs a) { step_rhs_body<RPT>(a, blockIdx.x); }
-__global__ void k_step_proj(StepArgs a) { step_proj_body(a, blockIdx.x, blockIdx.y); }
-__global__ void __launch_bounds__(192, 4) k_solve_ld(StepArgs a) { solve_ld_body(a, blockIdx.x); }
-__global__ void __launch_bounds__(LDR_BT) k_solve_ldr(StepArgs a) { solve_ld_rebuild_body(a, blockIdx.x); }
-__global__ void __launch_bounds__(64, 8) k_solve_pnp2(StepArgs a) { solve_pnp2_body(a, blockIdx.x); }
-__global__ void __launch_bounds__(192, 3) k_solve_ld2(StepArgs a) { solve_ld2_body(a, blockIdx.x); }
-template <bool WIDE>
-__global__ void __launch_bounds__(192, 4) k_solve_ldw(StepArgs a) { solve_ldw_body<WIDE>(a, blockIdx.x); }
-__global__ void __launch_bounds__(64, 8) k_solve_pnpw(StepArgs a) { solve_pnpw_body(a, blockIdx.x); }
-__global__ void __launch_bounds__(TM *TR) k_step_final(StepArgs a) { step_final_body(a, blockIdx.x); }
-
-#define PF_BATCH1(NAME, BODY, BOUNDS)                                                          \
-    __global__ void BOUNDS NAME(const StepArgs *__restrict__ args, const int2 *__restrict__ blk) { \
-        const int2 pb = blk[blockIdx.x];                                                       \
-        const StepArgs a = args[pb.x]; /* by value: stores cannot alias it */                  \
-        BODY(a, pb.y);                                                                         \
-    }
-PF_BATCH1(k_solve_ld_batch, solve_ld_body, __launch_bounds__(192, 4))
-PF_BATCH1(k_solve_ldr_batch, solve_ld_rebuild_body, __launch_bounds__(LDR_BT))
-PF_BATCH1(k_solve_pnp2_batch, solve_pnp2_body, __launch_bounds__(64, 8))
-PF_BATCH1(k_solve_ld2_batch, solve_ld2_body, __launch_bounds__(192, 3))
-PF_BATCH1(k_solve_pnpw_batch, solve_pnpw_body, __launch_bounds__(64, 8))
-PF_BATCH1(k_solve_ldw_batch0, solve_ldw_body<false>, __launch_bounds__(192, 4))
-PF_BATCH1(k_solve_ldw_batch1, solve_ldw_body<true>, __launch_bounds__(192, 4))
-PF_BATCH1(k_step_final_batch, step_final_body, __launch_bounds__(TM *TR))
-#undef PF_BATCH1
-
-// four blocks per SM in the batch (64 registers; the spilled bytes cost less
-// than the extra warps gain: 4.80 -> 4.73 ms per 64-pipe batch step)
-template <int RPT>
-__global__ void __launch_bounds__(HM *HR, 4) k_step_rhs_batch(const StepArgs *__restrict__ args,
-                                                             const int2 *__restrict__ blk) {
-    const int2 pb = blk[blockIdx.x];
-    const StepArgs a = args[pb.x];  // by value: stores cannot alias it
-    step_rhs_body<RPT>(a, pb.y);
+// Lone pipe: the m = 0 tiles and the paired tiles in one launch.  Batch: one
+// launch per kind of tile and radial size over the tiles of every such pipe,
+// blk[b] = (pipe, tile).  MINB: resident blocks per SM that shared memory
+// allows at that size and the registers are capped for.
+template <int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) k_step(const __grid_constant__ StepArgs a, const StepSmem lay) {
+    if ((int)blockIdx.x < pf_mean_tiles(a.g)) step_tile<NT, 16>(a, blockIdx.x, lay);
+    else step_tile<NT, 8>(a, blockIdx.x, lay);
 }
 
-__global__ void __launch_bounds__(128) k_step_proj_batch(const StepArgs *__restrict__ args, const int2 *__restrict__ blk) {
+template <int NT, int MINB, int W>
+__global__ void __launch_bounds__(NT, MINB) k_step_batch(const StepArgs *__restrict__ args, const int2 *__restrict__ blk,
+                                                         const StepSmem lay) {
     const int2 pb = blk[blockIdx.x];
-    const StepArgs a = args[pb.x];
-    const int gx = (a.g.H + 127) / 128;
-    step_proj_body(a, pb.y % gx, pb.y / gx);
+    const StepArgs a = args[pb.x];  // by value: stores through its pointers cannot alias it
+    step_tile<NT, W>(a, pb.y, lay);
 }
 
 // ------------------------------------------------------------------ host
+static constexpr int STEP_MAX_N = 128;
+
+// (N limit, threads, resident blocks): shared memory, 1 KB a radial point
+// plus the rings, allows that many blocks
+#define PF_STEP_SHAPES(X) X(32, 192, 4) X(64, 256, 2) X(128, 256, 1)
+
+// The rings when `blocks` blocks are to share an SM: what their fields leave
+// free, at least two groups of 16 matrices.  The Helmholtz rings lie apart
+// from the fields where each then has two groups a chunk, or half a sweep:
+// a block alone on its SM has its whole factors in flight from the start.
+static constexpr size_t SM_SMEM = 228 * 1024;
+static StepSmem step_rings(int N, int blocks) {
+    const int room = (int)std::min(SM_SMEM / blocks - 1024, (size_t)227 * 1024) - STEP_HEAD - N * 1024;
+    const int unit = RING * group_bytes(8);  // one group a chunk for W = 8
+    const int half = 2 * ((N + 19) / 20);    // groups of half a forward sweep, an even number
+    StepSmem l{};
+    const int each = std::min(room / 4 / unit, half);
+    l.apart = each >= std::min(2, half);
+    l.ppe = std::max(l.apart ? each : room / unit, 1) * unit;
+    // a stream needs two chunks of a group of 16 matrices: fewer blocks then fit
+    while (!l.apart && (N * 256 + l.ppe) / 3 < 2 * group_bytes(16) + 128) l.ppe += unit;
+    l.ld = l.apart ? l.ppe : ((N * 256 + l.ppe) / 3) & ~127;
+    return l;
+}
+static size_t step_smem(int N, const StepSmem &l) {
+    return (size_t)STEP_HEAD + N * 1024 + l.ppe + (l.apart ? 3 * l.ld : 0);
+}
+
 static StepArgs make_step_args(const pf_ctx *ctx, int corrector) {
     StepArgs a;
     for (int i = 0; i < 3; ++i) {
         a.u_[i] = ctx->prev[i].d;
         a.Nl[i] = ctx->vel[3 + i].d;
         a.N_[i] = ctx->prev[3 + i].d;
-        a.v[i] = ctx->s[i].d;
         a.u[i] = ctx->vel[i].d;
     }
-    a.prhs = ctx->s[3].d;
-    a.p = ctx->s[4].d;
-    a.rl[0] = ctx->s[5].d;
-    a.rl[1] = ctx->s[6].d;
-    a.rl[2] = ctx->s[3].d;  // free once the pressure is solved
-    a.lnp = ctx->LNp.lu;
-    a.pivd = ctx->LNp.pivd;
     const pf_lumesh *ld[3] = {&ctx->LDp, &ctx->LDm, &ctx->LDz};
+    a.lnp = ctx->LNp.tiles;
     for (int i = 0; i < 3; ++i) {
-        a.pivld[i] = ld[i]->pivd;
+        a.ld[i] = ld[i]->tiles;
         a.ldpiv[i] = ld[i]->pivoted;
-        a.ldc[i] = ld[i]->luc;
-        a.pivldc[i] = ld[i]->pivdc;
     }
-    a.lnpc = ctx->LNp.luc;
-    a.pivdc = ctx->LNp.pivdc;
-    a.Hcp = pf_compact_modes_padded(ctx->g);
-    a.ldc1 = ctx->LDp.c1;
-    a.ldc2 = ctx->LDp.c2;
-    a.ldp = ctx->LDp.lu;
-    a.ldm = ctx->LDm.lu;
-    a.ldz = ctx->LDz.lu;
     a.U = ctx->U;
     a.Ainv = ctx->Ainv;
     a.Ui = ctx->Ui;
@@ -1340,76 +700,14 @@ static StepArgs make_step_args(const pf_ctx *ctx, int corrector) {
     return a;
 }
 
-static bool any_ld_pivoted(const pf_ctx *ctx) {
-    return ctx->LDp.pivoted || ctx->LDm.pivoted || ctx->LDz.pivoted;
-}
-
-// The Helmholtz solves rebuild their factors on chip when the tuning asks
-// for it (PF_LD_REBUILT), no factorisation pivoted and N >= 2 KL + 2; the
-// built-in choice streams them.
-static bool ld_rebuild(const pf_ctx *ctx) {
-    return !any_ld_pivoted(ctx) && ctx->g.N >= 2 * KL + 2 && ctx->tune.ld_solver == PF_LD_REBUILT;
-}
-
-// The streamed solves with modes k and -k paired on one factor stream
-// (pressure and Helmholtz); PF_LD_AUTO takes the built-in choice.
-static constexpr int LD_BUILTIN = PF_LD_STREAMED;
-static int ld_choice(const pf_ctx *ctx) {
-    return ctx->tune.ld_solver == PF_LD_AUTO ? LD_BUILTIN : ctx->tune.ld_solver;
-}
-static bool ld_paired(const pf_ctx *ctx) { return ld_choice(ctx) == PF_LD_PAIRED; }
-// The streamed solves with the factor ring of a mode shared by its real and
-// imaginary lanes (pressure and Helmholtz)
-static bool ld_warpring(const pf_ctx *ctx) { return ld_choice(ctx) == PF_LD_WARPRING; }
-static size_t ldw_smem(bool wide) {
-    return (size_t)(192 / 32) * RING * (wide ? rw_slot<true>() : rw_slot<false>()) * sizeof(double);
-}
-static size_t pnpw_smem() { return (size_t)(64 / 32) * RING * rw_slot<true>() * sizeof(double); }
-static size_t ld2_smem(bool piv) { return (size_t)192 * RING * (piv ? KV + 1 : KL + 2) * sizeof(double); }
-static size_t pnp_smem() { return (size_t)64 * RING * (KV + 1) * sizeof(double); }
-
-static size_t rhs_smem(int N) { return (size_t)N * HM * sizeof(double2); }
-
-static int step_attrs() {
-    static bool attrs_set = false;
-    if (!attrs_set) {
-        const int ld = (int)(192 * RING * (KV + 1) * sizeof(double));
-        const int pnp = (int)(64 * RING * (KV + 1) * sizeof(double));
-        PF_CUDA(cudaFuncSetAttribute(k_solve_ld, cudaFuncAttributeMaxDynamicSharedMemorySize, ld));
-        PF_CUDA(cudaFuncSetAttribute(k_solve_ld_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, ld));
-        const int ldr = (int)ldr_smem(HR * 8);
-        PF_CUDA(cudaFuncSetAttribute(k_solve_ldr, cudaFuncAttributeMaxDynamicSharedMemorySize, ldr));
-        PF_CUDA(cudaFuncSetAttribute(k_solve_ldr_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, ldr));
-        PF_CUDA(cudaFuncSetAttribute(k_solve_ld2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ld2_smem(true)));
-        PF_CUDA(cudaFuncSetAttribute(k_solve_ld2_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)ld2_smem(true)));
-        PF_CUDA(cudaFuncSetAttribute(k_solve_pnp2, cudaFuncAttributeMaxDynamicSharedMemorySize, pnp));
-        PF_CUDA(cudaFuncSetAttribute(k_solve_pnp2_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, pnp));
-        const int ldw = (int)ldw_smem(true), pnpw = (int)pnpw_smem();
-        PF_CUDA(cudaFuncSetAttribute(k_solve_ldw<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ldw));
-        PF_CUDA(cudaFuncSetAttribute(k_solve_ldw<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, ldw));
-        PF_CUDA(cudaFuncSetAttribute(k_solve_ldw_batch0, cudaFuncAttributeMaxDynamicSharedMemorySize, ldw));
-        PF_CUDA(cudaFuncSetAttribute(k_solve_ldw_batch1, cudaFuncAttributeMaxDynamicSharedMemorySize, ldw));
-        PF_CUDA(cudaFuncSetAttribute(k_solve_pnpw, cudaFuncAttributeMaxDynamicSharedMemorySize, pnpw));
-        PF_CUDA(cudaFuncSetAttribute(k_solve_pnpw_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, pnpw));
-        const int rhs = (int)rhs_smem(128);
-        PF_CUDA(cudaFuncSetAttribute(k_step_rhs<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, rhs));
-        PF_CUDA(cudaFuncSetAttribute(k_step_rhs<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, rhs));
-        PF_CUDA(cudaFuncSetAttribute(k_step_rhs_batch<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, rhs));
-        PF_CUDA(cudaFuncSetAttribute(k_step_rhs_batch<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, rhs));
-        attrs_set = true;
-    }
-    return PF_OK;
-}
-
-static bool pf_fused_step_geo_ok(const Geo &g) { return g.N <= HR * 8; }
+bool pf_fused_step_ok(const pf_ctx *ctx) { return ctx->g.N <= STEP_MAX_N; }
 
 // One predictor (corrector=0) or corrector (corrector=1) vel_step.  The
 // predictor's u_ := u copy is a pointer swap of vel[0..2] and prev[0..2].
 int pf_vel_step_fused(pf_ctx *ctx, int corrector) {
     const Geo &g = ctx->g;
-    if (!pf_fused_step_geo_ok(g)) {
-        pf_set_error("fused step supports N <= 128");
+    if (!pf_fused_step_ok(ctx)) {
+        pf_set_error("fused step supports N <= %d", STEP_MAX_N);
         return PF_ERR_ARG;
     }
     if (!corrector) {
@@ -1417,47 +715,26 @@ int pf_vel_step_fused(pf_ctx *ctx, int corrector) {
         ctx->parity ^= 1;
     }
     const StepArgs a = make_step_args(ctx, corrector);
-    const int ldsw = any_ld_pivoted(ctx) ? KV + 1 : KL + 1;  // ring slot width of the Helmholtz solves
-    const unsigned tiles = grid1(g.H, TM);
-    PF_TRY(step_attrs());
+    const int blocks = pf_step_tiles(g);
+    int sms = 0;
+    PF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
     {
         ProfScope ps_(ctx, PF_K_STEP);
-        if (g.N <= HR * 4)
-            k_step_rhs<4><<<grid1(g.H, HM), HM * HR, rhs_smem(g.N), ctx->stream>>>(a);
-        else
-            k_step_rhs<8><<<grid1(g.H, HM), HM * HR, rhs_smem(g.N), ctx->stream>>>(a);
+#define PF_CASE(NMAX, NT, MINB)                                             \
+    else if (g.N <= NMAX) {                                                 \
+        const StepSmem lay = step_rings(g.N, MINB);                         \
+        const size_t sm = step_smem(g.N, lay);                              \
+        PF_TRY(pf_raise_smem((const void *)k_step<NT, MINB>, sm));          \
+        k_step<NT, MINB><<<blocks, NT, sm, ctx->stream>>>(a, lay);          \
     }
-    PF_LAUNCHED(ctx);
-    {
-        ProfScope ps_(ctx, PF_K_PPE);
-        if (ld_paired(ctx))
-            k_solve_pnp2<<<pair_tiles(g), 64, pnp_smem(), ctx->stream>>>(a);
-        else  // every other choice: the shared-ring pressure solve (10% faster than a ring per lane)
-            k_solve_pnpw<<<tiles, 64, pnpw_smem(), ctx->stream>>>(a);
-    }
-    PF_LAUNCHED(ctx);
-    {
-        ProfScope ps_(ctx, PF_K_STEP);
-        k_step_proj<<<dim3(grid1(g.H, 128), grid1(g.N, PR)), 128, 0, ctx->stream>>>(a);
-    }
-    PF_LAUNCHED(ctx);
-    {
-        ProfScope ps_(ctx, PF_K_LUSOLVE);
-        if (ld_rebuild(ctx))
-            k_solve_ldr<<<ldr_tiles(g), LDR_BT, ldr_smem(g.N), ctx->stream>>>(a);
-        else if (ld_paired(ctx))
-            k_solve_ld2<<<pair_tiles(g), 192, ld2_smem(any_ld_pivoted(ctx)), ctx->stream>>>(a);
-        else if (ld_warpring(ctx) && any_ld_pivoted(ctx))
-            k_solve_ldw<true><<<tiles, 192, ldw_smem(true), ctx->stream>>>(a);
-        else if (ld_warpring(ctx))
-            k_solve_ldw<false><<<tiles, 192, ldw_smem(false), ctx->stream>>>(a);
-        else
-            k_solve_ld<<<tiles, 192, (size_t)192 * RING * ldsw * sizeof(double), ctx->stream>>>(a);
-    }
-    PF_LAUNCHED(ctx);
-    {
-        ProfScope ps_(ctx, PF_K_INFL);
-        k_step_final<<<tiles, TM * TR, 0, ctx->stream>>>(a);
+        if (blocks <= sms) {  // a block to an SM: all its threads and shared memory for latency
+            const StepSmem lay = step_rings(g.N, 1);
+            const size_t sm = step_smem(g.N, lay);
+            PF_TRY(pf_raise_smem((const void *)k_step<256, 1>, sm));
+            k_step<256, 1><<<blocks, 256, sm, ctx->stream>>>(a, lay);
+        }
+        PF_STEP_SHAPES(PF_CASE)
+#undef PF_CASE
     }
     PF_LAUNCHED(ctx);
     return PF_OK;
@@ -1465,190 +742,126 @@ int pf_vel_step_fused(pf_ctx *ctx, int corrector) {
 
 // ---------------------------------------------------------------- batched
 // Step arguments of every pipe for both pointer parities and both modes,
-// and the tile maps of the five stages.
+// and one (pipe, tile) map per radial size and kind of tile.  The m = 0 tiles
+// launch by themselves: they hold sixteen factor columns instead of eight.  The launches are
+// independent and run concurrently, forked onto auxiliary streams.
+namespace {
+struct StepGroup {
+    int N, W;  // radial points; 16: m = 0 tiles, 8: paired tiles
+    int2 *blk;
+    int nblk;
+};
+}  // namespace
 struct pf_step_batch {
-    int n;
+    void *mem;               // the argument records, then the maps
     StepArgs *d_args[2][2];  // [pointer state after the predictor's swap][mode]
-    int2 *tile, *proj, *half;  // (pipe, tile) maps: 32-mode tiles, 128-mode x row tiles, 16-mode tiles
-    int ntile, nproj, nhalf;
-    int2 *ldmap[2];            // 32-mode tiles of the pipes whose Helmholtz factors [0] never / [1] pivot
-    int nld[2];
-    int2 *ldrmap;              // tiles of the pipes whose Helmholtz factors are rebuilt on chip
-    int nldr, ldrN;            // their count and largest N
-    int2 *pmap;                // 32-item pair tiles of the pipes whose solves pair modes k and -k
-    int np2;
-    int2 *ld2map[2];           // the same tiles split by whether any Helmholtz factorisation [1] pivoted
-    int nld2[2];
-    int2 *pwmap;               // 32-mode tiles of the other pipes (pressure solve, a ring per mode)
-    int npw;
-    int2 *ldwmap[2];           // the same tiles split by whether any Helmholtz factorisation [1] pivoted
-    int nldw[2];
-    int maxN;
-    bool anypiv;
+    std::vector<StepGroup> groups;
+    pf_aux *aux;
 };
 
 void pf_step_batch_free(pf_step_batch *b) {
     if (!b) return;
-    for (int s = 0; s < 2; ++s)
-        for (int m = 0; m < 2; ++m) cudaFree(b->d_args[s][m]);
-    cudaFree(b->tile);
-    cudaFree(b->half);
-    cudaFree(b->ldmap[0]);
-    cudaFree(b->ldmap[1]);
-    cudaFree(b->ldrmap);
-    cudaFree(b->pmap);
-    cudaFree(b->ld2map[0]);
-    cudaFree(b->ld2map[1]);
-    cudaFree(b->pwmap);
-    cudaFree(b->ldwmap[0]);
-    cudaFree(b->ldwmap[1]);
-    cudaFree(b->proj);
+    cudaFree(b->mem);
     delete b;
 }
 
-// state 0: the pointers as the pipes hold them now; state 1: vel/prev swapped
-int pf_step_batch_build(pf_ctx *const *pipes, int n, pf_step_batch **out) {
-    *out = nullptr;
-    pf_step_batch *b = new pf_step_batch();
-    b->n = n;
-    b->maxN = 0;
-    b->anypiv = false;
-    std::vector<StepArgs> h(n);
-    std::vector<int2> tile, proj, half, ldm[2], ldr, pm, ld2m[2], pwm, ldwm[2];
-    b->ldrN = 0;
-    for (int i = 0; i < n; ++i) {
-        const Geo &g = pipes[i]->g;
-        if (!pf_fused_step_geo_ok(g)) {
-            pf_step_batch_free(b);
-            pf_set_error("batched step supports N <= 128");
-            return PF_ERR_ARG;
-        }
-        b->maxN = std::max(b->maxN, g.N);
-        b->anypiv |= any_ld_pivoted(pipes[i]);
-        for (int t = 0; t < (int)grid1(g.H, TM); ++t) tile.push_back(make_int2(i, t));
-        if (ld_paired(pipes[i])) {
-            for (int t = 0; t < pair_tiles(g); ++t) pm.push_back(make_int2(i, t));
-        } else {
-            for (int t = 0; t < (int)grid1(g.H, TM); ++t) pwm.push_back(make_int2(i, t));
-        }
-        if (ld_paired(pipes[i])) {
-            for (int t = 0; t < pair_tiles(g); ++t) ld2m[any_ld_pivoted(pipes[i]) ? 1 : 0].push_back(make_int2(i, t));
-        } else if (ld_warpring(pipes[i])) {
-            for (int t = 0; t < (int)grid1(g.H, TM); ++t) ldwm[any_ld_pivoted(pipes[i]) ? 1 : 0].push_back(make_int2(i, t));
-        } else if (ld_rebuild(pipes[i])) {
-            for (int t = 0; t < ldr_tiles(g); ++t) ldr.push_back(make_int2(i, t));
-            b->ldrN = std::max(b->ldrN, g.N);
-        } else {
-            for (int t = 0; t < (int)grid1(g.H, TM); ++t) ldm[any_ld_pivoted(pipes[i]) ? 1 : 0].push_back(make_int2(i, t));
-        }
-        for (int t = 0; t < (int)grid1(g.H, HM); ++t) half.push_back(make_int2(i, t));
-        for (int t = 0; t < (int)(grid1(g.H, 128) * grid1(g.N, PR)); ++t) proj.push_back(make_int2(i, t));
-    }
+static int step_batch_fill(pf_step_batch *b, pf_ctx *const *pipes, int n) {
+    std::vector<StepArgs> args;
     for (int s = 0; s < 2; ++s)
-        for (int m = 0; m < 2; ++m) {
+        for (int m = 0; m < 2; ++m)
             for (int i = 0; i < n; ++i) {
                 pf_ctx *c = pipes[i];
                 if (s) for (int k = 0; k < 3; ++k) std::swap(c->vel[k].d, c->prev[k].d);
-                h[i] = make_step_args(c, m);
+                args.push_back(make_step_args(c, m));
                 if (s) for (int k = 0; k < 3; ++k) std::swap(c->vel[k].d, c->prev[k].d);
             }
-            if (cudaMalloc((void **)&b->d_args[s][m], n * sizeof(StepArgs)) != cudaSuccess ||
-                cudaMemcpy(b->d_args[s][m], h.data(), n * sizeof(StepArgs), cudaMemcpyHostToDevice) != cudaSuccess) {
-                pf_step_batch_free(b);
-                pf_set_error("batched step: argument upload failed");
-                return PF_ERR_CUDA;
+    std::vector<int> sizes;
+    for (int i = 0; i < n; ++i) sizes.push_back(pipes[i]->g.N);
+    std::sort(sizes.begin(), sizes.end(), std::greater<int>());  // the longest blocks first
+    sizes.erase(std::unique(sizes.begin(), sizes.end()), sizes.end());
+    std::vector<int2> maps;
+    std::vector<size_t> at;
+    for (const int W : {16, 8})
+        for (const int N : sizes) {
+            const size_t from = maps.size();
+            for (int i = 0; i < n; ++i) {
+                const Geo &g = pipes[i]->g;
+                if (g.N != N) continue;
+                const int nz = pf_mean_tiles(g), all = pf_step_tiles(g);
+                for (int t = W == 16 ? 0 : nz; t < (W == 16 ? nz : all); ++t) maps.push_back(make_int2(i, t));
             }
+            if (maps.size() == from) continue;
+            b->groups.push_back(StepGroup{N, W, nullptr, (int)(maps.size() - from)});
+            at.push_back(from);
         }
-    b->ntile = (int)tile.size();
-    b->nhalf = (int)half.size();
-    for (int q = 0; q < 2; ++q) {
-        b->nld[q] = (int)ldm[q].size();
-        if (cudaMalloc((void **)&b->ldmap[q], std::max<size_t>(1, ldm[q].size()) * sizeof(int2)) != cudaSuccess ||
-            (!ldm[q].empty() && cudaMemcpy(b->ldmap[q], ldm[q].data(), ldm[q].size() * sizeof(int2),
-                                           cudaMemcpyHostToDevice) != cudaSuccess)) {
-            pf_step_batch_free(b);
-            pf_set_error("batched step: tile map upload failed");
-            return PF_ERR_CUDA;
+    const size_t abytes = args.size() * sizeof(StepArgs);  // a multiple of 8, as the maps need
+    std::vector<unsigned char> host(abytes + maps.size() * sizeof(int2));
+    std::memcpy(host.data(), args.data(), abytes);
+    std::memcpy(host.data() + abytes, maps.data(), maps.size() * sizeof(int2));
+    PF_CUDA(cudaMalloc(&b->mem, host.size()));
+    PF_CUDA(cudaMemcpy(b->mem, host.data(), host.size(), cudaMemcpyHostToDevice));
+    for (int q = 0; q < 4; ++q) b->d_args[q / 2][q % 2] = reinterpret_cast<StepArgs *>(b->mem) + (size_t)q * n;
+    int2 *blk = reinterpret_cast<int2 *>(reinterpret_cast<unsigned char *>(b->mem) + abytes);
+    for (size_t k = 0; k < at.size(); ++k) b->groups[k].blk = blk + at[k];
+    return b->aux->reserve(b->groups.size());
+}
+
+// state 0: the pointers as the pipes hold them now; state 1: vel/prev swapped
+int pf_step_batch_build(pf_ctx *const *pipes, int n, pf_aux *aux, pf_step_batch **out) {
+    *out = nullptr;
+    for (int i = 0; i < n; ++i)
+        if (!pf_fused_step_ok(pipes[i])) {
+            pf_set_error("batched step supports N <= %d", STEP_MAX_N);
+            return PF_ERR_ARG;
         }
-    }
-    auto upload_map = [&](int2 **d, const std::vector<int2> &h, int *count) {
-        *count = (int)h.size();
-        return cudaMalloc((void **)d, std::max<size_t>(1, h.size()) * sizeof(int2)) == cudaSuccess &&
-               (h.empty() || cudaMemcpy(*d, h.data(), h.size() * sizeof(int2), cudaMemcpyHostToDevice) == cudaSuccess);
-    };
-    if (!upload_map(&b->ldrmap, ldr, &b->nldr) || !upload_map(&b->pmap, pm, &b->np2) ||
-        !upload_map(&b->ld2map[0], ld2m[0], &b->nld2[0]) || !upload_map(&b->ld2map[1], ld2m[1], &b->nld2[1]) ||
-        !upload_map(&b->pwmap, pwm, &b->npw) ||
-        !upload_map(&b->ldwmap[0], ldwm[0], &b->nldw[0]) || !upload_map(&b->ldwmap[1], ldwm[1], &b->nldw[1])) {
+    pf_step_batch *b = new pf_step_batch();
+    b->aux = aux;
+    const int s = step_batch_fill(b, pipes, n);
+    if (s != PF_OK) {
         pf_step_batch_free(b);
-        pf_set_error("batched step: tile map upload failed");
-        return PF_ERR_CUDA;
-    }
-    if (cudaMalloc((void **)&b->half, half.size() * sizeof(int2)) != cudaSuccess ||
-        cudaMemcpy(b->half, half.data(), half.size() * sizeof(int2), cudaMemcpyHostToDevice) != cudaSuccess) {
-        pf_step_batch_free(b);
-        pf_set_error("batched step: tile map upload failed");
-        return PF_ERR_CUDA;
-    }
-    b->nproj = (int)proj.size();
-    if (cudaMalloc((void **)&b->tile, tile.size() * sizeof(int2)) != cudaSuccess ||
-        cudaMalloc((void **)&b->proj, proj.size() * sizeof(int2)) != cudaSuccess ||
-        cudaMemcpy(b->tile, tile.data(), tile.size() * sizeof(int2), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(b->proj, proj.data(), proj.size() * sizeof(int2), cudaMemcpyHostToDevice) != cudaSuccess) {
-        pf_step_batch_free(b);
-        pf_set_error("batched step: tile map upload failed");
-        return PF_ERR_CUDA;
+        return s;
     }
     *out = b;
     return PF_OK;
 }
 
-// One predictor or corrector vel_step of every pipe in five launches; the
-// caller tracks the pointer state (the predictor's swap is the caller's).
+static int step_group_launch(const StepGroup &gr, const StepArgs *a, cudaStream_t st) {
+#define PF_CASE(NMAX, NT, MINB)                                                \
+    else if (gr.N <= NMAX) {                                                   \
+        const StepSmem lay = step_rings(gr.N, MINB);                           \
+        const size_t sm = step_smem(gr.N, lay);                                \
+        if (gr.W == 16) {                                                      \
+            PF_TRY(pf_raise_smem((const void *)k_step_batch<NT, MINB, 16>, sm)); \
+            k_step_batch<NT, MINB, 16><<<gr.nblk, NT, sm, st>>>(a, gr.blk, lay); \
+        } else {                                                               \
+            PF_TRY(pf_raise_smem((const void *)k_step_batch<NT, MINB, 8>, sm));  \
+            k_step_batch<NT, MINB, 8><<<gr.nblk, NT, sm, st>>>(a, gr.blk, lay);  \
+        }                                                                      \
+    }
+    if (false) {
+    }
+    PF_STEP_SHAPES(PF_CASE)
+#undef PF_CASE
+    PF_CHECK_LAUNCH();
+    return PF_OK;
+}
+
+// One predictor or corrector vel_step of every pipe, one launch per group;
+// the caller tracks the pointer state (the predictor's swap is the caller's).
 int pf_step_batch_launch(pf_step_batch *b, int state, int corrector, cudaStream_t st, pf_stage_prof *prof,
                          unsigned long long *nk) {
-    PF_TRY(step_attrs());
     const StepArgs *a = b->d_args[state][corrector ? 1 : 0];
-    {
-        StageScope ss_(prof, PF_K_STEP, st);
-        if (b->maxN <= HR * 4)
-            k_step_rhs_batch<4><<<b->nhalf, HM * HR, rhs_smem(b->maxN), st>>>(a, b->half);
-        else
-            k_step_rhs_batch<8><<<b->nhalf, HM * HR, rhs_smem(b->maxN), st>>>(a, b->half);
+    StageScope ss_(prof, PF_K_STEP, st);
+    const size_t more = b->groups.size() - 1;
+    if (more > 0) PF_CUDA(cudaEventRecord(b->aux->fork, st));
+    for (size_t k = 0; k < more; ++k) PF_CUDA(cudaStreamWaitEvent(b->aux->st[k], b->aux->fork, 0));
+    for (size_t k = 0; k <= more; ++k) {
+        PF_TRY(step_group_launch(b->groups[k], a, k ? b->aux->st[k - 1] : st));
+        ++*nk;
     }
-    PF_CHECK_LAUNCH();
-    {
-        StageScope ss_(prof, PF_K_PPE, st);
-        if (b->np2 > 0) k_solve_pnp2_batch<<<b->np2, 64, pnp_smem(), st>>>(a, b->pmap);
-        if (b->npw > 0) k_solve_pnpw_batch<<<b->npw, 64, pnpw_smem(), st>>>(a, b->pwmap);
+    for (size_t k = 0; k < more; ++k) {
+        PF_CUDA(cudaEventRecord(b->aux->join[k], b->aux->st[k]));
+        PF_CUDA(cudaStreamWaitEvent(st, b->aux->join[k], 0));
     }
-    PF_CHECK_LAUNCH();
-    {
-        StageScope ss_(prof, PF_K_STEP, st);
-        k_step_proj_batch<<<b->nproj, 128, 0, st>>>(a, b->proj);
-    }
-    PF_CHECK_LAUNCH();
-    {
-        StageScope ss_(prof, PF_K_LUSOLVE, st);
-        // pipes whose Helmholtz factors never pivot take the narrow ring (more
-        // blocks per SM), the others the wide one
-        for (int q = 0; q < 2; ++q)
-            if (b->nld[q] > 0)
-                k_solve_ld_batch<<<b->nld[q], 192, (size_t)192 * RING * (q ? KV + 1 : KL + 1) * sizeof(double), st>>>(
-                    a, b->ldmap[q]);
-        if (b->nldr > 0) k_solve_ldr_batch<<<b->nldr, LDR_BT, ldr_smem(b->ldrN), st>>>(a, b->ldrmap);
-        for (int q = 0; q < 2; ++q)
-            if (b->nld2[q] > 0) k_solve_ld2_batch<<<b->nld2[q], 192, ld2_smem(q == 1), st>>>(a, b->ld2map[q]);
-        if (b->nldw[0] > 0) k_solve_ldw_batch0<<<b->nldw[0], 192, ldw_smem(false), st>>>(a, b->ldwmap[0]);
-        if (b->nldw[1] > 0) k_solve_ldw_batch1<<<b->nldw[1], 192, ldw_smem(true), st>>>(a, b->ldwmap[1]);
-    }
-    PF_CHECK_LAUNCH();
-    {
-        StageScope ss_(prof, PF_K_INFL, st);
-        k_step_final_batch<<<b->ntile, TM * TR, 0, st>>>(a, b->tile);
-    }
-    PF_CHECK_LAUNCH();
-    *nk += 3 + (b->np2 > 0) + (b->npw > 0) + (b->nld[0] > 0) + (b->nld[1] > 0) + (b->nldr > 0) +
-           (b->nld2[0] > 0) + (b->nld2[1] > 0) + (b->nldw[0] > 0) + (b->nldw[1] > 0);
     return PF_OK;
 }

@@ -86,9 +86,7 @@ static int vel_step(pf_ctx *ctx) {
     return pf_launch_zero_mode0(ctx);
 }
 
-bool pf_fused_step_ok(const pf_ctx *ctx);
 static bool fused_step_ok(const pf_ctx *ctx) { return pf_fused_step_ok(ctx); }
-bool pf_fused_step_ok(const pf_ctx *ctx) { return ctx->g.N <= 128; }
 
 // velocity.f90:400-410
 extern "C" int pf_vel_predictor(pf_ctx *ctx) {
@@ -120,6 +118,7 @@ int pf_read_dterr(pf_ctx *ctx) {
     PF_CUDA(cudaMemcpyAsync(ctx->hsc, ctx->dsc, sizeof(DevScalars), cudaMemcpyDeviceToHost, ctx->stream));
     PF_CUDA(cudaStreamSynchronize(ctx->stream));
     pf_graph_events_collect(ctx);
+    PF_TRY(pf_step_status(*ctx->hsc));
     const double d2 = bits_to_double(ctx->hsc->dterr2_bits);
     ctx->tim.dterr = std::max(ctx->tim.dterr, std::sqrt(d2));
     return PF_OK;

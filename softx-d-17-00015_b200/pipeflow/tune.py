@@ -4,12 +4,8 @@ No counterpart in the reference: its only tuning is FFTW's own plan search
 (FFTW_PATIENT, transform.fftw3.f90:36-57), which picks radices per transform
 length.  Here the choices are those pf_ctx_set_tuning exposes:
 
-  ld_solver  the banded solves stream the stored LU factors from HBM
-             (PF_LD_STREAMED), share the Helmholtz rings of a mode between
-             its real and imaginary lanes (PF_LD_WARPRING), pair the modes k
-             and -k on one factor stream (PF_LD_PAIRED), or rebuild the
-             Helmholtz factors on chip (PF_LD_REBUILT, for factorisations
-             that did not pivot);
+  ld_solver  accepted for callers that set it; the solves have one form (they
+             run inside the one-launch vel_step), so its candidates tie;
   nl_fused   in mixed precision, the three-pass transforms (0) or those of
              one radial point in one block (1);
   nl_mc      columns (azimuthal modes m) per block of the z transform passes
