@@ -340,15 +340,9 @@ static int staged_body(pf_batch *b, int orbit, int par, unsigned long long *nk) 
     const int s0 = par ^ b->par0, s1 = s0 ^ 1;  // pointer state before / after the predictor's swap
     cudaStream_t st = b->master;
     pf_stage_prof *pr = &b->sprof;
-    {
-        StageScope ss_(pr, PF_K_EW, st);
-        k_batch_sym0<<<b->n, 64, 0, st>>>(b->d_sym[s0]);
-    }
-    PF_CHECK_LAUNCH();
-    ++*nk;
-    PF_TRY(pf_nl_batch_launch(b->nlb, s0, st, pr, nk));
+    PF_TRY(pf_nl_batch_launch(b->nlb, s0, PF_NL_SYM, st, pr, nk));
     PF_TRY(pf_step_batch_launch(b->stb, s1, 0, st, pr, nk));
-    PF_TRY(pf_nl_batch_launch(b->nlb, s1, st, pr, nk));
+    PF_TRY(pf_nl_batch_launch(b->nlb, s1, PF_NL_STEPPED, st, pr, nk));
     PF_TRY(pf_step_batch_launch(b->stb, s1, 1, st, pr, nk));
     if (orbit) {
         {
@@ -393,10 +387,9 @@ static int staged_capture(pf_batch *b, int orbit, int par, cudaGraphExec_t *exec
 
 // one pipe's body of the batch graph
 static int pipe_body(pf_ctx *c, int orbit) {
-    PF_TRY(pf_vel_imposesym(c));
-    PF_TRY(pf_transform_nonlinear(c));
+    PF_TRY(pf_first_nonlinear(c));
     PF_TRY(pf_vel_step_fused(c, 0));
-    PF_TRY(pf_transform_nonlinear(c));
+    PF_TRY(pf_next_nonlinear(c));
     PF_TRY(pf_vel_step_fused(c, 1));
     if (orbit) PF_TRY(pf_vel_imposesym(c));
     return PF_OK;

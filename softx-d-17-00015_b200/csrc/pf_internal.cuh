@@ -133,6 +133,28 @@ __device__ __forceinline__ double lumesh_entry(const DevMesh &dm, int N, int Mp,
     return v;
 }
 
+// curl(u) of one mode at one radial point (variables.f90:408-436) from u there
+// and the radial derivatives of u_t and u_z; rounded alike wherever it is used.
+struct Curl {
+    double2 r, t, z;
+};
+__device__ __forceinline__ Curl mode_curl(double2 ur, double2 ut, double2 uz, double2 dt, double2 dz, double rm1,
+                                          double m1r1, double k1a1) {
+    Curl c;
+    c.r = make_double2(fma(-uz.y, m1r1, __dmul_rn(ut.y, k1a1)), fma(uz.x, m1r1, -__dmul_rn(ut.x, k1a1)));
+    c.t = make_double2(fma(-ur.y, k1a1, -dz.x), fma(ur.x, k1a1, -dz.y));
+    c.z = make_double2(fma(ur.y, m1r1, fma(ut.x, rm1, dt.x)), fma(-ur.x, m1r1, fma(ut.y, rm1, dt.y)));
+    return c;
+}
+// its contribution to the grid mean of u x curl(u)
+__device__ __forceinline__ void mean_terms(bool zero, double2 ur, double2 ut, double2 uz, const Curl &c, double (&s)[3]) {
+    const double w = zero ? 1.0 : 2.0;
+    auto dot = [&](double2 f, double2 h) { return zero ? __dmul_rn(f.x, h.x) : fma(f.x, h.x, __dmul_rn(f.y, h.y)); };
+    s[0] = w * (dot(ut, c.z) - dot(uz, c.t));
+    s[1] = w * (dot(uz, c.r) - dot(ur, c.z));
+    s[2] = w * (dot(ur, c.t) - dot(ut, c.r));
+}
+
 // Device scalars of one context.
 struct DevScalars {
     double Pr0;                      // vel_Pr0
@@ -426,7 +448,8 @@ struct StageScope {
 struct pf_nl_batch;
 bool pf_nl_batch_supported(pf_ctx *const *pipes, int n);
 int pf_nl_batch_build(pf_ctx *const *pipes, int n, bool worklist, pf_nl_batch **out);
-int pf_nl_batch_launch(pf_nl_batch *b, int state, cudaStream_t st, pf_stage_prof *prof, unsigned long long *nk);
+int pf_nl_batch_launch(pf_nl_batch *b, int state, int mode, cudaStream_t st, pf_stage_prof *prof,
+                       unsigned long long *nk);
 void pf_nl_batch_free(pf_nl_batch *b);
 // Streams onto which a batch forks the concurrent launches of a stage, and
 // their events; they live with the batch, whose launches are rebuilt at every
@@ -463,10 +486,19 @@ int pf_step_batch_build(pf_ctx *const *pipes, int n, pf_aux *aux, pf_step_batch 
 int pf_step_batch_launch(pf_step_batch *b, int state, int corrector, cudaStream_t st, pf_stage_prof *prof,
                          unsigned long long *nk);
 void pf_step_batch_free(pf_step_batch *b);
-int pf_launch_nl_fused(pf_ctx *ctx);
+// What the nonlinear terms start from: u alone, u with the mean-mode symmetry
+// still to be imposed, or what a fused predictor has just left (u and its
+// curl, and the mean mode's partial sums).
+#define PF_NL_FRESH 0
+#define PF_NL_SYM 1
+#define PF_NL_STEPPED 2
+int pf_launch_nl_fused(pf_ctx *ctx, int mode);
+void *pf_curl_field(const pf_ctx *ctx, int c);
 int pf_vel_step_fused(pf_ctx *ctx, int corrector);
 void pf_graphs_reset(pf_ctx *ctx);
 int pf_transform_nonlinear(pf_ctx *ctx);
+int pf_first_nonlinear(pf_ctx *ctx);
+int pf_next_nonlinear(pf_ctx *ctx);
 int pf_read_dterr(pf_ctx *ctx);
 bool pf_fused_step_ok(const pf_ctx *ctx);
 void pf_graph_events_collect(pf_ctx *ctx);  // after a host sync

@@ -1,9 +1,11 @@
 // Fused nonlinear term: vel_transform + vel_nonlinear (velocity.f90:304-361)
 // without materialising the six physical fields.
 //
-//   k_nl_zinv  : per (m-chunk, n, component): u or curl(u) (var_coll_curl,
-//                variables.f90:408-436, computed in the load stage), zero-pad
-//                k to 3K, Hermitian fill of m=0, c2c along z (sign +1)
+//   k_nl_prep  : per 32 modes: curl(u) (var_coll_curl, variables.f90:408-436)
+//                in the compute type, and in mixed precision the FP64 sums of
+//                the mean mode; a predictor step leaves both itself (pf_step.cu)
+//   k_nl_zinv  : per (m-chunk, n, component): u or curl(u), zero-pad k to 3K,
+//                Hermitian fill of m=0, c2c along z (sign +1)
 //   k_nl_theta : per (z-chunk, n): c2r along theta for the six components
 //                (two real rows per complex FFT), u x curl(u), scale by
 //                1/(9KM), r2c along theta, CFL maxima of velocity.f90:459-467
@@ -19,7 +21,7 @@
 #include "pf_fftcore.cuh"
 
 static constexpr int NL_THREADS = 256;
-static constexpr int MEAN_THREADS = 256;  // FP64 mean-mode partial sums (mixed precision)
+static constexpr int PREP_THREADS = 256;  // curl(u) and the mean mode's partial sums
 
 struct NLArgs {
     const double2 *u[3];
@@ -32,49 +34,14 @@ struct NLArgs {
     void *T;                  // (m, z) intermediate, compute type
     const void *twz, *twt;    // twiddle tables, compute type
     int MC, ZC;               // z-pass columns and theta-pass rows per block
-    double *mpart;            // FP64 mean-mode partial sums [ceil(H/32)][N][3]
-    float2 *curlf;            // mixed precision: curl(u) in FP32, [(c*N + n)*Hp + nh], made by the
-                              // mean-mode pass before the z pass reads it (null in FP64)
+    double *mpart;            // mixed precision: FP64 mean-mode partial sums [chunk][N][3]
+    void *curl[3];            // curl(u) in the compute type, [n*Hp + nh]
 };
 
 template <typename C> __device__ __forceinline__ C to_c(double2 v);
 template <> __device__ __forceinline__ double2 to_c<double2>(double2 v) { return v; }
 template <> __device__ __forceinline__ float2 to_c<float2>(double2 v) { return make_float2((float)v.x, (float)v.y); }
-
-__device__ __forceinline__ double2 band_row_d(const double *__restrict__ band, int N, int Hp,
-                                              const double2 *__restrict__ in, int n, int nh) {
-    const int lo = max(0, n - KL), hi = min(N - 1, n + KL);
-    double2 acc = make_double2(0.0, 0.0);
-    for (int j = lo; j <= hi; ++j) {
-        const double w = band[(KL + n - j) * N + j];
-        const double2 v = in[(size_t)j * Hp + nh];
-        acc.x = fma(w, v.x, acc.x);
-        acc.y = fma(w, v.y, acc.y);
-    }
-    return acc;
-}
-
-// component `comp` of (u_r, u_t, u_z, curl_r, curl_t, curl_z) at (n, nh)
-__device__ __forceinline__ double2 nl_input(const NLArgs &a, int comp, int n, int nh, int k, int m) {
-    const Geo &g = a.g;
-    const size_t at = (size_t)n * g.Hp + nh;
-    if (comp < 3) return pick3(a.u, comp)[at];
-    const double rm1 = a.dm.rp[2 * g.N + n];
-    const double m1r1 = rm1 * g.Mp * m;
-    const double k1a1 = g.alpha * k;
-    if (comp == 3) {
-        const double2 c2 = a.u[1][at], c3 = a.u[2][at];
-        return make_double2(-c3.y * m1r1 + c2.y * k1a1, c3.x * m1r1 - c2.x * k1a1);
-    }
-    if (comp == 4) {
-        const double2 c1 = a.u[0][at];
-        const double2 dz = band_row_d(a.dm.dr, g.N, g.Hp, a.u[2], n, nh);
-        return make_double2(-c1.y * k1a1 - dz.x, c1.x * k1a1 - dz.y);
-    }
-    const double2 c1 = a.u[0][at], c2 = a.u[1][at];
-    const double2 dt = band_row_d(a.dm.dr, g.N, g.Hp, a.u[1], n, nh);
-    return make_double2(c2.x * rm1 + dt.x + c1.y * m1r1, c2.y * rm1 + dt.y - c1.x * m1r1);
-}
+template <typename C> __device__ __forceinline__ C to_c(float2 v) { return v; }
 
 template <int ZL, typename C>
 __device__ __forceinline__ void nl_zinv_body(const NLArgs &a, int bx, int by, int bz) {
@@ -84,60 +51,35 @@ __device__ __forceinline__ void nl_zinv_body(const NLArgs &a, int bx, int by, in
     const int MC = a.MC;
     if (a.cfl && bx == 0 && by == 0 && bz == 0)  // reset the CFL maxima the theta pass raises
         for (int i = threadIdx.x; i < 3 * a.g.N; i += blockDim.x) a.cfl[i] = 0ull;
-    using FR = FFTRows<ZL, C>;
-    constexpr int RS = FR::pitch;
+    using FR = RowsIO<ZL, C>;
     C *rows = reinterpret_cast<C *>(smraw);
-    C *tw = rows + (FR::smem_elems(MC) - 2 * ZL), *tw2 = tw + ZL;
+    C *tw = rows + (FR::smem_elems(MC) - ZL);
     const Geo &g = a.g;
-    const int K = g.K;
+    constexpr int K = ZL / 3;  // = g.K
     const int comp = bz, n = by, m0 = bx * MC;
     const int mc = min(MC, g.M - m0);
-    fft4_tables<ZL>(tw, tw2, twz);
-    // FP32 transforms (mixed precision): u, or the curl(u) the mean-mode pass
-    // formed once; FP64: u, or curl(u) from 9-row stencils here
-    const float2 *__restrict__ cf = (a.curlf && comp >= 3) ? a.curlf + (size_t)((comp - 3) * g.N + n) * g.Hp : nullptr;
-    const double2 *__restrict__ uc = comp < 3 ? pick3(a.u, comp) + (size_t)n * g.Hp : nullptr;
-    auto input = [&](int nh, int k, int m) -> C {
-        if constexpr (sizeof(C) == 8) {
-            return comp >= 3 ? cf[nh] : to_c<C>(uc[nh]);
-        } else {
-            return to_c<C>(nl_input(a, comp, n, nh, k, m));
-        }
-    };
-#pragma unroll 4
-    for (int idx = threadIdx.x; idx < mc * ZL; idx += blockDim.x) {
-        const int c = idx / ZL, j = idx - c * ZL;
-        const int m = m0 + c;
-        C v = CTraits<C>::make(0, 0);
-        if (m == 0) {
-            if (j < K) v = input(j, j, 0);
-            else if (j >= 2 * K + 1) {
-                v = input(ZL - j, ZL - j, 0);
-                v.y = -v.y;
-            }
-        } else {
-            const int kk = j < K ? j : (j >= 2 * K + 1 ? j - ZL : K);
-            if (kk < K) v = input(m * (2 * K - 1) + kk, kk, m);
-        }
-        rows[c * RS + j] = v;
-    }
-    __syncthreads();
-    FR::template run<+1>(rows, mc, tw, tw2);
+    FR::table(tw, twz);
     C *out = T + ((size_t)(comp * g.N + n) * g.M + m0) * ZL;
-    if constexpr (sizeof(C) == 8 && ZL % 2 == 0) {
-        // FP32, even length: two z values per 16-byte store (every column
-        // of the intermediate starts on a 16-byte boundary)
-        for (int idx = threadIdx.x; idx < mc * ZL / 2; idx += blockDim.x) {
-            const int c = (2 * idx) / ZL, j = 2 * idx - c * ZL;
-            const C x0 = rows[c * RS + j], x1 = rows[c * RS + j + 1];
-            reinterpret_cast<float4 *>(out)[idx] = make_float4(x0.x, x0.y, x1.x, x1.y);
-        }
-    } else {
-        for (int idx = threadIdx.x; idx < mc * ZL; idx += blockDim.x) {
-            const int c = idx / ZL, j = idx - c * ZL;
-            out[idx] = rows[c * RS + j];
-        }
-    }
+    auto pass = [&](auto *__restrict__ src) {
+        FR::template run<+1>(
+            rows, mc, tw,
+            [&](int c, int j) -> C {  // zero-padded in k, the Hermitian fill at m = 0
+                const int m = m0 + c;
+                const int kk = j < K ? j : j - ZL;
+                const bool zero = j >= K && j <= 2 * K, conj = m == 0 && kk < 0;
+                C v = CTraits<C>::make(0, 0);
+                if (!zero) v = to_c<C>(src[conj ? -kk : m * (2 * K - 1) + kk]);
+                v.y = conj ? -v.y : v.y;
+                return v;
+            },
+            [&](int c, int j, int step, auto &v) {
+#pragma unroll
+                for (int q = 0; q < (int)(sizeof(v) / sizeof(C)); ++q) out[c * ZL + j + step * q] = v[q];
+            });
+    };
+    // u in FP64, curl(u) in the compute type
+    if (comp < 3) pass(pick3(a.u, comp) + (size_t)n * g.Hp);
+    else pass(reinterpret_cast<const C *>(pick3(a.curl, comp - 3)) + (size_t)n * g.Hp);
 }
 
 __device__ __forceinline__ void atomic_max_pos(unsigned long long *p, double v) {
@@ -295,32 +237,15 @@ __device__ __forceinline__ void nl_zfwd_body(const NLArgs &a, int bx, int by, in
     const C *__restrict__ T = reinterpret_cast<const C *>(a.T);
     const C *__restrict__ twz = reinterpret_cast<const C *>(a.twz);
     const int MC = a.MC;
-    using FR = FFTRows<ZL, C>;
-    constexpr int RS = FR::pitch;
+    using FR = RowsIO<ZL, C>;
     C *rows = reinterpret_cast<C *>(smraw);
-    C *tw = rows + (FR::smem_elems(MC) - 2 * ZL), *tw2 = tw + ZL;
+    C *tw = rows + (FR::smem_elems(MC) - ZL);
     const Geo &g = a.g;
-    const int K = g.K;
+    constexpr int K = ZL / 3;  // = g.K
     const int comp = bz, n = by, m0 = bx * MC;
     const int mc = min(MC, g.M - m0);
-    fft4_tables<ZL>(tw, tw2, twz);
+    FR::table(tw, twz);
     const C *in = T + ((size_t)(comp * g.N + n) * g.M + m0) * ZL;
-    if constexpr (sizeof(C) == 8 && ZL % 2 == 0) {  // FP32, even length: 16-byte loads
-        for (int idx = threadIdx.x; idx < mc * ZL / 2; idx += blockDim.x) {
-            const int c = (2 * idx) / ZL, j = 2 * idx - c * ZL;
-            const float4 q = reinterpret_cast<const float4 *>(in)[idx];
-            rows[c * RS + j] = CTraits<C>::make(q.x, q.y);
-            rows[c * RS + j + 1] = CTraits<C>::make(q.z, q.w);
-        }
-    } else {
-        for (int idx = threadIdx.x; idx < mc * ZL; idx += blockDim.x) {
-            const int c = idx / ZL, j = idx - c * ZL;
-            rows[c * RS + j] = in[idx];
-        }
-    }
-    __syncthreads();
-    FR::template run<-1>(rows, mc, tw, tw2);
-    const C *res = rows;
     const double U = a.dm.velU[n], b = -a.dm.velUp[n];
     // the constant-flux pressure Pr0 enters at k = m = 0 only: the first
     // m-chunk of the axial component needs it (vel_addHPF, velocity.f90:355-359)
@@ -333,19 +258,34 @@ __device__ __forceinline__ void nl_zfwd_body(const NLArgs &a, int bx, int by, in
     double2 *__restrict__ f = pick3(a.N, comp) + (size_t)n * g.Hp;
     const double2 *__restrict__ uc = pick3(a.u, comp) + (size_t)n * g.Hp;
     const double2 *__restrict__ ur0 = a.u[0] + (size_t)n * g.Hp;
-    const float ik = 1.0f / (2 * K - 1);
-#pragma unroll 4
-    for (int idx = threadIdx.x; idx < mc * (2 * K - 1); idx += blockDim.x) {
-        const int c = fdiv(idx, 2 * K - 1, ik), kk = idx - c * (2 * K - 1) - (K - 1);
-        const int m = m0 + c;
-        if (m == 0 && kk < 0) continue;
-        const int nh = m * (2 * K - 1) + kk;
-        const C x = res[c * RS + (kk >= 0 ? kk : ZL + kk)];
-        const double av = g.alpha * kk * U;
-        const double2 vr = comp == 2 ? ur0[nh] : make_double2(0.0, 0.0);
-        f[nh] = hpf_out(make_double2((double)x.x, (double)x.y), comp, av, b, uc[nh], vr, nh == 0 && a.const_flux,
-                        Pr0, g.Re);
-    }
+    FR::template run<-1>(
+        rows, mc, tw, [&](int c, int j) -> C { return in[c * ZL + j]; },
+        [&](int c, int j, int step, auto &v) {  // the kept |k| < K, k >= 0 only at m = 0
+            constexpr int R = sizeof(v) / sizeof(C), G = R % 4 == 0 ? 4 : R % 3 == 0 ? 3 : 2;
+            const int m = m0 + c;
+            // the velocity at a few modes is read before any of them is stored
+#pragma unroll
+            for (int q0 = 0; q0 < R; q0 += G) {
+                double2 u[G], ur[G];
+#pragma unroll
+                for (int q = 0; q < G; ++q) {
+                    const int t = j + step * (q0 + q), kk = t < K ? t : t - ZL;
+                    const bool on = !(t >= K && t <= 2 * K) && !(m == 0 && kk < 0);
+                    u[q] = ur[q] = make_double2(0.0, 0.0);
+                    if (on) u[q] = uc[m * (2 * K - 1) + kk];
+                    if (on && comp == 2) ur[q] = ur0[m * (2 * K - 1) + kk];
+                }
+#pragma unroll
+                for (int q = 0; q < G; ++q) {
+                    const int t = j + step * (q0 + q), kk = t < K ? t : t - ZL, nh = m * (2 * K - 1) + kk;
+                    const bool on = !(t >= K && t <= 2 * K) && !(m == 0 && kk < 0);
+                    const C x = v[q0 + q];
+                    if (on)
+                        f[nh] = hpf_out(make_double2((double)x.x, (double)x.y), comp, g.alpha * kk * U, b, u[q], ur[q],
+                                        nh == 0 && a.const_flux, Pr0, g.Re);
+                }
+            }
+        });
 }
 
 // ------------------------------------------- one radial point in one block
@@ -382,8 +322,8 @@ __device__ __forceinline__ void nl_fused_body(const NLArgs &a, int n) {
     float2 *twz = Q + 3 * ZC * PT, *twz2 = twz + ZL, *twt = twz2 + ZL, *twt2 = twt + TL;
     fft4_tables<ZL>(twz, twz2, reinterpret_cast<const float2 *>(a.twz));
     fft4_tables<TL>(twt, twt2, reinterpret_cast<const float2 *>(a.twt));
-    const size_t Hp = g.Hp, fs = (size_t)g.N * Hp;
-    // z inverse input: u, or the FP32 curl(u) of the mean-mode pass,
+    const size_t Hp = g.Hp;
+    // z inverse input: u, or the FP32 curl(u),
     // zero-padded to ZL with the Hermitian fill of m = 0 (as k_nl_zinv)
     const float inZ = 1.0f / ZL, inM = 1.0f / M;
 #pragma unroll 4
@@ -402,13 +342,13 @@ __device__ __forceinline__ void nl_fused_body(const NLArgs &a, int n) {
         float2 v = make_float2(0.f, 0.f);
         if (nh >= 0) {
             const size_t at = (size_t)n * Hp + nh;
-            v = comp < 3 ? to_c<float2>(pick3(a.u, comp)[at]) : a.curlf[(comp - 3) * fs + at];
+            v = comp < 3 ? to_c<float2>(pick3(a.u, comp)[at]) : reinterpret_cast<const float2 *>(pick3(a.curl, comp - 3))[at];
             if (conj) v.y = -v.y;
         }
         P[r * PZ + j] = v;
     }
     __syncthreads();
-    fft4_rows<ZL, +1>(P, 6 * M, PZ, twz, twz2);
+    fft4_rows<ZL, +1>(P, 6 * M, PZ, twz2);
     // theta pass, ZC z rows at a time (as k_nl_theta)
     const float scale = (float)(1.0 / (double)(g.Z * g.Th));
     const float base = (float)(1.0 - a.dm.rp[4 * g.N + n] * a.dm.rp[4 * g.N + n]);
@@ -434,7 +374,7 @@ __device__ __forceinline__ void nl_fused_body(const NLArgs &a, int n) {
             Q[(comp * np + zp) * PT + t] = x;
         }
         __syncthreads();
-        fft4_rows<TL, +1>(Q, 6 * np, PT, twt, twt2);
+        fft4_rows<TL, +1>(Q, 6 * np, PT, twt2);
         // u x curl(u) (velocity.f90:325-329) in place over the first three
         // components' rows, scaled for the forward transform
         for (int idx = threadIdx.x; idx < np * TL; idx += blockDim.x) {
@@ -456,7 +396,7 @@ __device__ __forceinline__ void nl_fused_body(const NLArgs &a, int n) {
             }
         }
         __syncthreads();
-        fft4_rows<TL, -1>(Q, 3 * np, PT, twt, twt2);
+        fft4_rows<TL, -1>(Q, 3 * np, PT, twt2);
         // separate the two packed real transforms, keep m < M, back into the
         // plane rows of the first three components
         for (int idx = threadIdx.x; idx < 3 * M * np; idx += blockDim.x) {
@@ -484,7 +424,7 @@ __device__ __forceinline__ void nl_fused_body(const NLArgs &a, int n) {
             cflw[2][threadIdx.x >> 5] = mz;
         }
     }
-    fft4_rows<ZL, -1>(P, 3 * M, PZ, twz, twz2);  // synchronises first: cflw is complete after it
+    fft4_rows<ZL, -1>(P, 3 * M, PZ, twz2);  // synchronises first: cflw is complete after it
     if (a.cfl && threadIdx.x < 3) {
         float v = 0.f;
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v = fmaxf(v, cflw[threadIdx.x][w]);
@@ -527,7 +467,7 @@ template <typename C, int L> struct NLOcc {
     static constexpr int zinv = L >= 144 ? 3 : 0, theta = L >= 144 ? 3 : 0, zfwd = L >= 144 ? 3 : 0;
 };
 template <int L> struct NLOcc<float2, L> {
-    static constexpr int zinv = L <= 192 ? 5 : 0, theta = L <= 192 ? 6 : 0, zfwd = L <= 192 ? 5 : 0;
+    static constexpr int zinv = L <= 192 ? 5 : 0, theta = L <= 192 ? 6 : 0, zfwd = L <= 192 ? 4 : 0;
 };
 
 template <int ZL, typename C>
@@ -618,6 +558,18 @@ template <typename C> static int rows_elems(int L, int B) {
     }
 }
 
+template <typename C> static int rows_io_elems(int L, int B) {
+    switch (L) {
+#define PF_CASE(L) \
+    case L:        \
+        return RowsIO<L, C>::smem_elems(B);
+        PF_NL_LENGTHS(PF_CASE)
+#undef PF_CASE
+    default:
+        return 2 * B * L + 2 * L;
+    }
+}
+
 // tiles and shared memory of one pipe's three launches
 template <typename C> struct NLTiles {
     int MC, ZC;
@@ -640,9 +592,9 @@ template <typename C> static NLTiles<C> nl_tiles(const Geo &g, const pf_tuning &
         t.MC = std::min(tu.nl_mc, g.M);
     } else {
         t.MC = g.M;
-        while (t.MC > 1 && (size_t)rows_elems<C>(g.Z, t.MC) * cs > (f32 ? 32 : 64) * 1024) --t.MC;
+        while (t.MC > 1 && (size_t)rows_io_elems<C>(g.Z, t.MC) * cs > (f32 ? 32 : 64) * 1024) --t.MC;
     }
-    t.zsm = (size_t)rows_elems<C>(g.Z, t.MC) * cs;
+    t.zsm = (size_t)rows_io_elems<C>(g.Z, t.MC) * cs;
     if (tu.nl_zc > 0) {
         t.ZC = tu.nl_zc;
     } else {
@@ -669,6 +621,14 @@ int pf_nl_tiles_check(const pf_ctx *ctx, const pf_tuning *tu) {
     return PF_OK;
 }
 
+// Where curl(u) waits for the z pass: FP64 in scratch fields; in mixed
+// precision after the first 6*N*M*Z float2 of T, which the FP32 transforms use.
+void *pf_curl_field(const pf_ctx *ctx, int c) {
+    if (ctx->cfg.precision != PF_PREC_MIXED) return ctx->s[c].d;
+    const Geo &g = ctx->g;
+    return reinterpret_cast<float2 *>(ctx->T) + (size_t)6 * g.N * g.M * g.Z + (size_t)c * g.N * g.Hp;
+}
+
 // The fused-transform arguments of one pipe in its current pointer state.
 static NLArgs make_nl_args(pf_ctx *ctx) {
     NLArgs a;
@@ -684,8 +644,7 @@ static NLArgs make_nl_args(pf_ctx *ctx) {
     a.T = ctx->T;
     a.mpart = ctx->mpart;
     const bool mixed = ctx->cfg.precision == PF_PREC_MIXED;
-    // FP32 transforms use the first 6*N*M*Z float2 of T; the curl fields follow
-    a.curlf = mixed ? reinterpret_cast<float2 *>(ctx->T) + (size_t)6 * ctx->g.N * ctx->g.M * ctx->g.Z : nullptr;
+    for (int i = 0; i < 3; ++i) a.curl[i] = pf_curl_field(ctx, i);
     a.twz = mixed ? (const void *)ctx->twZf : (const void *)ctx->twZ;
     a.twt = mixed ? (const void *)ctx->twTf : (const void *)ctx->twT;
     int fzc = 0;
@@ -778,60 +737,77 @@ static int launch_nl(pf_ctx *ctx, const NLArgs &a) {
     return PF_OK;
 }
 
-__global__ void k_nl_mean64_part(NLArgs a);
-__global__ void k_nl_mean64_fin(NLArgs a);
-static int mean_attrs();
-static size_t mean_smem(int N);
+template <bool MIXED> __global__ void k_nl_prep(NLArgs a, int sym);
+__global__ void k_nl_mean64_fin(NLArgs a, int stepped);
+static int prep_attrs();
+static size_t prep_smem(int N);
+static constexpr int PREP_MAX_N = 128;  // its two staged components fill 1 KB of shared memory a radial point
 
-// vel_transform + vel_nonlinear in three launches (five in mixed precision:
-// first the FP64 mean-mode sums, which also leave curl(u) in FP32 for the z
-// pass, last their reduction into the k=m=0 coefficients); CFL maxima per
-// radial point are left in ctx->cflmax.
-int pf_launch_nl_fused(pf_ctx *ctx) {
+// vel_transform + vel_nonlinear: curl(u) (PF_NL_STEPPED: left by the fused
+// predictor that made u), the three transform launches, and in mixed
+// precision the exact mean mode; PF_NL_SYM imposes the mean-mode symmetry on
+// u first.  CFL maxima per radial point are left in ctx->cflmax.
+int pf_launch_nl_fused(pf_ctx *ctx, int mode) {
     const NLArgs a = make_nl_args(ctx);
-    if (ctx->cfg.precision == PF_PREC_MIXED) {
+    const bool mixed = ctx->cfg.precision == PF_PREC_MIXED;
+    const int N = ctx->g.N;
+    if (mode != PF_NL_STEPPED && !mixed && N > PREP_MAX_N) {
+        if (mode == PF_NL_SYM) PF_TRY(pf_launch_imposesym(ctx, 0, ctx->vel[0].d, ctx->vel[1].d, ctx->vel[2].d));
+        PF_TRY(pf_launch_curl(ctx, ctx->vel[0].d, ctx->vel[1].d, ctx->vel[2].d, ctx->s[0].d, ctx->s[1].d, ctx->s[2].d));
+    } else if (mode != PF_NL_STEPPED) {
         {
-            ProfScope ps_(ctx, PF_K_ZINV);
-            PF_TRY(mean_attrs());
-            k_nl_mean64_part<<<(ctx->g.H + 31) / 32, MEAN_THREADS, mean_smem(ctx->g.N), ctx->stream>>>(a);
+            ProfScope ps_(ctx, PF_K_STENCIL);
+            PF_TRY(prep_attrs());
+            const int blocks = (ctx->g.H + 31) / 32, sym = mode == PF_NL_SYM;
+            if (mixed) k_nl_prep<true><<<blocks, PREP_THREADS, prep_smem(N), ctx->stream>>>(a, sym);
+            else k_nl_prep<false><<<blocks, PREP_THREADS, prep_smem(N), ctx->stream>>>(a, sym);
         }
         PF_LAUNCHED(ctx);
-        PF_TRY(launch_nl<float2>(ctx, a));
-        {
-            ProfScope ps_(ctx, PF_K_ZFWD);
-            k_nl_mean64_fin<<<(ctx->g.N + 3) / 4, 128, 0, ctx->stream>>>(a);
-        }
-        PF_LAUNCHED(ctx);
-        return PF_OK;
     }
-    return launch_nl<double2>(ctx, a);
+    if (!mixed) return launch_nl<double2>(ctx, a);
+    PF_TRY(launch_nl<float2>(ctx, a));
+    {
+        ProfScope ps_(ctx, PF_K_ZFWD);
+        k_nl_mean64_fin<<<(N + 3) / 4, 128, 0, ctx->stream>>>(a, mode == PF_NL_STEPPED);
+    }
+    PF_LAUNCHED(ctx);
+    return PF_OK;
 }
 
-
-// ------------------------------------------------- FP64 mean mode (mixed)
+// ----------------------------------------- curl(u) and the FP64 mean mode
+// One block per 32-mode chunk, u_t and u_z of those modes at every radial
+// point staged in shared memory (each value read from HBM once), one warp per
+// radial point at a time (lanes = modes): curl(u) (variables.f90:408-436) from
+// the staged rows, stored for the z pass.
+//
 // With FP32 transforms the k=m=0 coefficient of u x curl(u) is replaced by
 // its exact FP64 value.  On the 3/2-dealiased grid no product of retained
 // modes aliases onto (0,0), so the grid mean equals the spectral sum
 //   mean(f g) = Re f00 Re g00 + 2 sum_{k>=1} Re(f_k0 conj g_k0)
 //             + 2 sum_{m>=1, all k} Re(f_km conj g_km)
-// (the c2r transform ignores Im f00).  Two launches.  The first: one block
-// per 32-mode chunk, u_t and u_z of those modes at every radial point staged
-// in shared memory (each value read from HBM once), one warp per radial
-// point at a time (lanes = modes), the curl formed from the staged rows and
-// the chunk's sums written as partials.  The second: one warp per radial
-// point adds the chunks' partials in a fixed order.
-__device__ __forceinline__ void nl_mean64_part_body(const NLArgs &a, int chunk) {
+// (the c2r transform ignores Im f00): the chunk's sums go out as partials
+// here, and one warp per radial point adds the chunks' partials in a fixed
+// order afterwards.
+template <bool MIXED> __device__ __forceinline__ void nl_prep_body(const NLArgs &a, int chunk, int sym) {
     extern __shared__ double2 msm[];  // [2][N][32]: u_t, u_z of this chunk's modes
     const Geo &g = a.g;
     const int N = g.N, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int nh = chunk * 32 + lane;
-    const bool live = nh < g.H;
+    const bool live = nh < g.H, mean = sym && nh == 0;
     const size_t Hp = g.Hp;
     double2 *st = msm, *sz = msm + N * 32;
+#pragma unroll 4
     for (int n = warp; n < N; n += nw) {
         const size_t at = (size_t)n * Hp + nh;
-        st[n * 32 + lane] = live ? a.u[1][at] : make_double2(0.0, 0.0);
-        sz[n * 32 + lane] = live ? a.u[2][at] : make_double2(0.0, 0.0);
+        double2 t = live ? a.u[1][at] : make_double2(0.0, 0.0), z = live ? a.u[2][at] : make_double2(0.0, 0.0);
+        if (mean) {  // var_imposesym of the mean mode (variables.f90:611-616)
+            t.y = z.y = 0.0;
+            const_cast<double2 *>(a.u[0])[at] = make_double2(0.0, 0.0);
+            const_cast<double2 *>(a.u[1])[at] = t;
+            const_cast<double2 *>(a.u[2])[at] = z;
+        }
+        st[n * 32 + lane] = t;
+        sz[n * 32 + lane] = z;
     }
     __syncthreads();
     int k = 0, m = 0;
@@ -839,11 +815,12 @@ __device__ __forceinline__ void nl_mean64_part_body(const NLArgs &a, int chunk) 
     const double k1a1 = g.alpha * k;
     const double *__restrict__ drb = a.dm.dr;
     for (int n = warp; n < N; n += nw) {
-        double s0 = 0.0, s1 = 0.0, s2 = 0.0;
+        double s[3] = {0.0, 0.0, 0.0};
         if (live) {
-            const double2 ur = a.u[0][(size_t)n * Hp + nh], ut = st[n * 32 + lane], uz = sz[n * 32 + lane];
+            const size_t at = (size_t)n * Hp + nh;
+            const double2 ur = mean ? make_double2(0.0, 0.0) : a.u[0][at];
+            const double2 ut = st[n * 32 + lane], uz = sz[n * 32 + lane];
             const double rm1 = a.dm.rp[2 * N + n];
-            const double m1r1 = rm1 * g.Mp * m;
             const int lo = max(0, n - KL), hi = min(N - 1, n + KL);
             double2 dz = make_double2(0.0, 0.0), dt = dz;
             for (int j = lo; j <= hi; ++j) {  // d/dr of u_z and u_t (var_coll_meshmult)
@@ -854,40 +831,34 @@ __device__ __forceinline__ void nl_mean64_part_body(const NLArgs &a, int chunk) 
                 dt.x = fma(w, t.x, dt.x);
                 dt.y = fma(w, t.y, dt.y);
             }
-            // curl (variables.f90:408-436)
-            const double2 cr = make_double2(-uz.y * m1r1 + ut.y * k1a1, uz.x * m1r1 - ut.x * k1a1);
-            const double2 ct = make_double2(-ur.y * k1a1 - dz.x, ur.x * k1a1 - dz.y);
-            const double2 cz = make_double2(ut.x * rm1 + dt.x + ur.y * m1r1, ut.y * rm1 + dt.y - ur.x * m1r1);
-            if (a.curlf) {  // the z pass's FP32 inputs of the curl components
-                const size_t at = (size_t)n * Hp + nh, fs = (size_t)N * Hp;
-                a.curlf[at] = make_float2((float)cr.x, (float)cr.y);
-                a.curlf[fs + at] = make_float2((float)ct.x, (float)ct.y);
-                a.curlf[2 * fs + at] = make_float2((float)cz.x, (float)cz.y);
+            const Curl c = mode_curl(ur, ut, uz, dt, dz, rm1, rm1 * g.Mp * m, k1a1);
+            if (MIXED) {
+                reinterpret_cast<float2 *>(a.curl[0])[at] = make_float2((float)c.r.x, (float)c.r.y);
+                reinterpret_cast<float2 *>(a.curl[1])[at] = make_float2((float)c.t.x, (float)c.t.y);
+                reinterpret_cast<float2 *>(a.curl[2])[at] = make_float2((float)c.z.x, (float)c.z.y);
+                mean_terms(nh == 0, ur, ut, uz, c, s);
+            } else {
+                reinterpret_cast<double2 *>(a.curl[0])[at] = c.r;
+                reinterpret_cast<double2 *>(a.curl[1])[at] = c.t;
+                reinterpret_cast<double2 *>(a.curl[2])[at] = c.z;
             }
-            const double w = (nh == 0) ? 1.0 : 2.0;
-            auto dot = [&](double2 f, double2 h) { return nh == 0 ? f.x * h.x : f.x * h.x + f.y * h.y; };
-            s0 = w * (dot(ut, cz) - dot(uz, ct));
-            s1 = w * (dot(uz, cr) - dot(ur, cz));
-            s2 = w * (dot(ur, ct) - dot(ut, cr));
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-            s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-            s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-        }
-        if (lane == 0) {
-            double *dst = a.mpart + ((size_t)chunk * N + n) * 3;
-            dst[0] = s0;
-            dst[1] = s1;
-            dst[2] = s2;
+        if (MIXED) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q)
+                for (int o = 16; o > 0; o >>= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
+            if (lane == 0) {
+                double *dst = a.mpart + ((size_t)chunk * N + n) * 3;
+                for (int q = 0; q < 3; ++q) dst[q] = s[q];
+            }
         }
     }
 }
 
-__device__ __forceinline__ void nl_mean64_fin_body(const NLArgs &a, int n) {
+__device__ __forceinline__ void nl_mean64_fin_body(const NLArgs &a, int n, int stepped) {
     const Geo &g = a.g;
     const int lane = threadIdx.x & 31;
-    const int nchunk = (g.H + 31) / 32;
+    const int nchunk = stepped ? pf_step_tiles(g) : (g.H + 31) / 32;  // partials per step tile or per prep chunk
     double t[3] = {0.0, 0.0, 0.0};
     for (int c = lane; c < nchunk; c += 32) {
         const double *src = a.mpart + ((size_t)c * g.N + n) * 3;
@@ -915,12 +886,14 @@ __device__ __forceinline__ void nl_mean64_fin_body(const NLArgs &a, int n) {
     a.N[2][at] = make_double2(zr, (-a.dm.velUp[n]) * ur.y);
 }
 
-static size_t mean_smem(int N) { return (size_t)2 * N * 32 * sizeof(double2); }
-__global__ void __launch_bounds__(MEAN_THREADS) k_nl_mean64_part(NLArgs a) { nl_mean64_part_body(a, blockIdx.x); }
+static size_t prep_smem(int N) { return (size_t)2 * N * 32 * sizeof(double2); }
+template <bool MIXED> __global__ void __launch_bounds__(PREP_THREADS) k_nl_prep(NLArgs a, int sym) {
+    nl_prep_body<MIXED>(a, blockIdx.x, sym);
+}
 // one warp per radial point
-__global__ void __launch_bounds__(128) k_nl_mean64_fin(NLArgs a) {
+__global__ void __launch_bounds__(128) k_nl_mean64_fin(NLArgs a, int stepped) {
     const int n = blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (n < a.g.N) nl_mean64_fin_body(a, n);
+    if (n < a.g.N) nl_mean64_fin_body(a, n, stepped);
 }
 
 // ------------------------------------------------------------------ batched
@@ -961,18 +934,20 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_nl_fused_b(const NLArgs *_
     nl_fused_body<ZL, TL>(a, pb.y);
 }
 
-__global__ void __launch_bounds__(MEAN_THREADS) k_nl_mean64_part_batch(const NLArgs *__restrict__ args,
-                                                                      const int2 *__restrict__ blk) {
+// the chunks of every pipe of either precision (nfp64: of the FP64 pipes)
+__global__ void __launch_bounds__(PREP_THREADS) k_nl_prep_batch(const NLArgs *__restrict__ args,
+                                                               const int2 *__restrict__ blk, int nfp64, int sym) {
     const int2 pb = blk[blockIdx.x];
     const NLArgs a = args[pb.x];
-    nl_mean64_part_body(a, pb.y);
+    if ((int)blockIdx.x < nfp64) nl_prep_body<false>(a, pb.y, sym);
+    else nl_prep_body<true>(a, pb.y, sym);
 }
 __global__ void __launch_bounds__(128) k_nl_mean64_fin_batch(const NLArgs *__restrict__ args,
-                                                            const int2 *__restrict__ blk) {
+                                                            const int2 *__restrict__ blk, int stepped) {
     const int2 pb = blk[blockIdx.x];
     const NLArgs a = args[pb.x];
     const int n = pb.y * 4 + (threadIdx.x >> 5);
-    if (n < a.g.N) nl_mean64_fin_body(a, n);
+    if (n < a.g.N) nl_mean64_fin_body(a, n, stepped);
 }
 
 // ------------------------------------------------- work-list stage kernels
@@ -1053,16 +1028,11 @@ __global__ void __launch_bounds__(NL_THREADS, ST == 1 ? 6 : 5)
     }
 }
 
-// shared-memory limit of the mean-mode partial-sum kernels (up to N = 128)
-static int mean_attrs() {
-    static bool set = false;
-    if (!set) {
-        const int bytes = (int)mean_smem(128);
-        PF_CUDA(cudaFuncSetAttribute(k_nl_mean64_part, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-        PF_CUDA(cudaFuncSetAttribute(k_nl_mean64_part_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-        set = true;
-    }
-    return PF_OK;
+// shared-memory limit of the prep kernels
+static int prep_attrs() {
+    PF_TRY(pf_raise_smem((const void *)k_nl_prep<true>, prep_smem(PREP_MAX_N)));
+    PF_TRY(pf_raise_smem((const void *)k_nl_prep<false>, prep_smem(PREP_MAX_N)));
+    return pf_raise_smem((const void *)k_nl_prep_batch, prep_smem(PREP_MAX_N));
 }
 
 namespace {
@@ -1082,9 +1052,9 @@ struct pf_nl_batch {
     int n;
     NLArgs *d_args[2];  // [pointer state]: 0 = as built, 1 = vel/prev swapped
     std::vector<NLGroup> groups[NLB_STAGES];
-    int2 *mean_blk, *fin_blk;  // FP64 mean mode of the mixed-precision pipes: chunks, radial points
-    int nmean, nfin;
-    size_t mean_sm;
+    int2 *prep_blk, *fin_blk;  // prep chunks of the FP64 pipes, then of the mixed ones; the mixed ones' radial points
+    int nprep, nprep64, nfin;
+    size_t prep_sm;
     cudaStream_t aux[NLB_MAXG];
     cudaEvent_t fork[NLB_STAGES], join[NLB_STAGES][NLB_MAXG];
     // pipes whose transforms run one block per radial point, one group per
@@ -1117,7 +1087,7 @@ void pf_nl_batch_free(pf_nl_batch *b) {
         for (int k = 0; k < NLB_MAXG; ++k)
             if (b->join[st][k]) cudaEventDestroy(b->join[st][k]);
     }
-    cudaFree(b->mean_blk);
+    cudaFree(b->prep_blk);
     cudaFree(b->fin_blk);
     for (int st = 0; st < NLB_STAGES; ++st) cudaFree(b->wl_items[st]);
     cudaFree(b->wl_ctr);
@@ -1215,18 +1185,22 @@ static int nlb_groups(pf_nl_batch *b, pf_ctx *const *pipes, int n) {
             PF_TRY(upload(&b->fgroups.back().blk, map));
         }
     }
-    std::vector<int2> mean, fin;
-    b->mean_sm = 0;
-    for (int i = 0; i < n; ++i)
-        if (is_mixed(pipes[i])) {
+    std::vector<int2> prep, fin;
+    b->prep_sm = 0;
+    for (const bool mixed : {false, true}) {
+        for (int i = 0; i < n; ++i) {
             const Geo &g = pipes[i]->g;
-            for (int l = 0; l < (g.H + 31) / 32; ++l) mean.push_back(make_int2(i, l));
-            for (int l = 0; l < (g.N + 3) / 4; ++l) fin.push_back(make_int2(i, l));
-            b->mean_sm = std::max(b->mean_sm, mean_smem(g.N));
+            if (is_mixed(pipes[i]) != mixed) continue;
+            for (int l = 0; l < (g.H + 31) / 32; ++l) prep.push_back(make_int2(i, l));
+            if (mixed)
+                for (int l = 0; l < (g.N + 3) / 4; ++l) fin.push_back(make_int2(i, l));
+            b->prep_sm = std::max(b->prep_sm, prep_smem(g.N));
         }
-    b->nmean = (int)mean.size();
+        if (!mixed) b->nprep64 = (int)prep.size();
+    }
+    b->nprep = (int)prep.size();
     b->nfin = (int)fin.size();
-    PF_TRY(upload(&b->mean_blk, mean));
+    PF_TRY(upload(&b->prep_blk, prep));
     return upload(&b->fin_blk, fin);
 }
 
@@ -1389,41 +1363,41 @@ static int nlb_stage(pf_nl_batch *b, int stage, const NLArgs *args, cudaStream_t
     return PF_OK;
 }
 
-// vel_transform + vel_nonlinear of every pipe: one launch per stage and
-// (transform length, precision) group, plus the FP64 mean-mode launch when
-// any pipe is in mixed precision; launches are counted into *nk.  state 0:
-// the pointers the pipes held when the batch was built; 1: vel/prev swapped.
-int pf_nl_batch_launch(pf_nl_batch *b, int state, cudaStream_t st, pf_stage_prof *prof, unsigned long long *nk) {
+// vel_transform + vel_nonlinear of every pipe: curl(u) unless the fused
+// predictor left it (mode as in pf_launch_nl_fused), one launch per stage and
+// (transform length, precision) group, and the mean mode of the pipes in mixed
+// precision; launches are counted into *nk.  state 0: the pointers the pipes
+// held when the batch was built; 1: vel/prev swapped.
+int pf_nl_batch_launch(pf_nl_batch *b, int state, int mode, cudaStream_t st, pf_stage_prof *prof,
+                       unsigned long long *nk) {
     const NLArgs *args = b->d_args[state];
     const int cats[NLB_STAGES] = {PF_K_ZINV, PF_K_THFWD, PF_K_ZFWD};
-    // mixed precision: the FP64 mean-mode sums first; they leave curl(u) in
-    // FP32 for the z pass
-    if (b->nmean > 0) {
-        StageScope ss_(prof, PF_K_ZINV, st);
-        PF_TRY(mean_attrs());
-        k_nl_mean64_part_batch<<<b->nmean, MEAN_THREADS, b->mean_sm, st>>>(args, b->mean_blk);
+    if (mode != PF_NL_STEPPED) {
+        StageScope ss_(prof, PF_K_STENCIL, st);
+        PF_TRY(prep_attrs());
+        k_nl_prep_batch<<<b->nprep, PREP_THREADS, b->prep_sm, st>>>(args, b->prep_blk, b->nprep64, mode == PF_NL_SYM);
         PF_CHECK_LAUNCH();
         *nk += 1;
-        // the pipes done one block per radial point, beside the three passes
-        // of the others (they need the mean-mode pass's FP32 curl)
-        if (!b->fgroups.empty()) {
-            PF_CUDA(cudaEventRecord(b->ffork, st));
-            for (size_t k = 0; k < b->fgroups.size(); ++k) {
-                PF_CUDA(cudaStreamWaitEvent(b->faux[k], b->ffork, 0));
-                PF_TRY(nlb_fused_launch(b->fgroups[k], args, b->faux[k]));
-                PF_CUDA(cudaEventRecord(b->fjoin[k], b->faux[k]));
-                ++*nk;
-            }
+    }
+    // the pipes done one block per radial point, beside the three passes of
+    // the others
+    if (!b->fgroups.empty()) {
+        PF_CUDA(cudaEventRecord(b->ffork, st));
+        for (size_t k = 0; k < b->fgroups.size(); ++k) {
+            PF_CUDA(cudaStreamWaitEvent(b->faux[k], b->ffork, 0));
+            PF_TRY(nlb_fused_launch(b->fgroups[k], args, b->faux[k]));
+            PF_CUDA(cudaEventRecord(b->fjoin[k], b->faux[k]));
+            ++*nk;
         }
     }
     for (int stage = 0; stage < NLB_STAGES; ++stage) {
         StageScope ss_(prof, cats[stage], st);
         PF_TRY(nlb_stage(b, stage, args, st, nk));
     }
-    if (b->nmean > 0) {
+    for (size_t k = 0; k < b->fgroups.size(); ++k) PF_CUDA(cudaStreamWaitEvent(st, b->fjoin[k], 0));
+    if (b->nfin > 0) {
         StageScope ss_(prof, PF_K_ZFWD, st);
-        for (size_t k = 0; k < b->fgroups.size(); ++k) PF_CUDA(cudaStreamWaitEvent(st, b->fjoin[k], 0));
-        k_nl_mean64_fin_batch<<<b->nfin, 128, 0, st>>>(args, b->fin_blk);
+        k_nl_mean64_fin_batch<<<b->nfin, 128, 0, st>>>(args, b->fin_blk, mode == PF_NL_STEPPED);
         PF_CHECK_LAUNCH();
         *nk += 1;
     }

@@ -28,6 +28,9 @@ struct StepArgs {
     const double *lnp, *ld[3];  // factor tiles of LNp, LDp, LDm, LDz
     int ldpiv[3];          // 1 if that Helmholtz factorisation pivoted
     const double *U, *Ainv, *Ui;
+    void *curl[3];         // curl(u) for the nonlinear terms that follow a predictor (null: not wanted),
+    int mixed;             // FP32 (mixed precision) or FP64,
+    double *mpart;         // and in mixed precision the mean mode's partial sums [tile][N][3]
     DevMesh dm;
     Geo g;
     double c1, c2;         // Lt coefficients: 1/dt and (1-implicit) nu/Re
@@ -602,8 +605,47 @@ __device__ __forceinline__ void step_tile(const StepArgs &a, int tile, const Ste
             u0[at] = ur;
             u1[at] = ut;
             u2[at] = zz;
+            b0[n * 16] = ur;
+            b1[n * 16] = ut;
+            b2[n * 16] = zz;
         }
         if (zero && ty == 0 && a.const_flux) a.sc->Pr0 = a.sc->Pr0 + d3 * g.Re / 4.0;
+    }
+    if (a.mode == 0 && a.curl[0]) {
+        // curl(u) and the mean mode's sums over this tile (k_nl_prep's, while
+        // u is still on the chip)
+        next.load(drb, N, ty);
+        __syncthreads();
+#pragma unroll 1
+        for (int n = ty; n < ((N + 1) & ~1); n += NR) {  // whole warps: the half-warps sum together
+            const BandRow row = next;
+            next.load(drb, N, n + NR);
+            double s[3] = {0.0, 0.0, 0.0};
+            if (live && n < N) {
+                const size_t at = (size_t)n * Hp + nh;
+                const double2 dt = row.apply(N, n, b1), dz = row.apply(N, n, b2);
+                const double2 ur = b0[n * 16], ut = b1[n * 16], uz = b2[n * 16];
+                const double rm1 = rp[2 * N + n];
+                const Curl c = mode_curl(ur, ut, uz, dt, dz, rm1, rm1 * mMp, kal);
+                if (a.mixed) {
+                    reinterpret_cast<float2 *>(a.curl[0])[at] = make_float2((float)c.r.x, (float)c.r.y);
+                    reinterpret_cast<float2 *>(a.curl[1])[at] = make_float2((float)c.t.x, (float)c.t.y);
+                    reinterpret_cast<float2 *>(a.curl[2])[at] = make_float2((float)c.z.x, (float)c.z.y);
+                    mean_terms(nh == 0, ur, ut, uz, c, s);
+                } else {
+                    reinterpret_cast<double2 *>(a.curl[0])[at] = c.r;
+                    reinterpret_cast<double2 *>(a.curl[1])[at] = c.t;
+                    reinterpret_cast<double2 *>(a.curl[2])[at] = c.z;
+                }
+            }
+            if (a.mixed) {
+#pragma unroll
+                for (int q = 0; q < 3; ++q)
+                    for (int o = 8; o > 0; o >>= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
+                if (slot == 0 && n < N)
+                    for (int q = 0; q < 3; ++q) a.mpart[((size_t)tile * N + n) * 3 + q] = s[q];
+            }
+        }
     }
     if (a.mode == 1) {
         // one atomic per block; the pipe's last block publishes the maximum
@@ -686,6 +728,10 @@ static StepArgs make_step_args(const pf_ctx *ctx, int corrector) {
         a.ld[i] = ld[i]->tiles;
         a.ldpiv[i] = ld[i]->pivoted;
     }
+    const bool follow = pf_nl_fused_supported(ctx) && !pf_util_active(ctx);  // the transforms that read curl(u)
+    for (int i = 0; i < 3; ++i) a.curl[i] = follow ? pf_curl_field(ctx, i) : nullptr;
+    a.mixed = ctx->cfg.precision == PF_PREC_MIXED;
+    a.mpart = ctx->mpart;
     a.U = ctx->U;
     a.Ainv = ctx->Ainv;
     a.Ui = ctx->Ui;

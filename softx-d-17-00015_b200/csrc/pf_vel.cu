@@ -132,17 +132,26 @@ extern "C" int pf_vel_corrector(pf_ctx *ctx) {
 
 // vel_transform + vel_nonlinear for the drivers: the fused three-launch
 // path when the transform lengths are instantiated, else the materialising one
-int pf_transform_nonlinear(pf_ctx *ctx);
-static int transform_nonlinear(pf_ctx *ctx) { return pf_transform_nonlinear(ctx); }
-int pf_transform_nonlinear(pf_ctx *ctx) {
+static int transform_nonlinear(pf_ctx *ctx, int mode) {
     if (pf_nl_fused_supported(ctx)) {
-        PF_TRY(pf_launch_nl_fused(ctx));
+        PF_TRY(pf_launch_nl_fused(ctx, mode));
         ctx->cfl_fused = true;
         return PF_OK;
     }
+    if (mode == PF_NL_SYM) PF_TRY(pf_vel_imposesym(ctx));
     PF_TRY(pf_vel_transform(ctx));
     return pf_vel_nonlinear(ctx);
 }
+int pf_transform_nonlinear(pf_ctx *ctx) { return transform_nonlinear(ctx, PF_NL_FRESH); }
+// vel_imposesym, then the terms; the mean-mode symmetry alone rides in the
+// kernel that forms curl(u)
+int pf_first_nonlinear(pf_ctx *ctx) {
+    if (!(ctx->cfg.mirrorsym || ctx->cfg.shiftrefl || ctx->cfg.shiftrott)) return transform_nonlinear(ctx, PF_NL_SYM);
+    PF_TRY(pf_vel_imposesym(ctx));
+    return transform_nonlinear(ctx, PF_NL_FRESH);
+}
+// the terms of the velocity a predictor has just made
+int pf_next_nonlinear(pf_ctx *ctx) { return transform_nonlinear(ctx, fused_step_ok(ctx) ? PF_NL_STEPPED : PF_NL_FRESH); }
 
 extern "C" int pf_vel_transform_nonlinear(pf_ctx *ctx) {
     PF_ARG(ctx, "null ctx");
@@ -279,8 +288,11 @@ static bool graphs_ok(const pf_ctx *ctx) {
 // vel_transform + vel_nonlinear + var_null(2) of the main loop (main.f90:21-23,
 // 36-38): with a plug-in the physical fields vel_r .. vel_curlz are made, as
 // the plug-ins read them
-static int main_nonlinear(pf_ctx *ctx) {
-    if (!pf_util_active(ctx)) return transform_nonlinear(ctx);
+enum { NL_FIRST, NL_NEXT, NL_AGAIN };  // before the predictor (with imposesym), after it, after a corrector
+static int main_nonlinear(pf_ctx *ctx, int when) {
+    if (!pf_util_active(ctx))
+        return when == NL_FIRST ? pf_first_nonlinear(ctx) : when == NL_NEXT ? pf_next_nonlinear(ctx) : pf_transform_nonlinear(ctx);
+    if (when == NL_FIRST) PF_TRY(pf_vel_imposesym(ctx));
     PF_TRY(pf_vel_transform(ctx));
     PF_TRY(pf_vel_nonlinear(ctx));
     return pf_util_run(ctx, 2);
@@ -302,10 +314,9 @@ extern "C" int pf_timestep(pf_ctx *ctx, int *ncorr) {
             // nonlinear evaluation inside the graph (its var_null(1) does
             // nothing on the device)
             PF_TRY(capture(ctx, p, &ctx->g_main[p], &ctx->g_main_n[p], [&]() {
-                PF_TRY(pf_vel_imposesym(ctx));
-                PF_TRY(main_nonlinear(ctx));
+                PF_TRY(main_nonlinear(ctx, NL_FIRST));
                 PF_TRY(pf_vel_step_fused(ctx, 0));
-                PF_TRY(main_nonlinear(ctx));
+                PF_TRY(main_nonlinear(ctx, NL_NEXT));
                 return pf_vel_step_fused(ctx, 1);
             }));
             // capture swapped the host pointers; the replay below does it for real
@@ -326,14 +337,13 @@ extern "C" int pf_timestep(pf_ctx *ctx, int *ncorr) {
             const int q = ctx->parity;
             if (!ctx->g_corr[q])
                 PF_TRY(capture(ctx, 2 + q, &ctx->g_corr[q], &ctx->g_corr_n[q], [&]() {
-                    PF_TRY(main_nonlinear(ctx));
+                    PF_TRY(main_nonlinear(ctx, NL_AGAIN));
                     return pf_vel_step_fused(ctx, 1);
                 }));
             PF_TRY(replay(ctx, 2 + q, ctx->g_corr[q], ctx->g_corr_n[q]));
         }
     } else {
-        PF_TRY(pf_vel_imposesym(ctx));
-        PF_TRY(main_nonlinear(ctx));
+        PF_TRY(main_nonlinear(ctx, NL_FIRST));
         if (ctx->cfg.dt < 0.0) {
             PF_TRY(pf_vel_maxtstep(ctx));
             PF_TRY(pf_tim_new_tstep(ctx));
@@ -343,7 +353,7 @@ extern "C" int pf_timestep(pf_ctx *ctx, int *ncorr) {
         PF_TRY(pf_vel_predictor(ctx));
         ctx->tim.it = 1;
         while (ctx->tim.it != 0) {
-            PF_TRY(main_nonlinear(ctx));
+            PF_TRY(main_nonlinear(ctx, nc == 0 ? NL_NEXT : NL_AGAIN));
             PF_TRY(pf_vel_corrector(ctx));
             const int s = pf_tim_check_cgce(ctx);
             if (s != PF_OK) status = s;
@@ -362,10 +372,9 @@ extern "C" int pf_steporbit(pf_ctx *ctx, int nsteps) {
     PF_ARG(ctx && nsteps >= 0, "pf_steporbit: bad argument");
     PF_TRY(require_matrices(ctx));
     for (int s = 0; s < nsteps; ++s) {
-        PF_TRY(pf_vel_imposesym(ctx));
-        PF_TRY(transform_nonlinear(ctx));
+        PF_TRY(pf_first_nonlinear(ctx));
         PF_TRY(pf_vel_predictor(ctx));
-        PF_TRY(transform_nonlinear(ctx));
+        PF_TRY(pf_next_nonlinear(ctx));
         PF_TRY(vel_corrector_async(ctx));
         PF_TRY(pf_vel_imposesym(ctx));
         ctx->tim.t = ctx->tim.t + ctx->tim.dt;
