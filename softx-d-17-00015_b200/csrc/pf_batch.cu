@@ -82,6 +82,7 @@ struct pf_batch {
     SymArgs *d_sym[2];               // [pointer state]
     DevScalars **d_scp;              // each pipe's device scalars
     DevScalars *d_scall;             // gathered scalars
+    int *d_act, *h_act;              // mask of a further corrector pass (h_act pinned)
     pf_stage_prof sprof;             // stage timing of the batched launches
     std::vector<pf_stage_prof::Open> sev[2][2];
     unsigned long long launches;     // batched kernels launched (not per pipe)
@@ -98,6 +99,9 @@ static void staged_free(pf_batch *b) {
         cudaFree(b->d_sym[s]);
         b->d_sym[s] = nullptr;
     }
+    cudaFree(b->d_act);
+    if (b->h_act) cudaFreeHost(b->h_act);
+    b->d_act = b->h_act = nullptr;
     cudaFree(b->d_scp);
     cudaFree(b->d_scall);
     b->d_scp = nullptr;
@@ -333,6 +337,18 @@ static int staged_build(pf_batch *b) {
     return PF_OK;
 }
 
+// every pipe's device scalars to pinned host memory
+static int staged_scalars(pf_batch *b, pf_stage_prof *pr, unsigned long long *nk) {
+    {
+        StageScope ss_(pr, PF_K_EW, b->master);
+        k_batch_scalars<<<grid1(b->n, 128), 128, 0, b->master>>>(b->d_scp, b->d_scall, b->n);
+    }
+    PF_CHECK_LAUNCH();
+    ++*nk;
+    PF_CUDA(cudaMemcpyAsync(b->hsc, b->d_scall, b->n * sizeof(DevScalars), cudaMemcpyDeviceToHost, b->master));
+    return PF_OK;
+}
+
 // The stage-batched step: imposesym, nonlinear terms, predictor, nonlinear
 // terms, corrector (and imposesym in orbit mode) of every pipe, then the
 // gathered device scalars to pinned host memory.
@@ -340,10 +356,10 @@ static int staged_body(pf_batch *b, int orbit, int par, unsigned long long *nk) 
     const int s0 = par ^ b->par0, s1 = s0 ^ 1;  // pointer state before / after the predictor's swap
     cudaStream_t st = b->master;
     pf_stage_prof *pr = &b->sprof;
-    PF_TRY(pf_nl_batch_launch(b->nlb, s0, PF_NL_SYM, st, pr, nk));
-    PF_TRY(pf_step_batch_launch(b->stb, s1, 0, st, pr, nk));
-    PF_TRY(pf_nl_batch_launch(b->nlb, s1, PF_NL_STEPPED, st, pr, nk));
-    PF_TRY(pf_step_batch_launch(b->stb, s1, 1, st, pr, nk));
+    PF_TRY(pf_nl_batch_launch(b->nlb, s0, PF_NL_SYM, nullptr, st, pr, nk));
+    PF_TRY(pf_step_batch_launch(b->stb, s1, 0, nullptr, st, pr, nk));
+    PF_TRY(pf_nl_batch_launch(b->nlb, s1, PF_NL_STEPPED, nullptr, st, pr, nk));
+    PF_TRY(pf_step_batch_launch(b->stb, s1, 1, nullptr, st, pr, nk));
     if (orbit) {
         {
             StageScope ss_(pr, PF_K_EW, st);
@@ -352,14 +368,18 @@ static int staged_body(pf_batch *b, int orbit, int par, unsigned long long *nk) 
         PF_CHECK_LAUNCH();
         ++*nk;
     }
-    {
-        StageScope ss_(pr, PF_K_EW, st);
-        k_batch_scalars<<<grid1(b->n, 128), 128, 0, st>>>(b->d_scp, b->d_scall, b->n);
-    }
-    PF_CHECK_LAUNCH();
-    ++*nk;
-    PF_CUDA(cudaMemcpyAsync(b->hsc, b->d_scall, b->n * sizeof(DevScalars), cudaMemcpyDeviceToHost, st));
-    return PF_OK;
+    return staged_scalars(b, pr, nk);
+}
+
+// A further corrector pass (main.f90:35-41) of the pipes in the mask h_act,
+// as one launch per stage over them; the other pipes' blocks leave at once.
+static int staged_corrector(pf_batch *b, int par, unsigned long long *nk) {
+    const int s = par ^ b->par0;
+    pf_stage_prof *pr = &b->sprof;
+    PF_CUDA(cudaMemcpyAsync(b->d_act, b->h_act, b->n * sizeof(int), cudaMemcpyHostToDevice, b->master));
+    PF_TRY(pf_nl_batch_launch(b->nlb, s, PF_NL_FRESH, b->d_act, b->master, pr, nk));
+    PF_TRY(pf_step_batch_launch(b->stb, s, 1, b->d_act, b->master, pr, nk));
+    return staged_scalars(b, pr, nk);
 }
 
 static int staged_capture(pf_batch *b, int orbit, int par, cudaGraphExec_t *exec, unsigned long long *nk) {
@@ -458,57 +478,6 @@ static std::vector<int> rel_parity(const pf_batch *b) {
     return r;
 }
 
-// Corrector control after a batched step (timestep.f90:214-253, main.f90:35-41)
-// from the scalars the step left in b->hsc; returns the passes taken.
-static long long batch_after_step(pf_batch *b, int orbit, int *status) {
-    long long passes = 0;
-    for (int i = 0; i < b->n; ++i) {
-        pf_ctx *c = b->pipes[i];
-        const double err2 = bits_to_double(b->hsc[i].dterr2_bits);
-        if (pf_step_status(b->hsc[i]) != PF_OK) *status = PF_ERR_CUDA;
-        c->tim.dterr = std::max(c->tim.dterr, std::sqrt(err2));
-        c->tim.it = 1;
-        c->last_status = PF_OK;
-        c->last_error.clear();
-        int s = pf_tim_check_cgce(c);
-        if (s != PF_OK) {
-            c->last_status = s;
-            c->last_error = pf_last_error();
-        }
-        // the state went non-finite: the max of the corrections' bit patterns
-        // is a NaN or Inf pattern (the reference would carry on with NaN)
-        if (!std::isfinite(err2) && c->last_status == PF_OK) {
-            c->last_status = PF_ERR_CONVERGE;
-            c->last_error = "non-finite corrector error: NaN or Inf in the state";
-        }
-        ++passes;
-        if (!orbit) {
-            while (c->tim.it != 0) {  // further corrector passes for this pipe only
-                int e = pf_transform_nonlinear(c);
-                if (e == PF_OK) e = pf_vel_step_fused(c, 1);
-                if (e == PF_OK) e = pf_read_dterr(c);
-                if (e != PF_OK) {
-                    *status = e;
-                    c->tim.it = 0;
-                    break;
-                }
-                s = pf_tim_check_cgce(c);
-                if (s != PF_OK && c->last_status == PF_OK) {
-                    c->last_status = s;
-                    c->last_error = pf_last_error();
-                }
-                ++passes;
-            }
-            if (s != PF_OK) *status = s;
-        } else {
-            c->tim.it = 0;
-        }
-        c->tim.t = c->tim.t + c->tim.dt;
-        c->tim.step = c->tim.step + 1;
-    }
-    return passes;
-}
-
 // Read the stage and kernel event pairs of a finished step into the totals.
 static void batch_collect_events(pf_batch *b, std::vector<pf_stage_prof::Open> *stage, bool release) {
     for (auto &e : *stage) {
@@ -525,6 +494,100 @@ static void batch_collect_events(pf_batch *b, std::vector<pf_stage_prof::Open> *
         }
     }
     if (release) stage->clear();
+}
+
+// One further corrector pass of every pipe in `act` (indexes), its scalars in
+// b->hsc.  Stage-batched: one masked launch per stage; a chain of small launches per pipe that
+// waited for the GPU each time was half of a step in which 39 of 64 mixed pipes
+// take a second pass (two such steps: 16.6 -> 10.9 ms).  Launched directly: recording
+// it costs the first pass of a batch more than a replay saves (8 FP64 pipes, a
+// new batch's first steps: 6.4 ms recorded, 5.1 ms direct; repeated 1.44-1.6).  Otherwise every pipe's pass on its own stream, all in flight together.
+static int batch_corrector(pf_batch *b, const std::vector<int> &act) {
+    if (b->kind != 1) {
+        for (int i : act) {
+            pf_ctx *c = b->pipes[i];
+            PF_TRY(pf_transform_nonlinear(c));
+            PF_TRY(pf_vel_step_fused(c, 1));
+            PF_CUDA(cudaMemcpyAsync(&b->hsc[i], c->dsc, sizeof(DevScalars), cudaMemcpyDeviceToHost, c->stream));
+        }
+        for (int i : act) {
+            PF_CUDA(cudaStreamSynchronize(b->pipes[i]->stream));
+            pf_graph_events_collect(b->pipes[i]);
+        }
+        return PF_OK;
+    }
+    if (!b->d_act) PF_CUDA(cudaMalloc((void **)&b->d_act, b->n * sizeof(int)));
+    if (!b->h_act) PF_CUDA(cudaMallocHost((void **)&b->h_act, b->n * sizeof(int)));
+    for (int i = 0; i < b->n; ++i) b->h_act[i] = 0;
+    for (int i : act) b->h_act[i] = 1;
+    const int p = b->pipes[0]->parity;
+    const size_t open0 = b->sprof.open.size();
+    PF_TRY(staged_corrector(b, b->pipes[0]->parity, &b->launches));
+    PF_CUDA(cudaStreamSynchronize(b->master));
+    std::vector<pf_stage_prof::Open> mine(b->sprof.open.begin() + open0, b->sprof.open.end());
+    b->sprof.open.resize(open0);
+    batch_collect_events(b, &mine, true);
+    return PF_OK;
+}
+
+// Corrector control after a batched step (timestep.f90:214-253, main.f90:35-41)
+// from the scalars the step left in b->hsc; returns the passes taken.
+static long long batch_after_step(pf_batch *b, int orbit, int *status) {
+    long long passes = 0;
+    std::vector<int> act;
+    for (int i = 0; i < b->n; ++i) {
+        pf_ctx *c = b->pipes[i];
+        c->tim.it = 1;
+        c->last_status = PF_OK;
+        c->last_error.clear();
+        act.push_back(i);
+    }
+    for (bool first = true; !act.empty(); first = false) {
+        if (!first) {
+            const int e = batch_corrector(b, act);
+            if (e != PF_OK) {
+                *status = e;
+                for (int i : act) b->pipes[i]->tim.it = 0;
+                break;
+            }
+        }
+        std::vector<int> again;
+        for (int i : act) {
+            pf_ctx *c = b->pipes[i];
+            const double err2 = bits_to_double(b->hsc[i].dterr2_bits);
+            if (pf_step_status(b->hsc[i]) != PF_OK) {
+                *status = PF_ERR_CUDA;
+                if (!first) {
+                    c->tim.it = 0;
+                    continue;
+                }
+            }
+            c->tim.dterr = std::max(c->tim.dterr, std::sqrt(err2));
+            const int s = pf_tim_check_cgce(c);
+            if (s != PF_OK) {
+                if (c->last_status == PF_OK) {
+                    c->last_status = s;
+                    c->last_error = pf_last_error();
+                }
+                if (!orbit) *status = s;
+            }
+            // the state went non-finite: the max of the corrections' bit patterns
+            // is a NaN or Inf pattern (the reference would carry on with NaN)
+            if (first && !std::isfinite(err2) && c->last_status == PF_OK) {
+                c->last_status = PF_ERR_CONVERGE;
+                c->last_error = "non-finite corrector error: NaN or Inf in the state";
+            }
+            ++passes;
+            if (orbit) c->tim.it = 0;
+            if (c->tim.it != 0) again.push_back(i);
+        }
+        act.swap(again);
+    }
+    for (pf_ctx *c : b->pipes) {
+        c->tim.t = c->tim.t + c->tim.dt;
+        c->tim.step = c->tim.step + 1;
+    }
+    return passes;
 }
 
 // Advance every pipe by nsteps timesteps.  orbit=0: the main.f90 step with

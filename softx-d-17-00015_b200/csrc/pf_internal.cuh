@@ -448,7 +448,7 @@ struct StageScope {
 struct pf_nl_batch;
 bool pf_nl_batch_supported(pf_ctx *const *pipes, int n);
 int pf_nl_batch_build(pf_ctx *const *pipes, int n, bool worklist, pf_nl_batch **out);
-int pf_nl_batch_launch(pf_nl_batch *b, int state, int mode, cudaStream_t st, pf_stage_prof *prof,
+int pf_nl_batch_launch(pf_nl_batch *b, int state, int mode, const int *act, cudaStream_t st, pf_stage_prof *prof,
                        unsigned long long *nk);
 void pf_nl_batch_free(pf_nl_batch *b);
 // Streams onto which a batch forks the concurrent launches of a stage, and
@@ -483,8 +483,8 @@ struct pf_aux {
 };
 struct pf_step_batch;
 int pf_step_batch_build(pf_ctx *const *pipes, int n, pf_aux *aux, pf_step_batch **out);
-int pf_step_batch_launch(pf_step_batch *b, int state, int corrector, cudaStream_t st, pf_stage_prof *prof,
-                         unsigned long long *nk);
+int pf_step_batch_launch(pf_step_batch *b, int state, int corrector, const int *act, cudaStream_t st,
+                         pf_stage_prof *prof, unsigned long long *nk);
 void pf_step_batch_free(pf_step_batch *b);
 // What the nonlinear terms start from: u alone, u with the mean-mode symmetry
 // still to be imposed, or what a fused predictor has just left (u and its

@@ -899,28 +899,33 @@ __global__ void __launch_bounds__(128) k_nl_mean64_fin(NLArgs a, int stepped) {
 // ------------------------------------------------------------------ batched
 // One launch per (stage, transform length) covers the blocks of every pipe
 // of a batch with that length: blk[b] = (pipe, block index within that pipe's
-// own grid), and each block runs the lone-pipe body.  The launches of one
+// own grid), and each block runs the lone-pipe body; with a mask `act`, only
+// the blocks of the pipes it names (a further corrector pass of some of the
+// batch).  The launches of one
 // stage for different lengths are independent and run concurrently (forked
 // onto auxiliary streams, joined before the next stage).
 template <int ZL, typename C>
-__global__ void __launch_bounds__(NL_THREADS, (NLOcc<C, ZL>::zinv)) k_nl_zinv_b(const NLArgs *__restrict__ args, const int2 *__restrict__ blk) {
+__global__ void __launch_bounds__(NL_THREADS, (NLOcc<C, ZL>::zinv)) k_nl_zinv_b(const NLArgs *__restrict__ args, const int2 *__restrict__ blk, const int *__restrict__ act) {
     const int2 pb = blk[blockIdx.x];
+    if (act && !act[pb.x]) return;
     const NLArgs a = args[pb.x];  // by value: stores through its pointers cannot alias it
     const int gx = (a.g.M + a.MC - 1) / a.MC;
     nl_zinv_body<ZL, C>(a, pb.y % gx, (pb.y / gx) % a.g.N, pb.y / (gx * a.g.N));
 }
 
 template <int TL, typename C>
-__global__ void __launch_bounds__(NL_THREADS, (NLOcc<C, TL>::theta)) k_nl_theta_b(const NLArgs *__restrict__ args, const int2 *__restrict__ blk) {
+__global__ void __launch_bounds__(NL_THREADS, (NLOcc<C, TL>::theta)) k_nl_theta_b(const NLArgs *__restrict__ args, const int2 *__restrict__ blk, const int *__restrict__ act) {
     const int2 pb = blk[blockIdx.x];
+    if (act && !act[pb.x]) return;
     const NLArgs a = args[pb.x];
     const int gx = (a.g.Z + a.ZC - 1) / a.ZC;
     nl_theta_body<TL, C>(a, pb.y % gx, pb.y / gx);
 }
 
 template <int ZL, typename C>
-__global__ void __launch_bounds__(NL_THREADS, (NLOcc<C, ZL>::zfwd)) k_nl_zfwd_b(const NLArgs *__restrict__ args, const int2 *__restrict__ blk) {
+__global__ void __launch_bounds__(NL_THREADS, (NLOcc<C, ZL>::zfwd)) k_nl_zfwd_b(const NLArgs *__restrict__ args, const int2 *__restrict__ blk, const int *__restrict__ act) {
     const int2 pb = blk[blockIdx.x];
+    if (act && !act[pb.x]) return;
     const NLArgs a = args[pb.x];
     const int gx = (a.g.M + a.MC - 1) / a.MC;
     nl_zfwd_body<ZL, C>(a, pb.y % gx, (pb.y / gx) % a.g.N, pb.y / (gx * a.g.N));
@@ -928,23 +933,29 @@ __global__ void __launch_bounds__(NL_THREADS, (NLOcc<C, ZL>::zfwd)) k_nl_zfwd_b(
 
 template <int ZL, int TL>
 __global__ void __launch_bounds__(FUSED_THREADS, 1) k_nl_fused_b(const NLArgs *__restrict__ args,
-                                                                const int2 *__restrict__ blk) {
+                                                                const int2 *__restrict__ blk,
+                                                                const int *__restrict__ act) {
     const int2 pb = blk[blockIdx.x];
+    if (act && !act[pb.x]) return;
     const NLArgs a = args[pb.x];
     nl_fused_body<ZL, TL>(a, pb.y);
 }
 
 // the chunks of every pipe of either precision (nfp64: of the FP64 pipes)
 __global__ void __launch_bounds__(PREP_THREADS) k_nl_prep_batch(const NLArgs *__restrict__ args,
-                                                               const int2 *__restrict__ blk, int nfp64, int sym) {
+                                                               const int2 *__restrict__ blk, int nfp64, int sym,
+                                                               const int *__restrict__ act) {
     const int2 pb = blk[blockIdx.x];
+    if (act && !act[pb.x]) return;
     const NLArgs a = args[pb.x];
     if ((int)blockIdx.x < nfp64) nl_prep_body<false>(a, pb.y, sym);
     else nl_prep_body<true>(a, pb.y, sym);
 }
 __global__ void __launch_bounds__(128) k_nl_mean64_fin_batch(const NLArgs *__restrict__ args,
-                                                            const int2 *__restrict__ blk, int stepped) {
+                                                            const int2 *__restrict__ blk, int stepped,
+                                                            const int *__restrict__ act) {
     const int2 pb = blk[blockIdx.x];
+    if (act && !act[pb.x]) return;
     const NLArgs a = args[pb.x];
     const int n = pb.y * 4 + (threadIdx.x >> 5);
     if (n < a.g.N) nl_mean64_fin_body(a, n, stepped);
@@ -1006,7 +1017,8 @@ template <int ST> __device__ __forceinline__ void nl_wl_item(const NLArgs *__res
 // ctr[0]: next item; ctr[1]: blocks that have left (both zero between launches)
 template <int ST>
 __global__ void __launch_bounds__(NL_THREADS, ST == 1 ? 6 : 5)
-    k_nl_stage_wl(const NLArgs *__restrict__ args, const int2 *__restrict__ items, int nitems, unsigned *ctr) {
+    k_nl_stage_wl(const NLArgs *__restrict__ args, const int2 *__restrict__ items, int nitems, unsigned *ctr,
+                  const int *__restrict__ act) {
     __shared__ int next[2];
     if (threadIdx.x == 0) next[0] = (int)atomicAdd(&ctr[0], 1u);
     __syncthreads();
@@ -1014,7 +1026,7 @@ __global__ void __launch_bounds__(NL_THREADS, ST == 1 ? 6 : 5)
     while (cur < nitems) {
         if (threadIdx.x == 0) next[slot ^ 1] = (int)atomicAdd(&ctr[0], 1u);
         const int2 pb = items[cur];
-        nl_wl_item<ST>(args, pb.x, pb.y);
+        if (!act || act[pb.x]) nl_wl_item<ST>(args, pb.x, pb.y);
         __syncthreads();  // the item's shared memory is free, next[slot ^ 1] is visible
         slot ^= 1;
         cur = next[slot];
@@ -1290,20 +1302,21 @@ int pf_nl_batch_build(pf_ctx *const *pipes, int n, bool worklist, pf_nl_batch **
     return PF_OK;
 }
 
-template <typename C> static int nlb_group_launch(int st, const NLGroup &gr, const NLArgs *args, cudaStream_t s) {
+template <typename C>
+static int nlb_group_launch(int st, const NLGroup &gr, const NLArgs *args, const int *act, cudaStream_t s) {
     switch (gr.L) {
 #define PF_CASE(L)                                                                                 \
     case L: {                                                                                      \
         static size_t set_[NLB_STAGES] = {0, 0, 0};                                                \
         if (st == 0) {                                                                             \
             PF_TRY(raise_smem(k_nl_zinv_b<L, C>, gr.smem, set_[0]));                               \
-            k_nl_zinv_b<L, C><<<gr.nblk, NL_THREADS, gr.smem, s>>>(args, gr.blk);                  \
+            k_nl_zinv_b<L, C><<<gr.nblk, NL_THREADS, gr.smem, s>>>(args, gr.blk, act);                  \
         } else if (st == 1) {                                                                      \
             PF_TRY(raise_smem(k_nl_theta_b<L, C>, gr.smem, set_[1]));                              \
-            k_nl_theta_b<L, C><<<gr.nblk, NL_THREADS, gr.smem, s>>>(args, gr.blk);                 \
+            k_nl_theta_b<L, C><<<gr.nblk, NL_THREADS, gr.smem, s>>>(args, gr.blk, act);                 \
         } else {                                                                                   \
             PF_TRY(raise_smem(k_nl_zfwd_b<L, C>, gr.smem, set_[2]));                               \
-            k_nl_zfwd_b<L, C><<<gr.nblk, NL_THREADS, gr.smem, s>>>(args, gr.blk);                  \
+            k_nl_zfwd_b<L, C><<<gr.nblk, NL_THREADS, gr.smem, s>>>(args, gr.blk, act);                  \
         }                                                                                          \
     } break;
         PF_NL_LENGTHS(PF_CASE)
@@ -1316,12 +1329,12 @@ template <typename C> static int nlb_group_launch(int st, const NLGroup &gr, con
     return PF_OK;
 }
 
-static int nlb_fused_launch(const NLGroup &gr, const NLArgs *args, cudaStream_t s) {
+static int nlb_fused_launch(const NLGroup &gr, const NLArgs *args, const int *act, cudaStream_t s) {
 #define PF_CASE(ZL, TL)                                                              \
     if (gr.L == ZL && gr.Th == TL) {                                                 \
         static size_t set_ = 0;                                                      \
         PF_TRY(raise_smem(k_nl_fused_b<ZL, TL>, gr.smem, set_));                     \
-        k_nl_fused_b<ZL, TL><<<gr.nblk, FUSED_THREADS, gr.smem, s>>>(args, gr.blk);  \
+        k_nl_fused_b<ZL, TL><<<gr.nblk, FUSED_THREADS, gr.smem, s>>>(args, gr.blk, act);  \
         PF_CHECK_LAUNCH();                                                           \
         return PF_OK;                                                                \
     }
@@ -1332,15 +1345,16 @@ static int nlb_fused_launch(const NLGroup &gr, const NLArgs *args, cudaStream_t 
 }
 
 // one stage: the first group on st, the others forked onto auxiliary streams
-static int nlb_stage(pf_nl_batch *b, int stage, const NLArgs *args, cudaStream_t st, unsigned long long *nk) {
+static int nlb_stage(pf_nl_batch *b, int stage, const NLArgs *args, const int *act, cudaStream_t st,
+                     unsigned long long *nk) {
     if (b->wl) {
         if (b->wl_n[stage] == 0) return PF_OK;
         const int g = b->wl_grid[stage], n = b->wl_n[stage];
         const size_t sm = b->wl_smem[stage];
         unsigned *ctr = b->wl_ctr + 2 * stage;
-        if (stage == 0) k_nl_stage_wl<0><<<g, NL_THREADS, sm, st>>>(args, b->wl_items[0], n, ctr);
-        else if (stage == 1) k_nl_stage_wl<1><<<g, NL_THREADS, sm, st>>>(args, b->wl_items[1], n, ctr);
-        else k_nl_stage_wl<2><<<g, NL_THREADS, sm, st>>>(args, b->wl_items[2], n, ctr);
+        if (stage == 0) k_nl_stage_wl<0><<<g, NL_THREADS, sm, st>>>(args, b->wl_items[0], n, ctr, act);
+        else if (stage == 1) k_nl_stage_wl<1><<<g, NL_THREADS, sm, st>>>(args, b->wl_items[1], n, ctr, act);
+        else k_nl_stage_wl<2><<<g, NL_THREADS, sm, st>>>(args, b->wl_items[2], n, ctr, act);
         PF_CHECK_LAUNCH();
         ++*nk;
         return PF_OK;
@@ -1352,8 +1366,8 @@ static int nlb_stage(pf_nl_batch *b, int stage, const NLArgs *args, cudaStream_t
     }
     for (size_t k = 0; k < gs.size(); ++k) {
         cudaStream_t s = k ? b->aux[k] : st;
-        if (gs[k].mixed) PF_TRY(nlb_group_launch<float2>(stage, gs[k], args, s));
-        else PF_TRY(nlb_group_launch<double2>(stage, gs[k], args, s));
+        if (gs[k].mixed) PF_TRY(nlb_group_launch<float2>(stage, gs[k], args, act, s));
+        else PF_TRY(nlb_group_launch<double2>(stage, gs[k], args, act, s));
         ++*nk;
     }
     for (size_t k = 1; k < gs.size(); ++k) {
@@ -1367,15 +1381,16 @@ static int nlb_stage(pf_nl_batch *b, int stage, const NLArgs *args, cudaStream_t
 // predictor left it (mode as in pf_launch_nl_fused), one launch per stage and
 // (transform length, precision) group, and the mean mode of the pipes in mixed
 // precision; launches are counted into *nk.  state 0: the pointers the pipes
-// held when the batch was built; 1: vel/prev swapped.
-int pf_nl_batch_launch(pf_nl_batch *b, int state, int mode, cudaStream_t st, pf_stage_prof *prof,
+// held when the batch was built; 1: vel/prev swapped.  act: null, or the mask
+// of the pipes to work on.
+int pf_nl_batch_launch(pf_nl_batch *b, int state, int mode, const int *act, cudaStream_t st, pf_stage_prof *prof,
                        unsigned long long *nk) {
     const NLArgs *args = b->d_args[state];
     const int cats[NLB_STAGES] = {PF_K_ZINV, PF_K_THFWD, PF_K_ZFWD};
     if (mode != PF_NL_STEPPED) {
         StageScope ss_(prof, PF_K_STENCIL, st);
         PF_TRY(prep_attrs());
-        k_nl_prep_batch<<<b->nprep, PREP_THREADS, b->prep_sm, st>>>(args, b->prep_blk, b->nprep64, mode == PF_NL_SYM);
+        k_nl_prep_batch<<<b->nprep, PREP_THREADS, b->prep_sm, st>>>(args, b->prep_blk, b->nprep64, mode == PF_NL_SYM, act);
         PF_CHECK_LAUNCH();
         *nk += 1;
     }
@@ -1385,19 +1400,19 @@ int pf_nl_batch_launch(pf_nl_batch *b, int state, int mode, cudaStream_t st, pf_
         PF_CUDA(cudaEventRecord(b->ffork, st));
         for (size_t k = 0; k < b->fgroups.size(); ++k) {
             PF_CUDA(cudaStreamWaitEvent(b->faux[k], b->ffork, 0));
-            PF_TRY(nlb_fused_launch(b->fgroups[k], args, b->faux[k]));
+            PF_TRY(nlb_fused_launch(b->fgroups[k], args, act, b->faux[k]));
             PF_CUDA(cudaEventRecord(b->fjoin[k], b->faux[k]));
             ++*nk;
         }
     }
     for (int stage = 0; stage < NLB_STAGES; ++stage) {
         StageScope ss_(prof, cats[stage], st);
-        PF_TRY(nlb_stage(b, stage, args, st, nk));
+        PF_TRY(nlb_stage(b, stage, args, act, st, nk));
     }
     for (size_t k = 0; k < b->fgroups.size(); ++k) PF_CUDA(cudaStreamWaitEvent(st, b->fjoin[k], 0));
     if (b->nfin > 0) {
         StageScope ss_(prof, PF_K_ZFWD, st);
-        k_nl_mean64_fin_batch<<<b->nfin, 128, 0, st>>>(args, b->fin_blk, mode == PF_NL_STEPPED);
+        k_nl_mean64_fin_batch<<<b->nfin, 128, 0, st>>>(args, b->fin_blk, mode == PF_NL_STEPPED, act);
         PF_CHECK_LAUNCH();
         *nk += 1;
     }

@@ -679,8 +679,9 @@ __global__ void __launch_bounds__(NT, MINB) k_step(const __grid_constant__ StepA
 
 template <int NT, int MINB, int W>
 __global__ void __launch_bounds__(NT, MINB) k_step_batch(const StepArgs *__restrict__ args, const int2 *__restrict__ blk,
-                                                         const StepSmem lay) {
+                                                         const StepSmem lay, const int *__restrict__ act) {
     const int2 pb = blk[blockIdx.x];
+    if (act && !act[pb.x]) return;
     const StepArgs a = args[pb.x];  // by value: stores through its pointers cannot alias it
     step_tile<NT, W>(a, pb.y, lay);
 }
@@ -871,17 +872,17 @@ int pf_step_batch_build(pf_ctx *const *pipes, int n, pf_aux *aux, pf_step_batch 
     return PF_OK;
 }
 
-static int step_group_launch(const StepGroup &gr, const StepArgs *a, cudaStream_t st) {
+static int step_group_launch(const StepGroup &gr, const StepArgs *a, const int *act, cudaStream_t st) {
 #define PF_CASE(NMAX, NT, MINB)                                                \
     else if (gr.N <= NMAX) {                                                   \
         const StepSmem lay = step_rings(gr.N, MINB);                           \
         const size_t sm = step_smem(gr.N, lay);                                \
         if (gr.W == 16) {                                                      \
             PF_TRY(pf_raise_smem((const void *)k_step_batch<NT, MINB, 16>, sm)); \
-            k_step_batch<NT, MINB, 16><<<gr.nblk, NT, sm, st>>>(a, gr.blk, lay); \
+            k_step_batch<NT, MINB, 16><<<gr.nblk, NT, sm, st>>>(a, gr.blk, lay, act); \
         } else {                                                               \
             PF_TRY(pf_raise_smem((const void *)k_step_batch<NT, MINB, 8>, sm));  \
-            k_step_batch<NT, MINB, 8><<<gr.nblk, NT, sm, st>>>(a, gr.blk, lay);  \
+            k_step_batch<NT, MINB, 8><<<gr.nblk, NT, sm, st>>>(a, gr.blk, lay, act);  \
         }                                                                      \
     }
     if (false) {
@@ -894,15 +895,16 @@ static int step_group_launch(const StepGroup &gr, const StepArgs *a, cudaStream_
 
 // One predictor or corrector vel_step of every pipe, one launch per group;
 // the caller tracks the pointer state (the predictor's swap is the caller's).
-int pf_step_batch_launch(pf_step_batch *b, int state, int corrector, cudaStream_t st, pf_stage_prof *prof,
-                         unsigned long long *nk) {
+// act: null, or the mask of the pipes to step.
+int pf_step_batch_launch(pf_step_batch *b, int state, int corrector, const int *act, cudaStream_t st,
+                         pf_stage_prof *prof, unsigned long long *nk) {
     const StepArgs *a = b->d_args[state][corrector ? 1 : 0];
     StageScope ss_(prof, PF_K_STEP, st);
     const size_t more = b->groups.size() - 1;
     if (more > 0) PF_CUDA(cudaEventRecord(b->aux->fork, st));
     for (size_t k = 0; k < more; ++k) PF_CUDA(cudaStreamWaitEvent(b->aux->st[k], b->aux->fork, 0));
     for (size_t k = 0; k <= more; ++k) {
-        PF_TRY(step_group_launch(b->groups[k], a, k ? b->aux->st[k - 1] : st));
+        PF_TRY(step_group_launch(b->groups[k], a, act, k ? b->aux->st[k - 1] : st));
         ++*nk;
     }
     for (size_t k = 0; k < more; ++k) {
