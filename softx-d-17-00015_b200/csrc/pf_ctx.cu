@@ -214,7 +214,7 @@ static int ctx_init(pf_ctx *ctx, const pf_config *cfg, int device) {
     PF_TRY(pf_alloc(ctx, (void **)&ctx->orbit_red, (size_t)(ORBIT_DOT_BLOCKS + 1) * sizeof(double)));
     PF_TRY(pf_alloc(ctx, (void **)&ctx->cflmax, (size_t)3 * N * sizeof(unsigned long long)));
     PF_TRY(pf_alloc(ctx, (void **)&ctx->mpart, (size_t)std::max((g.H + 31) / 32, pf_step_tiles(g)) * N * 3 * sizeof(double)));
-    PF_TRY(pf_alloc(ctx, (void **)&ctx->anypiv, sizeof(int)));
+    PF_TRY(pf_alloc(ctx, &ctx->lustat, 64));
     // the (m, z) intermediate in FP64; in mixed precision its FP32 copy takes
     // the first 6*N*M*Z float2 and the FP32 curl(u) fields (3*N*Hp float2) follow
     ctx->T_bytes = std::max((size_t)6 * N * g.M * g.Z * sizeof(double2),

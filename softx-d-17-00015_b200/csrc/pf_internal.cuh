@@ -265,7 +265,7 @@ struct pf_ctx {
     unsigned long long util_evals;  // plug-in evaluations since pf_util_set
     unsigned long long *cflmax;  // 3*N CFL maxima of the last fused transform
     bool cfl_fused;              // cflmax is current (else use vel_r/t/z)
-    int *anypiv;         // per LU set: 1 if dgbtf2 swapped any row
+    void *lustat;        // what a factorisation leaves for the host (pf_lu.cu)
     void *T;             // FFT scratch: 6*N*M*Z complex (FP64)
     size_t T_bytes;
     int zinv_mc, zfwd_mc, th_zc;   // tile sizes
@@ -385,7 +385,6 @@ int pf_launch_measurecorr(pf_ctx *ctx, const double2 *a0, const double2 *b0,
                           const double2 *a1, const double2 *b1,
                           const double2 *a2, const double2 *b2, bool reset);
 int pf_launch_addHPF(pf_ctx *ctx);
-int pf_launch_lu_factor(pf_ctx *ctx, pf_lumesh *A);
 int pf_launch_lu_solve(pf_ctx *ctx, int BC, const pf_lumesh *A, double2 *b);
 int pf_launch_adjppe2(pf_ctx *ctx);
 int pf_launch_flux1(pf_ctx *ctx);
