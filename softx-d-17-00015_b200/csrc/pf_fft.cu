@@ -8,10 +8,16 @@
 //                  truncation to |k|<K, m<M.
 // FFTW's sign conventions are kept: +1 is the unnormalised backward transform;
 // the c2r transform ignores the imaginary part of the theta DC bin.
+#include <algorithm>
 #include <cmath>
 #include "pf_internal.cuh"
+#include "pf_fftcore.cuh"
 
 static constexpr int FFT_THREADS = 256;
+
+// the lengths 3K, 3M whose row transforms are compiled (codelets in registers);
+// others take the mixed-radix passes of smem_fft
+#define PF_FFT_LENGTHS(X) X(12) X(15) X(18) X(24) X(36) X(48) X(72) X(96) X(144) X(192) X(288) X(384)
 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
     return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -23,70 +29,116 @@ __device__ __forceinline__ double2 cmuli(double2 a, int sign) {
     return sign > 0 ? make_double2(-a.y, a.x) : make_double2(a.y, -a.x);
 }
 
+// An R-point transform of v in registers.  w[p] = exp(2 pi i p/R), 1 <= p <=
+// (R-1)/2, for the odd radices above 3, whose outputs q and R-q share the
+// real sums of v[p] + v[R-p] and v[p] - v[R-p].
+template <int R> __device__ __forceinline__ void gen_dft(double2 (&v)[R], const double2 (&w)[(R + 1) / 2], int sign) {
+    if constexpr (R == 2) {
+        const double2 a = v[0];
+        v[0] = cadd(a, v[1]);
+        v[1] = csub(a, v[1]);
+    } else if constexpr (R == 4) {
+        const double2 a = cadd(v[0], v[2]), b = csub(v[0], v[2]);
+        const double2 c = cadd(v[1], v[3]), d = cmuli(csub(v[1], v[3]), sign);
+        v[0] = cadd(a, c);
+        v[1] = cadd(b, d);
+        v[2] = csub(a, c);
+        v[3] = csub(b, d);
+    } else if constexpr (R == 3) {
+        const double s3 = 0.86602540378443864676;  // sin(2 pi/3)
+        const double2 t = cadd(v[1], v[2]);
+        const double2 u = make_double2(v[0].x - 0.5 * t.x, v[0].y - 0.5 * t.y);
+        const double2 x = cmuli(make_double2(s3 * (v[1].x - v[2].x), s3 * (v[1].y - v[2].y)), sign);
+        v[0] = cadd(v[0], t);
+        v[1] = cadd(u, x);
+        v[2] = csub(u, x);
+    } else {
+        constexpr int H = (R - 1) / 2;
+        double2 a[H], b[H], o = v[0];
+#pragma unroll
+        for (int p = 1; p <= H; ++p) {
+            a[p - 1] = cadd(v[p], v[R - p]);
+            b[p - 1] = cmuli(csub(v[p], v[R - p]), sign);
+            o = cadd(o, a[p - 1]);
+        }
+        const double2 v0 = v[0];
+        v[0] = o;
+#pragma unroll
+        for (int q = 1; q <= H; ++q) {
+            double2 c = v0, d = make_double2(0.0, 0.0);
+#pragma unroll
+            for (int p = 1; p <= H; ++p) {
+                const int e = p * q % R;
+                const double2 x = w[e <= H ? e : R - e];
+                const double sn = e <= H ? x.y : -x.y;
+                c = make_double2(fma(x.x, a[p - 1].x, c.x), fma(x.x, a[p - 1].y, c.y));
+                d = make_double2(fma(sn, b[p - 1].x, d.x), fma(sn, b[p - 1].y, d.y));
+            }
+            v[q] = cadd(c, d);
+            v[R - q] = csub(c, d);
+        }
+    }
+}
+
+// One Stockham pass of radix R over B batches of length L: butterfly j
+// (k = j mod Ns) goes to outputs (j/Ns)*Ns*R + k + q*Ns with twiddles
+// W^(sign q k L/(Ns R)).
+template <int R>
+__device__ __forceinline__ void smem_pass(const double2 *src, double2 *dst, int B, int L, int Ns, const double2 *tw,
+                                          int sign) {
+    const int nb = L / R, stride = nb / Ns;
+    const float inb = 1.0f / nb, ins = 1.0f / Ns;
+    double2 w[(R + 1) / 2];
+#pragma unroll
+    for (int p = 1; p <= (R - 1) / 2; ++p) w[p] = tw[p * nb];
+    for (int idx = threadIdx.x; idx < nb * B; idx += blockDim.x) {
+        const int b = fdiv(idx, nb, inb), j = idx - b * nb;
+        const int jn = fdiv(j, Ns, ins), k = j - jn * Ns;
+        const double2 *sp = src + b * L + j;
+        double2 *dp = dst + b * L + jn * Ns * R + k;
+        double2 v[R];
+#pragma unroll
+        for (int q = 0; q < R; ++q) v[q] = sp[q * nb];
+        if (Ns > 1) {
+            const int t = k * stride;
+#pragma unroll
+            for (int q = 1; q < R; ++q) {
+                double2 x = tw[q * t];
+                if (sign < 0) x.y = -x.y;
+                v[q] = cmul(v[q], x);
+            }
+        }
+        gen_dft<R>(v, w, sign);
+#pragma unroll
+        for (int q = 0; q < R; ++q) dp[q * Ns] = v[q];
+    }
+}
+
 // B batches of length L (batch stride L) in `buf`; `tmp` is the ping-pong
 // buffer; tw[t] = exp(+2 pi i t/L).  Returns the buffer holding the result.
-// Stockham autosort: pass with radix r maps butterfly j (k = j mod Ns) to
-// outputs (j/Ns)*Ns*r + k + q*Ns with twiddles W^(sign q k L/(Ns r)).
-__device__ double2 *smem_fft(double2 *buf, double2 *tmp, int B, const FFTPlan &pl, const double2 *tw, int sign) {
-    const int L = pl.L;
+// Stockham autosort.  Each radix has its own code with the butterfly in
+// registers: with the radix a variable the butterfly lived in local memory and
+// the primes took a table product per term (N=37, 3K=60, 3M=33, six fields: z
+// 9.8, theta 23.2 us; now 9.0, 8.2).
+__device__ __forceinline__ double2 *smem_fft(double2 *buf, double2 *tmp, int B, const FFTPlan &pl, const double2 *tw,
+                                             int sign) {
     double2 *src = buf, *dst = tmp;
     int Ns = 1;
     for (int s = 0; s < pl.nf; ++s) {
-        const int r = pl.f[s];
-        const int nb = L / r;
-        const int stride = L / (Ns * r);
-        for (int idx = threadIdx.x; idx < nb * B; idx += blockDim.x) {
-            const int b = idx / nb, j = idx - b * nb;
-            const int k = j % Ns;
-            const double2 *sp = src + b * L;
-            double2 *dp = dst + b * L;
-            const int base = (j / Ns) * Ns * r + k;
-            double2 v[16];
-            for (int q = 0; q < r; ++q) {
-                double2 x = sp[j + q * nb];
-                if (q > 0 && k > 0) {
-                    double2 w = tw[q * k * stride];
-                    if (sign < 0) w.y = -w.y;
-                    x = cmul(x, w);
-                }
-                v[q] = x;
-            }
-            if (r == 2) {
-                dp[base] = cadd(v[0], v[1]);
-                dp[base + Ns] = csub(v[0], v[1]);
-            } else if (r == 4) {
-                const double2 a = cadd(v[0], v[2]), b2 = csub(v[0], v[2]);
-                const double2 c = cadd(v[1], v[3]), d = cmuli(csub(v[1], v[3]), sign);
-                dp[base] = cadd(a, c);
-                dp[base + Ns] = cadd(b2, d);
-                dp[base + 2 * Ns] = csub(a, c);
-                dp[base + 3 * Ns] = csub(b2, d);
-            } else if (r == 3) {
-                const double s3 = 0.86602540378443864676;  // sin(2 pi/3)
-                const double2 t = cadd(v[1], v[2]);
-                const double2 u = make_double2(v[0].x - 0.5 * t.x, v[0].y - 0.5 * t.y);
-                const double2 w = cmuli(make_double2(s3 * (v[1].x - v[2].x), s3 * (v[1].y - v[2].y)), sign);
-                dp[base] = cadd(v[0], t);
-                dp[base + Ns] = cadd(u, w);
-                dp[base + 2 * Ns] = csub(u, w);
-            } else {  // generic small prime radix: direct DFT with table twiddles
-                const int st = L / r;
-                for (int q = 0; q < r; ++q) {
-                    double2 acc = v[0];
-                    for (int p = 1; p < r; ++p) {
-                        double2 w = tw[((p * q) % r) * st];
-                        if (sign < 0) w.y = -w.y;
-                        acc = cadd(acc, cmul(v[p], w));
-                    }
-                    dp[base + q * Ns] = acc;
-                }
-            }
+        switch (pl.f[s]) {
+        case 2: smem_pass<2>(src, dst, B, pl.L, Ns, tw, sign); break;
+        case 3: smem_pass<3>(src, dst, B, pl.L, Ns, tw, sign); break;
+        case 4: smem_pass<4>(src, dst, B, pl.L, Ns, tw, sign); break;
+        case 5: smem_pass<5>(src, dst, B, pl.L, Ns, tw, sign); break;
+        case 7: smem_pass<7>(src, dst, B, pl.L, Ns, tw, sign); break;
+        case 11: smem_pass<11>(src, dst, B, pl.L, Ns, tw, sign); break;
+        default: smem_pass<13>(src, dst, B, pl.L, Ns, tw, sign); break;
         }
         __syncthreads();
         double2 *t = src;
         src = dst;
         dst = t;
-        Ns *= r;
+        Ns *= pl.f[s];
     }
     return src;
 }
@@ -105,7 +157,7 @@ struct DstPtrs {
 };
 
 // z pass, spectral -> (m, z) columns: grid (m-chunk, n, comp)
-__global__ void k_zinv(SrcPtrs src, double2 *__restrict__ T, Geo g, FFTPlan pz, const double2 *__restrict__ twz,
+__global__ void __launch_bounds__(FFT_THREADS, 2) k_zinv(SrcPtrs src, double2 *__restrict__ T, Geo g, FFTPlan pz, const double2 *__restrict__ twz,
                        int MC) {
     extern __shared__ double2 sm[];
     const int Z = g.Z, K = g.K;
@@ -114,21 +166,16 @@ __global__ void k_zinv(SrcPtrs src, double2 *__restrict__ T, Geo g, FFTPlan pz, 
     const int mc = min(MC, g.M - m0);
     const double2 *f = src.p[comp] + (size_t)n * g.Hp;
     for (int i = threadIdx.x; i < Z; i += blockDim.x) tw[i] = twz[i];
+    const float iZ = 1.0f / Z;
+#pragma unroll 4
     for (int idx = threadIdx.x; idx < mc * Z; idx += blockDim.x) {
-        const int c = idx / Z, j = idx - c * Z;
-        const int m = m0 + c;
+        const int c = fdiv(idx, Z, iZ), j = idx - c * Z, m = m0 + c;
+        // zero-padded in k, the Hermitian fill at m = 0
+        const int kk = j < K ? j : j - Z;
+        const bool zero = j >= K && j <= 2 * K, conj = m == 0 && kk < 0;
         double2 v = make_double2(0.0, 0.0);
-        if (m == 0) {
-            if (j < K) v = f[j];
-            else if (j >= 2 * K + 1) {
-                v = f[Z - j];
-                v.y = -v.y;
-            }
-        } else {
-            const int base = m * (2 * K - 1);
-            if (j < K) v = f[base + j];
-            else if (j >= 2 * K + 1) v = f[base + (j - Z)];
-        }
+        if (!zero) v = f[conj ? -kk : m * (2 * K - 1) + kk];
+        v.y = conj ? -v.y : v.y;
         buf[idx] = v;
     }
     __syncthreads();
@@ -139,7 +186,7 @@ __global__ void k_zinv(SrcPtrs src, double2 *__restrict__ T, Geo g, FFTPlan pz, 
 
 // theta pass, (m, z) columns -> physical: grid (z-chunk, n); ncomp comps,
 // ZC rows per block, two rows per complex FFT
-__global__ void k_thinv(const double2 *__restrict__ T, PhysPtrs dst, int ncomp, Geo g, FFTPlan pt,
+__global__ void __launch_bounds__(FFT_THREADS, 2) k_thinv(const double2 *__restrict__ T, PhysPtrs dst, int ncomp, Geo g, FFTPlan pt,
                         const double2 *__restrict__ twt, int ZC) {
     extern __shared__ double2 sm[];
     const int Th = g.Th, M = g.M, Z = g.Z;
@@ -147,18 +194,21 @@ __global__ void k_thinv(const double2 *__restrict__ T, PhysPtrs dst, int ncomp, 
     double2 *buf = sm, *tmp = sm + B * Th, *tw = sm + 2 * B * Th;
     const int n = blockIdx.y, z0 = blockIdx.x * ZC;
     for (int i = threadIdx.x; i < Th; i += blockDim.x) tw[i] = twt[i];
-    for (int i = threadIdx.x; i < B * Th; i += blockDim.x) buf[i] = make_double2(0.0, 0.0);
-    __syncthreads();
+    const float inp = 1.0f / np, iM = 1.0f / M;
+    // Th = 3M: mode m's thread also clears X[M + m] of the zero band (m = 0 X[2M])
+#pragma unroll 4
     for (int idx = threadIdx.x; idx < ncomp * M * np; idx += blockDim.x) {
-        const int zp = idx % np, rest = idx / np;
-        const int m = rest % M, comp = rest / M;
+        const int rest = fdiv(idx, np, inp), zp = idx - rest * np;
+        const int comp = fdiv(rest, M, iM), m = rest - comp * M;
         const int za = z0 + 2 * zp, zb = za + 1;
         const double2 *col = T + ((size_t)(comp * g.N + n) * M + m) * Z;
         double2 a = (za < Z) ? col[za] : make_double2(0.0, 0.0);
         double2 b = (zb < Z) ? col[zb] : make_double2(0.0, 0.0);
         double2 *X = buf + (comp * np + zp) * Th;
+        X[M + m] = make_double2(0.0, 0.0);
         if (m == 0) {
             X[0] = make_double2(a.x, b.x);  // c2r: DC imaginary parts ignored
+            X[2 * M] = make_double2(0.0, 0.0);
         } else {
             X[m] = make_double2(a.x - b.y, a.y + b.x);            // a + i b
             X[Th - m] = make_double2(a.x + b.y, -a.y + b.x);      // conj(a) + i conj(b)
@@ -166,9 +216,10 @@ __global__ void k_thinv(const double2 *__restrict__ T, PhysPtrs dst, int ncomp, 
     }
     __syncthreads();
     const double2 *res = smem_fft(buf, tmp, B, pt, tw, +1);
+    const float iC = 1.0f / ZC, iT = 1.0f / Th;
     for (int idx = threadIdx.x; idx < ncomp * Th * ZC; idx += blockDim.x) {
-        const int zz = idx % ZC, rest = idx / ZC;
-        const int t = rest % Th, comp = rest / Th;
+        const int rest = fdiv(idx, ZC, iC), zz = idx - rest * ZC;
+        const int comp = fdiv(rest, Th, iT), t = rest - comp * Th;
         const int z = z0 + zz;
         if (z >= Z) continue;
         const double2 v = res[(comp * np + zz / 2) * Th + t];
@@ -179,7 +230,7 @@ __global__ void k_thinv(const double2 *__restrict__ T, PhysPtrs dst, int ncomp, 
 // theta pass, physical -> (m, z) columns (scaled): grid (z-chunk, n).
 // cross != 0: inputs are (r,t,z,curlr,curlt,curlz) and the three outputs are
 // the components of u x curl(u) (velocity.f90:325-330).
-__global__ void k_thfwd(CPhysPtrs src, int ncomp, int cross, double2 *__restrict__ T, Geo g, FFTPlan pt,
+__global__ void __launch_bounds__(FFT_THREADS, 2) k_thfwd(CPhysPtrs src, int ncomp, int cross, double2 *__restrict__ T, Geo g, FFTPlan pt,
                         const double2 *__restrict__ twt, int ZC, double scale) {
     extern __shared__ double2 sm[];
     const int Th = g.Th, M = g.M, Z = g.Z;
@@ -188,33 +239,35 @@ __global__ void k_thfwd(CPhysPtrs src, int ncomp, int cross, double2 *__restrict
     const int n = blockIdx.y, z0 = blockIdx.x * ZC;
     for (int i = threadIdx.x; i < Th; i += blockDim.x) tw[i] = twt[i];
     double *bre = reinterpret_cast<double *>(buf);
-    for (int idx = threadIdx.x; idx < ncomp * Th * ZC; idx += blockDim.x) {
-        const int zz = idx % ZC, rest = idx / ZC;
-        const int t = rest % Th, comp = rest / Th;
-        const int z = z0 + zz;
-        double v = 0.0;
-        if (z < Z) {
-            const size_t at = ((size_t)n * Th + t) * Z + z;
-            if (cross) {
-                const double ur = src.p[0][at], ut = src.p[1][at], uz = src.p[2][at];
-                const double cr = src.p[3][at], ct = src.p[4][at], cz = src.p[5][at];
-                if (comp == 0) v = ut * cz - uz * ct;
-                else if (comp == 1) v = uz * cr - ur * cz;
-                else v = ur * ct - ut * cr;
-            } else {
-                v = src.p[comp][at];
-            }
-            v = scale * v;
+    const float iC = 1.0f / ZC, iT = 1.0f / Th, inp = 1.0f / np, iM = 1.0f / M;
+    if (cross) {  // a grid point's three components together
+#pragma unroll 2
+        for (int idx = threadIdx.x; idx < Th * ZC; idx += blockDim.x) {
+            const int t = fdiv(idx, ZC, iC), zz = idx - t * ZC, z = z0 + zz;
+            const size_t at = ((size_t)n * Th + t) * Z + min(z, Z - 1);
+            const double ur = src.p[0][at], ut = src.p[1][at], uz = src.p[2][at];
+            const double cr = src.p[3][at], ct = src.p[4][at], cz = src.p[5][at];
+            double *o = bre + 2 * (zz / 2 * Th + t) + (zz & 1);
+            o[0] = z < Z ? scale * (ut * cz - uz * ct) : 0.0;
+            o[2 * np * Th] = z < Z ? scale * (uz * cr - ur * cz) : 0.0;
+            o[4 * np * Th] = z < Z ? scale * (ur * ct - ut * cr) : 0.0;
         }
-        bre[2 * ((comp * np + zz / 2) * Th + t) + (zz & 1)] = v;
+    } else {
+#pragma unroll 4
+        for (int idx = threadIdx.x; idx < ncomp * Th * ZC; idx += blockDim.x) {
+            const int rest = fdiv(idx, ZC, iC), zz = idx - rest * ZC, z = z0 + zz;
+            const int comp = fdiv(rest, Th, iT), t = rest - comp * Th;
+            const double v = src.p[comp][((size_t)n * Th + t) * Z + min(z, Z - 1)];
+            bre[2 * ((comp * np + zz / 2) * Th + t) + (zz & 1)] = z < Z ? scale * v : 0.0;
+        }
     }
     __syncthreads();
     const double2 *res = smem_fft(buf, tmp, B, pt, tw, -1);
     for (int idx = threadIdx.x; idx < ncomp * M * np; idx += blockDim.x) {
-        const int zp = idx % np, rest = idx / np;
-        const int m = rest % M, comp = rest / M;
+        const int rest = fdiv(idx, np, inp), zp = idx - rest * np;
+        const int comp = fdiv(rest, M, iM), m = rest - comp * M;
         const double2 *X = res + (comp * np + zp) * Th;
-        const double2 A = X[m], Bv = X[(Th - m) % Th];
+        const double2 A = X[m], Bv = X[m ? Th - m : 0];
         // separate the two packed real transforms
         const double2 a = make_double2(0.5 * (A.x + Bv.x), 0.5 * (A.y - Bv.y));
         const double2 b = make_double2(0.5 * (A.y + Bv.y), -0.5 * (A.x - Bv.x));
@@ -226,7 +279,7 @@ __global__ void k_thfwd(CPhysPtrs src, int ncomp, int cross, double2 *__restrict
 }
 
 // z pass, (m, z) columns -> spectral with truncation: grid (m-chunk, n, comp)
-__global__ void k_zfwd(const double2 *__restrict__ T, DstPtrs dst, Geo g, FFTPlan pz,
+__global__ void __launch_bounds__(FFT_THREADS, 2) k_zfwd(const double2 *__restrict__ T, DstPtrs dst, Geo g, FFTPlan pz,
                        const double2 *__restrict__ twz, int MC) {
     extern __shared__ double2 sm[];
     const int Z = g.Z, K = g.K;
@@ -235,12 +288,14 @@ __global__ void k_zfwd(const double2 *__restrict__ T, DstPtrs dst, Geo g, FFTPla
     const int mc = min(MC, g.M - m0);
     for (int i = threadIdx.x; i < Z; i += blockDim.x) tw[i] = twz[i];
     const double2 *in = T + ((size_t)(comp * g.N + n) * g.M + m0) * Z;
+#pragma unroll 4
     for (int idx = threadIdx.x; idx < mc * Z; idx += blockDim.x) buf[idx] = in[idx];
     __syncthreads();
     const double2 *res = smem_fft(buf, tmp, mc, pz, tw, -1);
     double2 *f = dst.p[comp] + (size_t)n * g.Hp;
+    const float iK = 1.0f / (2 * K - 1);
     for (int idx = threadIdx.x; idx < mc * (2 * K - 1); idx += blockDim.x) {
-        const int c = idx / (2 * K - 1), kk = idx - c * (2 * K - 1) - (K - 1);
+        const int c = fdiv(idx, 2 * K - 1, iK), kk = idx - c * (2 * K - 1) - (K - 1);
         const int m = m0 + c;
         if (m == 0) {
             if (kk >= 0) f[kk] = res[c * Z + kk];
@@ -248,6 +303,162 @@ __global__ void k_zfwd(const double2 *__restrict__ T, DstPtrs dst, Geo g, FFTPla
             f[m * (2 * K - 1) + kk] = res[c * Z + (kk >= 0 ? kk : Z + kk)];
         }
     }
+}
+
+// ------------------------------------------------ the compiled lengths
+// The same four passes with the row transform known at compile time: a z pass
+// keeps its columns' rows in registers on both sides (RowsIO), a theta pass
+// takes one field (or the three components of the product) of ROW_ZC z rows.
+// Bound by latency at these sizes: N=40, M=16, 3K=72, 3M=48, three fields,
+// z 10.6 -> 3.1, theta 13.5 -> 6.1 us inverse, z 9.5 -> 3.4, theta 11.3 -> 5.2
+// forward against the mixed-radix passes.
+static constexpr int ROW_ZC = 16;
+// the product of a long (two-buffer) length: half the rows, to fit in shared memory
+__host__ __device__ constexpr int thfwd_zc(int L, int nc) { return nc == 3 && L > 192 ? ROW_ZC / 2 : ROW_ZC; }
+
+template <int ZL>
+__global__ void __launch_bounds__(FFT_THREADS) k_zinv_rows(SrcPtrs src, double2 *__restrict__ T, Geo g,
+                                                           const double2 *__restrict__ twz, int MC) {
+    extern __shared__ double2 sm[];
+    using FR = RowsIO<ZL, double2>;
+    constexpr int K = ZL / 3;
+    double2 *tw = sm + (FR::smem_elems(MC) - ZL);
+    const int comp = blockIdx.z, n = blockIdx.y, m0 = blockIdx.x * MC;
+    const int mc = min(MC, g.M - m0);
+    const double2 *__restrict__ f = src.p[comp] + (size_t)n * g.Hp;
+    double2 *out = T + ((size_t)(comp * g.N + n) * g.M + m0) * ZL;
+    FR::table(tw, twz);
+    FR::template run<+1>(
+        sm, mc, tw,
+        [&](int c, int j) -> double2 {  // zero-padded in k, the Hermitian fill at m = 0
+            const int m = m0 + c, kk = j < K ? j : j - ZL;
+            const bool zero = j >= K && j <= 2 * K, conj = m == 0 && kk < 0;
+            double2 v = make_double2(0.0, 0.0);
+            if (!zero) v = f[conj ? -kk : m * (2 * K - 1) + kk];
+            v.y = conj ? -v.y : v.y;
+            return v;
+        },
+        [&](int c, int j, int step, auto &v) {
+#pragma unroll
+            for (int q = 0; q < (int)(sizeof(v) / sizeof(double2)); ++q) out[c * ZL + j + step * q] = v[q];
+        });
+}
+
+template <int TL>
+__global__ void __launch_bounds__(FFT_THREADS) k_thinv_rows(const double2 *__restrict__ T, PhysPtrs dst, Geo g,
+                                                            const double2 *__restrict__ twt) {
+    extern __shared__ double2 sm[];
+    using FR = FFTRows<TL, double2>;
+    constexpr int M = TL / 3, np = ROW_ZC / 2, RS = FR::pitch;
+    double2 *tw = sm + (FR::smem_elems(np) - 2 * TL), *tw2 = tw + TL;
+    const int Z = g.Z, n = blockIdx.y, z0 = blockIdx.x * ROW_ZC, comp = blockIdx.z;
+    fft4_tables<TL>(tw, tw2, twt);
+    const double2 *in = T + (size_t)(comp * g.N + n) * M * Z;
+    // mode m's thread also clears X[M + m] of the zero band (m = 0 X[2M])
+#pragma unroll 4
+    for (int idx = threadIdx.x; idx < M * np; idx += blockDim.x) {
+        const int zp = idx % np, m = idx / np;
+        const int za = z0 + 2 * zp, zb = za + 1;
+        const double2 a = (za < Z) ? in[m * Z + za] : make_double2(0.0, 0.0);
+        const double2 b = (zb < Z) ? in[m * Z + zb] : make_double2(0.0, 0.0);
+        double2 *X = sm + zp * RS;
+        X[M + m] = make_double2(0.0, 0.0);
+        if (m == 0) {
+            X[0] = make_double2(a.x, b.x);  // c2r: DC imaginary parts ignored
+            X[2 * M] = make_double2(0.0, 0.0);
+        } else {
+            X[m] = make_double2(a.x - b.y, a.y + b.x);
+            X[TL - m] = make_double2(a.x + b.y, -a.y + b.x);
+        }
+    }
+    __syncthreads();
+    FR::template run<+1>(sm, np, tw, tw2);
+    double *__restrict__ out = dst.p[comp] + (size_t)n * TL * Z;
+    for (int idx = threadIdx.x; idx < TL * ROW_ZC; idx += blockDim.x) {
+        const int zz = idx % ROW_ZC, t = idx / ROW_ZC, z = z0 + zz;
+        const double2 v = sm[(zz / 2) * RS + t];
+        if (z < Z) out[t * Z + z] = (zz & 1) ? v.y : v.x;
+    }
+}
+
+// NC = 3: the components of u x curl(u) from six fields; 1: field blockIdx.z
+template <int TL, int NC>
+__global__ void __launch_bounds__(FFT_THREADS) k_thfwd_rows(CPhysPtrs src, double2 *__restrict__ T, Geo g,
+                                                            const double2 *__restrict__ twt, double scale) {
+    extern __shared__ double2 sm[];
+    using FR = FFTRows<TL, double2>;
+    constexpr int ZC = thfwd_zc(TL, NC), M = TL / 3, np = ZC / 2, RS = FR::pitch;
+    double2 *tw = sm + (FR::smem_elems(NC * np) - 2 * TL), *tw2 = tw + TL;
+    const int Z = g.Z, n = blockIdx.y, z0 = blockIdx.x * ZC;
+    fft4_tables<TL>(tw, tw2, twt);
+    double *re = reinterpret_cast<double *>(sm);
+#pragma unroll 4
+    for (int idx = threadIdx.x; idx < TL * ZC; idx += blockDim.x) {
+        const int zz = idx % ZC, t = idx / ZC, z = z0 + zz;
+        const size_t at = ((size_t)n * TL + t) * Z + min(z, Z - 1);
+        double *o = re + 2 * (zz / 2 * RS + t) + (zz & 1);
+        if (NC == 3) {
+            const double ur = src.p[0][at], ut = src.p[1][at], uz = src.p[2][at];
+            const double cr = src.p[3][at], ct = src.p[4][at], cz = src.p[5][at];
+            o[0] = z < Z ? scale * (ut * cz - uz * ct) : 0.0;
+            o[2 * np * RS] = z < Z ? scale * (uz * cr - ur * cz) : 0.0;
+            o[4 * np * RS] = z < Z ? scale * (ur * ct - ut * cr) : 0.0;
+        } else {
+            const double v = src.p[blockIdx.z][at];
+            o[0] = z < Z ? scale * v : 0.0;
+        }
+    }
+    __syncthreads();
+    FR::template run<-1>(sm, NC * np, tw, tw2);
+    for (int idx = threadIdx.x; idx < NC * M * np; idx += blockDim.x) {
+        const int zp = idx % np, m = idx / np % M, c = idx / (np * M);
+        const double2 *X = sm + (c * np + zp) * RS;
+        const double2 A = X[m], B = X[m ? TL - m : 0];
+        // separate the two packed real transforms
+        const int za = z0 + 2 * zp, zb = za + 1;
+        double2 *col = T + ((size_t)((NC == 3 ? c : blockIdx.z) * g.N + n) * M + m) * Z;
+        if (za < Z) col[za] = make_double2(0.5 * (A.x + B.x), 0.5 * (A.y - B.y));
+        if (zb < Z) col[zb] = make_double2(0.5 * (A.y + B.y), -0.5 * (A.x - B.x));
+    }
+}
+
+template <int ZL>
+__global__ void __launch_bounds__(FFT_THREADS) k_zfwd_rows(const double2 *__restrict__ T, DstPtrs dst, Geo g,
+                                                           const double2 *__restrict__ twz, int MC) {
+    extern __shared__ double2 sm[];
+    using FR = RowsIO<ZL, double2>;
+    constexpr int K = ZL / 3;
+    double2 *tw = sm + (FR::smem_elems(MC) - ZL);
+    const int comp = blockIdx.z, n = blockIdx.y, m0 = blockIdx.x * MC;
+    const int mc = min(MC, g.M - m0);
+    const double2 *__restrict__ in = T + ((size_t)(comp * g.N + n) * g.M + m0) * ZL;
+    double2 *__restrict__ f = dst.p[comp] + (size_t)n * g.Hp;
+    FR::table(tw, twz);
+    FR::template run<-1>(
+        sm, mc, tw, [&](int c, int j) -> double2 { return in[c * ZL + j]; },
+        [&](int c, int j, int step, auto &v) {  // the kept |k| < K, k >= 0 only at m = 0
+            const int m = m0 + c;
+#pragma unroll
+            for (int q = 0; q < (int)(sizeof(v) / sizeof(double2)); ++q) {
+                const int t = j + step * q, kk = t < K ? t : t - ZL;
+                if (!(t >= K && t <= 2 * K) && !(m == 0 && kk < 0)) f[m * (2 * K - 1) + kk] = v[q];
+            }
+        });
+}
+
+// columns and threads of a z pass's block
+struct RowsLaunch {
+    int MC, threads;
+    size_t smem;
+};
+template <int L> static RowsLaunch zrows_plan(const Geo &g) {
+    using FR = RowsIO<L, double2>;
+    const int per = FR::four ? FR::L2 : L / 8;  // threads that work on a row
+    RowsLaunch r;
+    r.MC = std::min(g.M, std::max(1, FFT_THREADS / per));
+    r.threads = std::min(FFT_THREADS, std::max(32, (r.MC * per + 31) / 32 * 32));
+    r.smem = FR::smem_elems(r.MC) * sizeof(double2);
+    return r;
 }
 
 static size_t zpass_smem(const pf_ctx *ctx, int MC) { return (size_t)(2 * MC + 1) * ctx->g.Z * sizeof(double2); }
@@ -278,22 +489,47 @@ int pf_launch_coll2phys(pf_ctx *ctx, int ncomp, const double2 *const *src, doubl
         sp.p[c] = src[c];
         pp.p[c] = dst[c];
     }
-    const int MC = pick_mc(ctx);
-    size_t sz = zpass_smem(ctx, MC);
-    PF_TRY(set_smem((const void *)k_zinv, sz));
-    dim3 gz((g.M + MC - 1) / MC, g.N, ncomp);
-    {
+    double2 *T = (double2 *)ctx->T;
+    switch (g.Z) {
+#define PF_CASE(L)                                                                                               \
+    case L: {                                                                                                    \
+        const RowsLaunch r = zrows_plan<L>(g);                                                                   \
+        PF_TRY(set_smem((const void *)k_zinv_rows<L>, r.smem));                                                  \
+        ProfScope ps_(ctx, PF_K_ZINV);                                                                           \
+        k_zinv_rows<L><<<dim3((g.M + r.MC - 1) / r.MC, g.N, ncomp), r.threads, r.smem, ctx->stream>>>(sp, T, g,  \
+                                                                                          ctx->twZ, r.MC);       \
+    } break;
+        PF_FFT_LENGTHS(PF_CASE)
+#undef PF_CASE
+    default: {
+        const int MC = pick_mc(ctx);
+        const size_t sz = zpass_smem(ctx, MC);
+        PF_TRY(set_smem((const void *)k_zinv, sz));
         ProfScope ps_(ctx, PF_K_ZINV);
-        k_zinv<<<gz, FFT_THREADS, sz, ctx->stream>>>(sp, (double2 *)ctx->T, g, ctx->planZ, ctx->twZ, MC);
+        k_zinv<<<dim3((g.M + MC - 1) / MC, g.N, ncomp), FFT_THREADS, sz, ctx->stream>>>(sp, T, g, ctx->planZ, ctx->twZ,
+                                                                                         MC);
+    }
     }
     PF_LAUNCHED(ctx);
-    const int ZC = pick_zc(ctx, ncomp);
-    sz = thpass_smem(ctx, ncomp, ZC);
-    PF_TRY(set_smem((const void *)k_thinv, sz));
-    dim3 gt((g.Z + ZC - 1) / ZC, g.N);
-    {
+    switch (g.Th) {
+#define PF_CASE(L)                                                                                               \
+    case L: {                                                                                                    \
+        const size_t sz = FFTRows<L, double2>::smem_elems(ROW_ZC / 2) * sizeof(double2);                         \
+        PF_TRY(set_smem((const void *)k_thinv_rows<L>, sz));                                                     \
+        ProfScope ps_(ctx, PF_K_THINV);                                                                          \
+        k_thinv_rows<L><<<dim3((g.Z + ROW_ZC - 1) / ROW_ZC, g.N, ncomp), 128, sz, ctx->stream>>>(T, pp, g,       \
+                                                                                                  ctx->twT);     \
+    } break;
+        PF_FFT_LENGTHS(PF_CASE)
+#undef PF_CASE
+    default: {
+        const int ZC = pick_zc(ctx, ncomp);
+        const size_t sz = thpass_smem(ctx, ncomp, ZC);
+        PF_TRY(set_smem((const void *)k_thinv, sz));
         ProfScope ps_(ctx, PF_K_THINV);
-        k_thinv<<<gt, FFT_THREADS, sz, ctx->stream>>>((const double2 *)ctx->T, pp, ncomp, g, ctx->planT, ctx->twT, ZC);
+        k_thinv<<<dim3((g.Z + ZC - 1) / ZC, g.N), FFT_THREADS, sz, ctx->stream>>>(T, pp, ncomp, g, ctx->planT, ctx->twT,
+                                                                                   ZC);
+    }
     }
     PF_LAUNCHED(ctx);
     return PF_OK;
@@ -306,24 +542,50 @@ int pf_launch_phys2coll(pf_ctx *ctx, int ncomp, const double *const *src, double
     const int nin = cross ? 6 : ncomp;
     for (int c = 0; c < nin; ++c) sp.p[c] = src[c];
     for (int c = 0; c < ncomp; ++c) dp.p[c] = dst[c];
-    const int ZC = pick_zc(ctx, ncomp);
-    size_t sz = thpass_smem(ctx, ncomp, ZC);
-    PF_TRY(set_smem((const void *)k_thfwd, sz));
-    dim3 gt((g.Z + ZC - 1) / ZC, g.N);
+    double2 *T = (double2 *)ctx->T;
     const double scale = 1.0 / (double)(g.Z * g.Th);  // transform.fftw3.f90:114
-    {
+    switch (g.Th) {
+#define PF_CASE(L)                                                                                               \
+    case L: {                                                                                                    \
+        const auto k = cross ? k_thfwd_rows<L, 3> : k_thfwd_rows<L, 1>;                                          \
+        const int zc = thfwd_zc(L, cross ? 3 : 1);                                                               \
+        const size_t sz = FFTRows<L, double2>::smem_elems((cross ? 3 : 1) * zc / 2) * sizeof(double2);           \
+        PF_TRY(set_smem((const void *)k, sz));                                                                   \
+        ProfScope ps_(ctx, PF_K_THFWD);                                                                          \
+        k<<<dim3((g.Z + zc - 1) / zc, g.N, cross ? 1 : ncomp), cross ? 256 : 128, sz, ctx->stream>>>(    \
+            sp, T, g, ctx->twT, scale);                                                                          \
+    } break;
+        PF_FFT_LENGTHS(PF_CASE)
+#undef PF_CASE
+    default: {
+        const int ZC = pick_zc(ctx, ncomp);
+        const size_t sz = thpass_smem(ctx, ncomp, ZC);
+        PF_TRY(set_smem((const void *)k_thfwd, sz));
         ProfScope ps_(ctx, PF_K_THFWD);
-        k_thfwd<<<gt, FFT_THREADS, sz, ctx->stream>>>(sp, ncomp, cross ? 1 : 0, (double2 *)ctx->T, g, ctx->planT,
-                                                       ctx->twT, ZC, scale);
+        k_thfwd<<<dim3((g.Z + ZC - 1) / ZC, g.N), FFT_THREADS, sz, ctx->stream>>>(sp, ncomp, cross ? 1 : 0, T, g,
+                                                                                   ctx->planT, ctx->twT, ZC, scale);
+    }
     }
     PF_LAUNCHED(ctx);
-    const int MC = pick_mc(ctx);
-    sz = zpass_smem(ctx, MC);
-    PF_TRY(set_smem((const void *)k_zfwd, sz));
-    dim3 gz((g.M + MC - 1) / MC, g.N, ncomp);
-    {
+    switch (g.Z) {
+#define PF_CASE(L)                                                                                               \
+    case L: {                                                                                                    \
+        const RowsLaunch r = zrows_plan<L>(g);                                                                   \
+        PF_TRY(set_smem((const void *)k_zfwd_rows<L>, r.smem));                                                  \
+        ProfScope ps_(ctx, PF_K_ZFWD);                                                                           \
+        k_zfwd_rows<L><<<dim3((g.M + r.MC - 1) / r.MC, g.N, ncomp), r.threads, r.smem, ctx->stream>>>(T, dp, g,  \
+                                                                                          ctx->twZ, r.MC);       \
+    } break;
+        PF_FFT_LENGTHS(PF_CASE)
+#undef PF_CASE
+    default: {
+        const int MC = pick_mc(ctx);
+        const size_t sz = zpass_smem(ctx, MC);
+        PF_TRY(set_smem((const void *)k_zfwd, sz));
         ProfScope ps_(ctx, PF_K_ZFWD);
-        k_zfwd<<<gz, FFT_THREADS, sz, ctx->stream>>>((const double2 *)ctx->T, dp, g, ctx->planZ, ctx->twZ, MC);
+        k_zfwd<<<dim3((g.M + MC - 1) / MC, g.N, ncomp), FFT_THREADS, sz, ctx->stream>>>(T, dp, g, ctx->planZ, ctx->twZ,
+                                                                                         MC);
+    }
     }
     PF_LAUNCHED(ctx);
     return PF_OK;

@@ -24,6 +24,7 @@
 // are kept per device ordinal for the life of the process; a cudaDeviceReset
 // in the caller discards the tables, and this entry point is not usable on
 // that device after one.
+#include <algorithm>
 #include <cmath>
 #include <mutex>
 #include "pf_internal.cuh"
@@ -90,81 +91,112 @@ static int scratch_address(int dev, unsigned char **out) {
     return PF_OK;
 }
 
-// z pass: reference coll layout in (re[nh*N+n], im[...]), (m, z) columns out
+// z pass: reference coll layout in (re[nh*N+n], im[...]), (m, z) columns out.
+// A block takes MC columns of four consecutive radial points, since n is the
+// fastest index of the input: a 32-byte sector then serves four rows of the
+// block (one radial point per block read each sector four times: 9.2 us a
+// field at N=64, K=64, M=32, now 6.3).
+static constexpr int NA_NR = 4;
 template <int ZL>
 __global__ void __launch_bounds__(256) k_na_zinv(const double *__restrict__ re, const double *__restrict__ im,
                                                  double2 *__restrict__ T, const double2 *__restrict__ twz, int N,
-                                                 int K, int M, int MC) {
+                                                 int M, int MC) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    double2 *buf = reinterpret_cast<double2 *>(smraw);
-    double2 *tmp = buf + MC * ZL, *tw = tmp + MC * ZL;
-    const int n = blockIdx.y, m0 = blockIdx.x * MC;
+    using FR = RowsIO<ZL, double2>;
+    constexpr int K = ZL / 3;
+    double2 *rows = reinterpret_cast<double2 *>(smraw);
+    double2 *tw = rows + (FR::smem_elems(MC * NA_NR) - ZL);
+    const int n0 = blockIdx.y * NA_NR, m0 = blockIdx.x * MC;
     const int mc = min(MC, M - m0);
-    for (int i = threadIdx.x; i < ZL; i += blockDim.x) tw[i] = twz[i];
-    for (int idx = threadIdx.x; idx < mc * ZL; idx += blockDim.x) {
-        const int c = idx / ZL, j = idx - c * ZL;
-        const int m = m0 + c;
-        double2 v = make_double2(0.0, 0.0);
-        int nh = -1;
-        bool conj = false;
-        if (m == 0) {
-            if (j < K) nh = j;
-            else if (j >= 2 * K + 1) {
-                nh = ZL - j;
-                conj = true;
+    FR::table(tw, twz);
+    FR::template run<+1>(
+        rows, mc * NA_NR, tw,
+        [&](int b, int j) -> double2 {  // zero-padded in k, the Hermitian fill at m = 0
+            const int m = m0 + b / NA_NR, n = min(n0 + b % NA_NR, N - 1);
+            const int kk = j < K ? j : j - ZL;
+            const bool zero = j >= K && j <= 2 * K, conj = m == 0 && kk < 0;
+            double2 v = make_double2(0.0, 0.0);
+            if (!zero) {
+                const size_t at = (size_t)(conj ? -kk : m * (2 * K - 1) + kk) * N + n;
+                v = make_double2(re[at], im[at]);
             }
-        } else if (j < K) {
-            nh = m * (2 * K - 1) + j;
-        } else if (j >= 2 * K + 1) {
-            nh = m * (2 * K - 1) + (j - ZL);
-        }
-        if (nh >= 0) {
-            v = make_double2(re[(size_t)nh * N + n], im[(size_t)nh * N + n]);
-            if (conj) v.y = -v.y;
-        }
-        buf[idx] = v;
-    }
-    __syncthreads();
-    const double2 *res = smem_fft_t<ZL, +1>(buf, tmp, mc, tw);
-    double2 *out = T + ((size_t)n * M + m0) * ZL;
-    for (int idx = threadIdx.x; idx < mc * ZL; idx += blockDim.x) out[idx] = res[idx];
+            v.y = conj ? -v.y : v.y;
+            return v;
+        },
+        [&](int b, int j, int step, auto &v) {
+            const int m = m0 + b / NA_NR, n = n0 + b % NA_NR;
+            if (n >= N) return;
+            double2 *out = T + ((size_t)n * M + m) * ZL + j;
+#pragma unroll
+            for (int q = 0; q < (int)(sizeof(v) / sizeof(double2)); ++q) out[step * q] = v[q];
+        });
 }
 
-// theta pass (c2r, two real rows per complex FFT) into the phys layout
+// theta pass (c2r, two real rows per complex FFT) into the phys layout:
+// NA_ZC rows of one radial point per block, four warps, which is what eight
+// packed rows of the row transform keep busy (256 threads and the radix-4
+// passes: 12.1 us a field, now 7.1)
+static constexpr int NA_ZC = 16, NA_TH_THREADS = 128;
 template <int TL>
-__global__ void __launch_bounds__(256) k_na_thinv(const double2 *__restrict__ T, double *__restrict__ phys,
-                                                  const double2 *__restrict__ twt, int M, int Z, int ZC) {
+__global__ void __launch_bounds__(NA_TH_THREADS) k_na_thinv(const double2 *__restrict__ T, double *__restrict__ phys,
+                                                            const double2 *__restrict__ twt, int Z) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    const int np = ZC / 2;
+    using FR = FFTRows<TL, double2>;
+    constexpr int M = TL / 3, np = NA_ZC / 2, RS = FR::pitch;
     double2 *buf = reinterpret_cast<double2 *>(smraw);
-    double2 *tmp = buf + np * TL, *tw = tmp + np * TL;
-    const int n = blockIdx.y, z0 = blockIdx.x * ZC;
-    for (int i = threadIdx.x; i < TL; i += blockDim.x) tw[i] = twt[i];
-    for (int i = threadIdx.x; i < np * TL; i += blockDim.x) buf[i] = make_double2(0.0, 0.0);
-    __syncthreads();
+    double2 *tw = buf + (FR::smem_elems(np) - 2 * TL), *tw2 = tw + TL;
+    const int n = blockIdx.y, z0 = blockIdx.x * NA_ZC;
+    fft4_tables<TL>(tw, tw2, twt);
+    // mode m's thread also clears X[M + m] of the zero band (m = 0 X[2M])
+#pragma unroll 4
     for (int idx = threadIdx.x; idx < M * np; idx += blockDim.x) {
         const int zp = idx % np, m = idx / np;
         const int za = z0 + 2 * zp, zb = za + 1;
         const double2 *col = T + ((size_t)n * M + m) * Z;
         const double2 a = (za < Z) ? col[za] : make_double2(0.0, 0.0);
         const double2 b = (zb < Z) ? col[zb] : make_double2(0.0, 0.0);
-        double2 *X = buf + zp * TL;
+        double2 *X = buf + zp * RS;
+        X[M + m] = make_double2(0.0, 0.0);
         if (m == 0) {
             X[0] = make_double2(a.x, b.x);
+            X[2 * M] = make_double2(0.0, 0.0);
         } else {
             X[m] = make_double2(a.x - b.y, a.y + b.x);
             X[TL - m] = make_double2(a.x + b.y, -a.y + b.x);
         }
     }
     __syncthreads();
-    const double2 *res = smem_fft_t<TL, +1>(buf, tmp, np, tw);
-    for (int idx = threadIdx.x; idx < TL * ZC; idx += blockDim.x) {
-        const int zz = idx % ZC, t = idx / ZC;
+    FR::template run<+1>(buf, np, tw, tw2);
+    for (int idx = threadIdx.x; idx < TL * NA_ZC; idx += blockDim.x) {
+        const int zz = idx % NA_ZC, t = idx / NA_ZC;
         const int z = z0 + zz;
         if (z >= Z) continue;
-        const double2 v = res[(zz / 2) * TL + t];
+        const double2 v = buf[(zz / 2) * RS + t];
         phys[((size_t)n * TL + t) * Z + z] = (zz & 1) ? v.y : v.x;
     }
+}
+
+template <int L>
+static int na_zinv(const double *re, const double *im, double2 *T, const double2 *tw, int N, int M, cudaStream_t st) {
+    using FR = RowsIO<L, double2>;
+    // threads a row keeps busy; enough columns for a block, and blocks for the GPU
+    const int per = FR::four ? FR::L2 : L / 8, nb = (N + NA_NR - 1) / NA_NR;
+    int MC = std::min(M, std::max(1, 256 / (per * NA_NR)));
+    while (MC > 1 && (M + MC - 1) / MC * nb < 2 * 148) MC = (MC + 1) / 2;
+    const int threads = std::min(256, (MC * NA_NR * per + 31) / 32 * 32);
+    const size_t sm = FR::smem_elems(MC * NA_NR) * sizeof(double2);
+    PF_TRY(pf_raise_smem((const void *)k_na_zinv<L>, sm));
+    k_na_zinv<L><<<dim3((M + MC - 1) / MC, nb), std::max(threads, 32), sm, st>>>(re, im, T, tw, N, M, MC);
+    PF_CHECK_LAUNCH();
+    return PF_OK;
+}
+
+template <int L> static int na_thinv(const double2 *T, double *phys, const double2 *tw, int N, int Z, cudaStream_t st) {
+    const size_t sm = FFTRows<L, double2>::smem_elems(NA_ZC / 2) * sizeof(double2);
+    PF_TRY(pf_raise_smem((const void *)k_na_thinv<L>, sm));
+    k_na_thinv<L><<<dim3((Z + NA_ZC - 1) / NA_ZC, N), NA_TH_THREADS, sm, st>>>(T, phys, tw, Z);
+    PF_CHECK_LAUNCH();
+    return PF_OK;
 }
 
 static bool na_length_ok(int L) {
@@ -203,32 +235,21 @@ extern "C" int pf_tra_coll2phys_noalloc(int N, int K, int M, const double *re, c
     const double2 *twz = tables + twiddle_offset(Z);
     const double2 *twt = tables + twiddle_offset(Th);
     double2 *T = reinterpret_cast<double2 *>(scratch + kTwiddleBytes);
-    int MC = M;
-    while (MC > 1 && (size_t)(2 * MC + 1) * Z * sizeof(double2) > 60 * 1024) --MC;
-    const size_t zsm = (size_t)(2 * MC + 1) * Z * sizeof(double2);
-    const dim3 gz((M + MC - 1) / MC, N);
     switch (Z) {
-#define PF_CASE(L)                                                                                        \
-    case L:                                                                                               \
-        PF_TRY(pf_raise_smem((const void *)k_na_zinv<L>, zsm));                                          \
-        k_na_zinv<L><<<gz, 256, zsm, st>>>(re, im, T, twz, N, K, M, MC);                                   \
+#define PF_CASE(L)                                          \
+    case L:                                                 \
+        PF_TRY((na_zinv<L>(re, im, T, twz, N, M, st)));     \
         break;
         PF_NA_LENGTHS(PF_CASE)
 #undef PF_CASE
     }
-    PF_CHECK_LAUNCH();
-    const int ZC = 16;
-    const size_t tsm = ((size_t)2 * (ZC / 2) + 1) * Th * sizeof(double2);
-    const dim3 gt((Z + ZC - 1) / ZC, N);
     switch (Th) {
-#define PF_CASE(L)                                                                                         \
-    case L:                                                                                                \
-        PF_TRY(pf_raise_smem((const void *)k_na_thinv<L>, tsm));                                          \
-        k_na_thinv<L><<<gt, 256, tsm, st>>>(T, phys, twt, M, Z, ZC);                                        \
+#define PF_CASE(L)                                          \
+    case L:                                                 \
+        PF_TRY((na_thinv<L>(T, phys, twt, N, Z, st)));      \
         break;
         PF_NA_LENGTHS(PF_CASE)
 #undef PF_CASE
     }
-    PF_CHECK_LAUNCH();
     return PF_OK;
 }
