@@ -96,6 +96,7 @@ __device__ __forceinline__ bool mbar_wait(unsigned mbar, unsigned parity) {
                      : "=r"(done) : "r"(mbar), "r"(parity) : "memory");
     return done != 0;
 }
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p)); }
 __device__ __forceinline__ void mbar_arrive(unsigned mbar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(mbar) : "memory");
 }
@@ -272,34 +273,43 @@ __device__ __forceinline__ double sq(double2 a) { return fma(a.x, a.x, __dmul_rn
 // NaN corrector error instead of a converged one
 __device__ __forceinline__ double nanmax(double a, double b) { return (b > a || b != b) ? b : a; }
 
-// Row n of a radial band, zero beyond the ends (and for n >= N).  Loaded a
-// row ahead of its use: the tables come from L2 more often than not, as the
-// blocks' shared memory leaves little L1.
+// A radial band in shared memory, ten doubles a row: the nine weights of rows
+// js .. js+8, js = row_start(n), zeros outside the band, and a power of r.
+// The window never leaves the field, so a product has no bounds to test, and a
+// row is five 16-byte reads that half a warp shares; read from global memory
+// (L2: the blocks' shared memory leaves little L1) with the bounds of each
+// entry, the rows were most of the instructions of the stages and what they
+// waited for (N=64, 12113 modes: 176 -> 163 us).
+static constexpr int STEP_ROW = 2 * 10 * 8;  // bytes a radial point of the two tables
+__device__ __forceinline__ int row_start(int n, int N) { return min(max(n - KL, 0), N - NBAND); }
 struct BandRow {
-    double w[NBAND];
-    __device__ __forceinline__ void load(const double *__restrict__ band, int N, int n) {
+    double w[NBAND + 1];
+    __device__ __forceinline__ explicit BandRow(const double *tab, int n) {
+        const double2 *t = reinterpret_cast<const double2 *>(tab + n * 10);
 #pragma unroll
-        for (int d = -KL; d <= KL; ++d) {
-            const int j = n + d;
-            w[d + KL] = j >= 0 && j < N && n < N ? __ldg(band + (KL - d) * N + j) : 0.0;
+        for (int i = 0; i < 5; ++i) {
+            const double2 v = t[i];
+            w[2 * i] = v.x;
+            w[2 * i + 1] = v.y;
         }
     }
+    __device__ __forceinline__ double power() const { return w[NBAND]; }
     // sum_j band(n, j) x(j), j ascending, x a field at this thread's slot
-    __device__ __forceinline__ double2 apply(int N, int n, const double2 *x) const {
+    __device__ __forceinline__ double2 apply(int js, const double2 *x) const {
         double2 acc = make_double2(0.0, 0.0);
 #pragma unroll
-        for (int d = -KL; d <= KL; ++d) {
-            const int j = n + d;
-            if (j < 0 || j >= N) continue;
-            const double2 v = x[j * 16];
-            acc.x = fma(w[d + KL], v.x, acc.x);
-            acc.y = fma(w[d + KL], v.y, acc.y);
+        for (int i = 0; i < NBAND; ++i) {
+            const double2 v = x[js * 16 + i * 16];
+            acc.x = fma(w[i], v.x, acc.x);
+            acc.y = fma(w[i], v.y, acc.y);
         }
         return acc;
     }
 };
+static_assert(NBAND == 9, "rows of ten doubles");
 
-// Dynamic shared memory of a block: StepHead, four fields b0..b3 of [N][16]
+// Dynamic shared memory of a block: StepHead, the rows of the radial Laplacian
+// (with r^-2) and derivative (r^-1), four fields b0..b3 of [N][16]
 // double2, the pressure ring of `ppe` bytes, then three Helmholtz rings of
 // `ld` bytes each if there is room for them (`apart`); else these share b3
 // and the pressure ring, once both are done with.
@@ -314,6 +324,7 @@ static constexpr int STEP_HEAD = 3584;
 static_assert(sizeof(StepHead) <= STEP_HEAD, "block header");
 struct StepSmem {
     int ppe, ld, apart;
+    int far;  // the launch works on more than L2 holds
 };
 
 // 16 slots by NT/16 row groups; W = 16: a tile of m = 0.  Products that feed
@@ -337,7 +348,9 @@ __device__ __forceinline__ void step_tile(const StepArgs &a, int tile, const Ste
     static_assert(NT >= 192, "a solving and a filling warp for each system");
     const int role = warp < 6 ? (warp + tile) % 6 : 6;
     const bool lane0 = (threadIdx.x & 31) == 0;
-    double2 *const b0 = reinterpret_cast<double2 *>(step_sm + STEP_HEAD) + slot;
+    const int fields = STEP_HEAD + N * STEP_ROW;
+    double *const lap = reinterpret_cast<double *>(step_sm + STEP_HEAD), *const der = lap + N * 10;
+    double2 *const b0 = reinterpret_cast<double2 *>(step_sm + fields) + slot;
     double2 *const b1 = b0 + N * 16, *const b2 = b1 + N * 16, *const b3 = b2 + N * 16;
     const unsigned sbase = (unsigned)__cvta_generic_to_shared(step_sm);
     int nh, k, m;
@@ -370,7 +383,7 @@ __device__ __forceinline__ void step_tile(const StepArgs &a, int tile, const Ste
         s.ft = (sys == 0 ? a.lnp : pick3(a.ld, sys - 1)) + ftile;
         s.flags = sys == 0 ? 3 : pick3(a.ldpiv, sys - 1);
         const int bytes = sys == 0 ? lay.ppe : lay.ld;
-        s.ring = sbase + STEP_HEAD + N * 1024;
+        s.ring = sbase + fields + N * 1024;
         if (sys > 0) s.ring += (lay.apart ? lay.ppe : -N * 256) + (sys - 1) * lay.ld;
         s.places = bytes >= RING * group_bytes(W) ? RING : 2;
         s.g = bytes / (s.places * group_bytes(W));
@@ -388,9 +401,13 @@ __device__ __forceinline__ void step_tile(const StepArgs &a, int tile, const Ste
         int h, kk, mm;
         if (tile_mode(g, tile, i & 15, h, kk, mm)) hd.ainv[i & 15][i >> 4] = h != 0 ? a.Ainv[(size_t)(i >> 4) * Hp + h] : 0.0;
     }
-    const double *__restrict__ radLap = a.dm.radLap;
-    const double *__restrict__ drb = a.dm.dr;
     const double *__restrict__ rp = a.dm.rp;
+    for (int i = threadIdx.x; i < 20 * N; i += NT) {  // the rows, column by column
+        const int c = i / N, n = i - c * N, t = c >= 10, j = row_start(n, N) + c - 10 * t;
+        const bool in = j >= n - KL && j <= n + KL;
+        const double *__restrict__ src = c == 9 || c == 19 ? rp + (t ? 2 : 1) * N + n : (t ? a.dm.dr : a.dm.radLap) + (in ? (KL + n - j) * N + j : 0);
+        lap[(t * N + n) * 10 + c - 10 * t] = in || c == 9 || c == 19 ? __ldg(src) : 0.0;
+    }
     const double mMp = (double)(m * g.Mp), kal = g.alpha * k, c2 = a.c2;
     // diagonal of Lt for the uz system at row n: c1 - c2 ((m Mp)^2/r^2 + (alpha k)^2)
     const double mm2 = __dmul_rn(mMp, mMp), kk2 = __dmul_rn(kal, kal);
@@ -406,8 +423,6 @@ __device__ __forceinline__ void step_tile(const StepArgs &a, int tile, const Ste
         if (a.mode == 1) vP = __ldcs(pick3(a.N_, c) + at);
     };
     load_N(2, ty);
-    BandRow next;
-    next.load(radLap, N, ty);
     cp_async_wait_all();
     __syncthreads();
     // st 0: rhs of uz, b1 -> b2; st 1: the off-diagonal part of Lt u_r plus
@@ -423,10 +438,9 @@ __device__ __forceinline__ void step_tile(const StepArgs &a, int tile, const Ste
             const double2 P = vP;
             const bool last = n + NR >= N;
             if (!last || st < 2) load_N(last ? st : comp, last ? ty : n + NR);
-            const BandRow row = next;
-            next.load(last && st == 2 ? drb : radLap, N, last ? ty : n + NR);
-            const double2 s = row.apply(N, n, src);
-            const double r2 = rp[N + n], d = diag0(r2);
+            const BandRow row(lap, n);
+            const double2 s = row.apply(row_start(n, N), src);
+            const double r2 = row.power(), d = diag0(r2);
             if (a.mode == 1) {  // N = c N + (1-c) N_
                 const double d1 = a.implicit, d2 = 1.0 - a.implicit;
                 v = make_double2(fma(d1, v.x, __dmul_rn(d2, P.x)), fma(d1, v.y, __dmul_rn(d2, P.y)));
@@ -449,22 +463,35 @@ __device__ __forceinline__ void step_tile(const StepArgs &a, int tile, const Ste
         }
         __syncthreads();
     }
+    // the last stage's reads, brought to L2 under the solves where they come
+    // from DRAM (64 pipes, N=64: 254 -> 247 us, N=32: 190 -> 181); from L2 they
+    // are quick enough, and asking costs more (N=48, 2985 modes: 40 -> 43).
+    // The slots at the ends of a row's runs cover its lines.
+    if (lay.far && live && nh != 0 && (slot < 2 || slot >= 14 || (W == 16 && slot == 8)))
+        for (int n = ty; n < N; n += NR) {
+            const size_t at = (size_t)n * Hp + nh;
+            if (k >= 0)
+#pragma unroll
+                for (int i = 0; i < 6; ++i) prefetch_l2(a.U + (size_t)i * N * Hp + at);
+            if (a.mode == 1)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) prefetch_l2(a.u[c] + at);
+        }
     // div(pm2rt(rhs)) (velocity.f90:98-114; variables.f90:472-477) with
     // tim_zerobc: b0, b1, b2 -> b3
 #pragma unroll 1
     for (int n = ty; n < N; n += NR) {
-        const BandRow row = next;
-        next.load(drb, N, n + NR);
+        const BandRow row(der, n);
         double2 dv = make_double2(0.0, 0.0);
         if (n != 0 && n != N - 1) {
             double2 s = make_double2(0.0, 0.0);
 #pragma unroll 1
             for (int f = 0; f < 2; ++f) {
-                const double2 e = row.apply(N, n, f ? b1 : b0);
+                const double2 e = row.apply(row_start(n, N), f ? b1 : b0);
                 s.x += e.x;
                 s.y += e.y;
             }
-            const double rm1 = rp[2 * N + n], m1r1 = rm1 * mMp;
+            const double rm1 = row.power(), m1r1 = rm1 * mMp;
             const double2 p = b0[n * 16], q = b1[n * 16], z = b2[n * 16];
             const double tx = 0.5 * (p.y - q.y), ty_ = -0.5 * (p.x - q.x);
             dv.x = fma(-z.y, kal, fma(-ty_, m1r1, fma(0.5 * (p.x + q.x), rm1, 0.5 * s.x)));
@@ -475,25 +502,23 @@ __device__ __forceinline__ void step_tile(const StepArgs &a, int tile, const Ste
     __syncthreads();
     // LNp of k = m = 0 is held as zeros, so its pressure is zero (timestep.f90:110-113)
     if (role == 0) {
-        ok &= tile_solve<true, true, W>(stream(0), STEP_HEAD + 3 * N * 256);
+        ok &= tile_solve<true, true, W>(stream(0), fields + 3 * N * 256);
     } else if (role == 3 && lane0) {
         ok &= stream_fill(stream(0), stream(0).places, 1 << 30);
     }
     __syncthreads();
     // rhs - rt2pm(grad p), grad p = (dr p, i m/r p, i alpha k p); zero boundary rows
-    next.load(drb, N, ty);
 #pragma unroll 1
     for (int n = ty; n < N; n += NR) {
         const int e = n * 16;
-        const BandRow row = next;
-        next.load(drb, N, n + NR);
+        const BandRow row(der, n);
         if (n == 0 || n == N - 1) {
             b0[e] = b1[e] = b2[e] = make_double2(0.0, 0.0);
             continue;
         }
-        const double2 s = row.apply(N, n, b3);
+        const double2 s = row.apply(row_start(n, N), b3);
         const double2 pv = b3[e];
-        const double m1r1 = rp[2 * N + n] * mMp;
+        const double m1r1 = row.power() * mMp;
         const double2 vp = b0[e], vm = b1[e], vz = b2[e];
         b0[e] = make_double2(vp.x - fma(-pv.x, m1r1, s.x), vp.y - fma(-pv.y, m1r1, s.y));
         b1[e] = make_double2(vm.x - fma(pv.x, m1r1, s.x), vm.y - fma(pv.y, m1r1, s.y));
@@ -505,7 +530,7 @@ __device__ __forceinline__ void step_tile(const StepArgs &a, int tile, const Ste
     __syncthreads();
     if (role < 3) {
         const FactorStream s = stream(1 + role);
-        const int f = STEP_HEAD + role * N * 256;
+        const int f = fields + role * N * 256;
         if (s.flags == 0) ok &= tile_solve<false, false, W>(s, f);
         else if (s.flags == 1) ok &= tile_solve<true, false, W>(s, f);
         else ok &= tile_solve<true, true, W>(s, f);  // low Re, small dt or very clustered meshes
@@ -548,7 +573,7 @@ __device__ __forceinline__ void step_tile(const StepArgs &a, int tile, const Ste
         }
     }
     if (W == 16 && tile == 0 && warp == 1) {  // the tile of k = m = 0 (slot 0)
-        const double2 *z = reinterpret_cast<const double2 *>(step_sm + STEP_HEAD) + 2 * N * 16;
+        const double2 *z = reinterpret_cast<const double2 *>(step_sm + fields) + 2 * N * 16;
         double s = 0.0;
         for (int n = threadIdx.x & 31; n < N; n += 32) s = fma(z[n * 16].x, a.dm.intrdr[n], s);
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
@@ -614,18 +639,17 @@ __device__ __forceinline__ void step_tile(const StepArgs &a, int tile, const Ste
     if (a.mode == 0 && a.curl[0]) {
         // curl(u) and the mean mode's sums over this tile (k_nl_prep's, while
         // u is still on the chip)
-        next.load(drb, N, ty);
         __syncthreads();
 #pragma unroll 1
         for (int n = ty; n < ((N + 1) & ~1); n += NR) {  // whole warps: the half-warps sum together
-            const BandRow row = next;
-            next.load(drb, N, n + NR);
+            const BandRow row(der, min(n, N - 1));
             double s[3] = {0.0, 0.0, 0.0};
             if (live && n < N) {
                 const size_t at = (size_t)n * Hp + nh;
-                const double2 dt = row.apply(N, n, b1), dz = row.apply(N, n, b2);
+                const int js = row_start(n, N);
+                const double2 dt = row.apply(js, b1), dz = row.apply(js, b2);
                 const double2 ur = b0[n * 16], ut = b1[n * 16], uz = b2[n * 16];
-                const double rm1 = rp[2 * N + n];
+                const double rm1 = row.power();
                 const Curl c = mode_curl(ur, ut, uz, dt, dz, rm1, rm1 * mMp, kal);
                 if (a.mixed) {
                     reinterpret_cast<float2 *>(a.curl[0])[at] = make_float2((float)c.r.x, (float)c.r.y);
@@ -689,7 +713,7 @@ __global__ void __launch_bounds__(NT, MINB) k_step_batch(const StepArgs *__restr
 // ------------------------------------------------------------------ host
 static constexpr int STEP_MAX_N = 128;
 
-// (N limit, threads, resident blocks): shared memory, 1 KB a radial point
+// (N limit, threads, resident blocks): shared memory, 1.2 KB a radial point
 // plus the rings, allows that many blocks
 #define PF_STEP_SHAPES(X) X(32, 192, 4) X(64, 256, 2) X(128, 256, 1)
 
@@ -698,21 +722,23 @@ static constexpr int STEP_MAX_N = 128;
 // from the fields where each then has two groups a chunk, or half a sweep:
 // a block alone on its SM has its whole factors in flight from the start.
 static constexpr size_t SM_SMEM = 228 * 1024;
-static StepSmem step_rings(int N, int blocks) {
-    const int room = (int)std::min(SM_SMEM / blocks - 1024, (size_t)227 * 1024) - STEP_HEAD - N * 1024;
+// `tiles` of 16 modes read and write about 470 bytes a mode and radial point.
+static StepSmem step_rings(int N, int blocks, size_t tiles) {
+    const int room = (int)std::min(SM_SMEM / blocks - 1024, (size_t)227 * 1024) - STEP_HEAD - N * (1024 + STEP_ROW);
     const int unit = RING * group_bytes(8);  // one group a chunk for W = 8
     const int half = 2 * ((N + 19) / 20);    // groups of half a forward sweep, an even number
     StepSmem l{};
+    l.far = tiles * 16 * N * 470 > ((size_t)126 << 20);
     const int each = std::min(room / 4 / unit, half);
     l.apart = each >= std::min(2, half);
     l.ppe = std::max(l.apart ? each : room / unit, 1) * unit;
     // a stream needs two chunks of a group of 16 matrices: fewer blocks then fit
-    while (!l.apart && (N * 256 + l.ppe) / 3 < 2 * group_bytes(16) + 128) l.ppe += unit;
+    if (!l.apart) l.ppe = std::max(l.ppe, (3 * (2 * group_bytes(16) + 128) - N * 256 + 127) & ~127);
     l.ld = l.apart ? l.ppe : ((N * 256 + l.ppe) / 3) & ~127;
     return l;
 }
 static size_t step_smem(int N, const StepSmem &l) {
-    return (size_t)STEP_HEAD + N * 1024 + l.ppe + (l.apart ? 3 * l.ld : 0);
+    return (size_t)STEP_HEAD + N * (1024 + STEP_ROW) + l.ppe + (l.apart ? 3 * l.ld : 0);
 }
 
 static StepArgs make_step_args(const pf_ctx *ctx, int corrector) {
@@ -769,13 +795,13 @@ int pf_vel_step_fused(pf_ctx *ctx, int corrector) {
         ProfScope ps_(ctx, PF_K_STEP);
 #define PF_CASE(NMAX, NT, MINB)                                             \
     else if (g.N <= NMAX) {                                                 \
-        const StepSmem lay = step_rings(g.N, MINB);                         \
+        const StepSmem lay = step_rings(g.N, MINB, blocks);                         \
         const size_t sm = step_smem(g.N, lay);                              \
         PF_TRY(pf_raise_smem((const void *)k_step<NT, MINB>, sm));          \
         k_step<NT, MINB><<<blocks, NT, sm, ctx->stream>>>(a, lay);          \
     }
         if (blocks <= sms) {  // a block to an SM: all its threads and shared memory for latency
-            const StepSmem lay = step_rings(g.N, 1);
+            const StepSmem lay = step_rings(g.N, 1, blocks);
             const size_t sm = step_smem(g.N, lay);
             PF_TRY(pf_raise_smem((const void *)k_step<256, 1>, sm));
             k_step<256, 1><<<blocks, 256, sm, ctx->stream>>>(a, lay);
@@ -875,7 +901,7 @@ int pf_step_batch_build(pf_ctx *const *pipes, int n, pf_aux *aux, pf_step_batch 
 static int step_group_launch(const StepGroup &gr, const StepArgs *a, const int *act, cudaStream_t st) {
 #define PF_CASE(NMAX, NT, MINB)                                                \
     else if (gr.N <= NMAX) {                                                   \
-        const StepSmem lay = step_rings(gr.N, MINB);                           \
+        const StepSmem lay = step_rings(gr.N, MINB, gr.nblk);                           \
         const size_t sm = step_smem(gr.N, lay);                                \
         if (gr.W == 16) {                                                      \
             PF_TRY(pf_raise_smem((const void *)k_step_batch<NT, MINB, 16>, sm)); \
