@@ -346,6 +346,32 @@ template <typename T> __device__ __forceinline__ T pick3(T const (&p)[3], int i)
     return i == 0 ? p[0] : (i == 1 ? p[1] : p[2]);
 }
 
+// The lone pipe's step is set up while the kernel before it drains
+// (launch_chained): its blocks start once every block of that kernel has passed
+// chain_open, make ready what the matrices alone decide, and touch what the
+// kernel reads or writes only after chain_wait, which returns when all of it
+// has finished and which every block calls.  Two steps of N=48 with 2985 modes
+// 566 -> 541 us, four of N=40 446 -> 414, of N=16 279 -> 267.  The transform
+// passes launched so gain nothing or lose (all of them chained as well: N=48
+// 590 us): several of their blocks share an SM, and blocks that start early
+// crowd the SMs that come free first.
+__device__ __forceinline__ void chain_open() { asm volatile("griddepcontrol.launch_dependents;\n" ::); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // x / d for 0 <= x < 2^22 and d > 0, given inv = 1.0f / d: a float
 // reciprocal estimate corrected by one step (cheaper than a run-time integer
 // division inside index loops)

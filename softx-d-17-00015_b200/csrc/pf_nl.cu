@@ -480,10 +480,12 @@ __global__ void __launch_bounds__(NL_THREADS, (NLOcc<C, TL>::theta)) k_nl_theta(
 }
 template <int ZL, typename C>
 __global__ void __launch_bounds__(NL_THREADS, (NLOcc<C, ZL>::zfwd)) k_nl_zfwd(NLArgs a) {
+    chain_open();
     nl_zfwd_body<ZL, C>(a, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 template <int ZL, int TL>
 __global__ void __launch_bounds__(FUSED_THREADS, 1) k_nl_fused(NLArgs a) {
+    chain_open();
     nl_fused_body<ZL, TL>(a, blockIdx.x);
 }
 
@@ -892,6 +894,7 @@ template <bool MIXED> __global__ void __launch_bounds__(PREP_THREADS) k_nl_prep(
 }
 // one warp per radial point
 __global__ void __launch_bounds__(128) k_nl_mean64_fin(NLArgs a, int stepped) {
+    chain_open();
     const int n = blockIdx.x * 4 + (threadIdx.x >> 5);
     if (n < a.g.N) nl_mean64_fin_body(a, n, stepped);
 }

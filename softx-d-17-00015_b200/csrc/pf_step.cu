@@ -333,7 +333,9 @@ struct StepSmem {
 // the rows it needs of other threads from fields nobody writes in that stage,
 // so a stage is one short loop over the thread's rows and one barrier; fully
 // unrolled rows held in registers took twice as long, waiting for instructions.
-template <int NT, int W>
+// CHAIN: launched behind the transforms (chain_wait), whose output and u are
+// asked for after the parts that only the matrices decide.
+template <int NT, int W, bool CHAIN>
 __device__ __forceinline__ void step_tile(const StepArgs &a, int tile, const StepSmem lay) {
     extern __shared__ __align__(128) unsigned char step_sm[];
     StepHead &hd = *reinterpret_cast<StepHead *>(step_sm);
@@ -363,17 +365,20 @@ __device__ __forceinline__ void step_tile(const StepArgs &a, int tile, const Ste
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     }
     // u_r, u_theta, u_z of the tile into b0, b3, b1
-    for (int n = ty; n < N; n += NR) {
-        const int e = n * 16;
-        if (live) {
-            const size_t at = (size_t)n * Hp + nh;
-            cp_async16((unsigned)__cvta_generic_to_shared(b0 + e), a.u_[0] + at);
-            cp_async16((unsigned)__cvta_generic_to_shared(b3 + e), a.u_[1] + at);
-            cp_async16((unsigned)__cvta_generic_to_shared(b1 + e), a.u_[2] + at);
-        } else {
-            b0[e] = b1[e] = b3[e] = make_double2(0.0, 0.0);
+    auto load_u = [&]() {
+        for (int n = ty; n < N; n += NR) {
+            const int e = n * 16;
+            if (live) {
+                const size_t at = (size_t)n * Hp + nh;
+                cp_async16((unsigned)__cvta_generic_to_shared(b0 + e), a.u_[0] + at);
+                cp_async16((unsigned)__cvta_generic_to_shared(b3 + e), a.u_[1] + at);
+                cp_async16((unsigned)__cvta_generic_to_shared(b1 + e), a.u_[2] + at);
+            } else {
+                b0[e] = b1[e] = b3[e] = make_double2(0.0, 0.0);
+            }
         }
-    }
+    };
+    if (!CHAIN) load_u();
     // the factor streams; those whose rings are free now are started
     const size_t ftile = (size_t)(W == 16 ? 16 * tile : 8 * (tile + nz)) * N * FT_ROWS;
     auto stream = [&](int sys) {  // 0: LNp, 1..3: LDp, LDm, LDz
@@ -422,6 +427,10 @@ __device__ __forceinline__ void step_tile(const StepArgs &a, int tile, const Ste
         vN = __ldcs(pick3(a.Nl, c) + at);
         if (a.mode == 1) vP = __ldcs(pick3(a.N_, c) + at);
     };
+    if (CHAIN) {
+        chain_wait();
+        load_u();
+    }
     load_N(2, ty);
     cp_async_wait_all();
     __syncthreads();
@@ -697,8 +706,8 @@ __device__ __forceinline__ void step_tile(const StepArgs &a, int tile, const Ste
 // allows at that size and the registers are capped for.
 template <int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) k_step(const __grid_constant__ StepArgs a, const StepSmem lay) {
-    if ((int)blockIdx.x < pf_mean_tiles(a.g)) step_tile<NT, 16>(a, blockIdx.x, lay);
-    else step_tile<NT, 8>(a, blockIdx.x, lay);
+    if ((int)blockIdx.x < pf_mean_tiles(a.g)) step_tile<NT, 16, true>(a, blockIdx.x, lay);
+    else step_tile<NT, 8, true>(a, blockIdx.x, lay);
 }
 
 template <int NT, int MINB, int W>
@@ -707,7 +716,7 @@ __global__ void __launch_bounds__(NT, MINB) k_step_batch(const StepArgs *__restr
     const int2 pb = blk[blockIdx.x];
     if (act && !act[pb.x]) return;
     const StepArgs a = args[pb.x];  // by value: stores through its pointers cannot alias it
-    step_tile<NT, W>(a, pb.y, lay);
+    step_tile<NT, W, false>(a, pb.y, lay);
 }
 
 // ------------------------------------------------------------------ host
@@ -798,13 +807,13 @@ int pf_vel_step_fused(pf_ctx *ctx, int corrector) {
         const StepSmem lay = step_rings(g.N, MINB, blocks);                         \
         const size_t sm = step_smem(g.N, lay);                              \
         PF_TRY(pf_raise_smem((const void *)k_step<NT, MINB>, sm));          \
-        k_step<NT, MINB><<<blocks, NT, sm, ctx->stream>>>(a, lay);          \
+        PF_CUDA(launch_chained(k_step<NT, MINB>, dim3(blocks), NT, sm, ctx->stream, a, lay)); \
     }
         if (blocks <= sms) {  // a block to an SM: all its threads and shared memory for latency
             const StepSmem lay = step_rings(g.N, 1, blocks);
             const size_t sm = step_smem(g.N, lay);
             PF_TRY(pf_raise_smem((const void *)k_step<256, 1>, sm));
-            k_step<256, 1><<<blocks, 256, sm, ctx->stream>>>(a, lay);
+            PF_CUDA(launch_chained(k_step<256, 1>, dim3(blocks), 256, sm, ctx->stream, a, lay));
         }
         PF_STEP_SHAPES(PF_CASE)
 #undef PF_CASE
