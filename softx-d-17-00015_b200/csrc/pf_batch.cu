@@ -17,8 +17,8 @@
 // bit-identical alone and in the batch.  After the replay one host
 // synchronisation reads every pipe's corrector error (gathered into one
 // pinned copy); the reference's corrector control (timestep.f90:214-253) is
-// then applied per pipe, and the rare pipe that needs another corrector pass
-// gets it on its own stream (main.f90:35-41).  In orbit mode every pipe takes
+// then applied per pipe, and the pipes that need another corrector pass take
+// it together (main.f90:35-41).  In orbit mode every pipe takes
 // exactly one corrector pass (newton.f90:740-762).
 #include <cmath>
 #include "pf_internal.cuh"
@@ -84,6 +84,8 @@ struct pf_batch {
     DevScalars *d_scall;             // gathered scalars
     int *d_act, *h_act;              // mask of a further corrector pass (h_act pinned)
     pf_stage_prof sprof;             // stage timing of the batched launches
+    double part_ms[PF_K_NCAT];       // of those that covered part of the batch (further corrector passes)
+    unsigned long long part_n[PF_K_NCAT];
     std::vector<pf_stage_prof::Open> sev[2][2];
     unsigned long long launches;     // batched kernels launched (not per pipe)
     struct BatchIO *io;              // pipelined state I/O (made on first use)
@@ -478,13 +480,14 @@ static std::vector<int> rel_parity(const pf_batch *b) {
     return r;
 }
 
-// Read the stage and kernel event pairs of a finished step into the totals.
-static void batch_collect_events(pf_batch *b, std::vector<pf_stage_prof::Open> *stage, bool release) {
+// Read the stage and kernel event pairs of a finished step into the totals
+// (of a pass over part of the batch: into its own).
+static void batch_collect_events(pf_batch *b, std::vector<pf_stage_prof::Open> *stage, bool release, bool part = false) {
     for (auto &e : *stage) {
         float ms = 0.f;
         if (cudaEventElapsedTime(&ms, e.a, e.b) == cudaSuccess) {
-            b->sprof.ms[e.cat] += ms;
-            b->sprof.n[e.cat] += 1;
+            (part ? b->part_ms : b->sprof.ms)[e.cat] += ms;
+            (part ? b->part_n : b->sprof.n)[e.cat] += 1;
         } else {
             cudaGetLastError();
         }
@@ -497,11 +500,13 @@ static void batch_collect_events(pf_batch *b, std::vector<pf_stage_prof::Open> *
 }
 
 // One further corrector pass of every pipe in `act` (indexes), its scalars in
-// b->hsc.  Stage-batched: one masked launch per stage; a chain of small launches per pipe that
-// waited for the GPU each time was half of a step in which 39 of 64 mixed pipes
-// take a second pass (two such steps: 16.6 -> 10.9 ms).  Launched directly: recording
-// it costs the first pass of a batch more than a replay saves (8 FP64 pipes, a
-// new batch's first steps: 6.4 ms recorded, 5.1 ms direct; repeated 1.44-1.6).  Otherwise every pipe's pass on its own stream, all in flight together.
+// b->hsc.  Stage-batched: one masked launch per stage; a chain of small
+// launches per pipe that waited for the GPU each time was half of a step in
+// which 39 of 64 mixed pipes take a second pass (two such steps: 16.6 -> 10.9
+// ms).  Launched directly: recording it costs the first pass of a batch more
+// than a replay saves (8 FP64 pipes, a new batch's first steps: 6.4 ms
+// recorded, 5.1 direct; repeated 1.44-1.6 either way).  Otherwise every pipe's
+// pass on its own stream, all in flight together.
 static int batch_corrector(pf_batch *b, const std::vector<int> &act) {
     if (b->kind != 1) {
         for (int i : act) {
@@ -526,7 +531,7 @@ static int batch_corrector(pf_batch *b, const std::vector<int> &act) {
     PF_CUDA(cudaStreamSynchronize(b->master));
     std::vector<pf_stage_prof::Open> mine(b->sprof.open.begin() + open0, b->sprof.open.end());
     b->sprof.open.resize(open0);
-    batch_collect_events(b, &mine, true);
+    batch_collect_events(b, &mine, true, true);
     return PF_OK;
 }
 
@@ -722,8 +727,8 @@ extern "C" int pf_batch_prof_enable(pf_batch *b, int mask) {
     for (pf_ctx *c : b->pipes) PF_TRY(pf_prof_enable(c, mask));
     b->sprof.mask = mask;
     for (int c = 0; c < PF_K_NCAT; ++c) {
-        b->sprof.ms[c] = 0.0;
-        b->sprof.n[c] = 0;
+        b->sprof.ms[c] = b->part_ms[c] = 0.0;
+        b->sprof.n[c] = b->part_n[c] = 0;
     }
     return PF_OK;
 }
@@ -740,8 +745,8 @@ extern "C" int pf_batch_prof_read(pf_batch *b, int cat, double *ms, unsigned lon
         t += m;
         n += k;
     }
-    if (ms) *ms = t + b->sprof.ms[cat];
-    if (launches) *launches = n + b->sprof.n[cat];
+    if (ms) *ms = t + b->sprof.ms[cat] + b->part_ms[cat];
+    if (launches) *launches = n + b->sprof.n[cat] + b->part_n[cat];
     return PF_OK;
 }
 

@@ -110,10 +110,8 @@ int pf_build_mesh(int N, const double *custom_r, HostMesh &hm);
 // Entry A(r, c), |r - c| <= KL, 0 <= r, c < N, of the system c1 I + c2 Lap(PM)
 // for mode (k, m) with the axis-parity first row dr0(:, 1-S) and the wall row
 // dr1(:, BC) (timestep.f90:46-90).  Every product and sum is rounded
-// explicitly (no contraction into fma), so every kernel that assembles an
-// entry gets the same bits: the factorisation (k_lu_factor) and the fused
-// Helmholtz solve that rebuilds its factors on chip.  The matrices of (k, m)
-// and (-k, m) are bitwise equal.
+// explicitly (no contraction into fma); the matrices of (k, m) and (-k, m) are
+// bitwise equal.
 __device__ __forceinline__ double lumesh_entry(const DevMesh &dm, int N, int Mp, double alpha, int PM, int BC,
                                                double c1, double c2, int k, int m, int S, int r, int c) {
     if (r == 0) return dm.dr0[(1 - S) * (PF_KL + 1) + c];
