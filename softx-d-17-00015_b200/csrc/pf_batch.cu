@@ -410,7 +410,7 @@ static int staged_capture(pf_batch *b, int orbit, int par, cudaGraphExec_t *exec
 // one pipe's body of the batch graph
 static int pipe_body(pf_ctx *c, int orbit) {
     PF_TRY(pf_first_nonlinear(c));
-    PF_TRY(pf_vel_step_fused(c, 0));
+    PF_TRY(pf_vel_step_fused(c, 0, true));
     PF_TRY(pf_next_nonlinear(c));
     PF_TRY(pf_vel_step_fused(c, 1));
     if (orbit) PF_TRY(pf_vel_imposesym(c));

@@ -272,6 +272,7 @@ struct pf_ctx {
     // predictor, nonlinear terms, corrector starting from pointer parity p;
     // corr[q] = nonlinear terms + corrector at parity q
     int parity;                    // vel/prev pointer swap state
+    bool curl_left;                // the last predictor left curl(u) for the terms that follow it
     bool use_graphs, graph_warm;
     cudaGraphExec_t g_main[2], g_corr[2];
     unsigned long long g_main_n[2], g_corr_n[2];
@@ -517,7 +518,7 @@ void pf_step_batch_free(pf_step_batch *b);
 #define PF_NL_STEPPED 2
 int pf_launch_nl_fused(pf_ctx *ctx, int mode);
 void *pf_curl_field(const pf_ctx *ctx, int c);
-int pf_vel_step_fused(pf_ctx *ctx, int corrector);
+int pf_vel_step_fused(pf_ctx *ctx, int corrector, bool leave_curl = false);
 void pf_graphs_reset(pf_ctx *ctx);
 int pf_transform_nonlinear(pf_ctx *ctx);
 int pf_first_nonlinear(pf_ctx *ctx);

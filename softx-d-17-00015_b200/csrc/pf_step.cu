@@ -750,7 +750,8 @@ static size_t step_smem(int N, const StepSmem &l) {
     return (size_t)STEP_HEAD + N * (1024 + STEP_ROW) + l.ppe + (l.apart ? 3 * l.ld : 0);
 }
 
-static StepArgs make_step_args(const pf_ctx *ctx, int corrector) {
+// leave_curl: the fused transforms follow and read curl(u)
+static StepArgs make_step_args(const pf_ctx *ctx, int corrector, bool leave_curl) {
     StepArgs a;
     for (int i = 0; i < 3; ++i) {
         a.u_[i] = ctx->prev[i].d;
@@ -764,8 +765,8 @@ static StepArgs make_step_args(const pf_ctx *ctx, int corrector) {
         a.ld[i] = ld[i]->tiles;
         a.ldpiv[i] = ld[i]->pivoted;
     }
-    const bool follow = pf_nl_fused_supported(ctx) && !pf_util_active(ctx);  // the transforms that read curl(u)
-    for (int i = 0; i < 3; ++i) a.curl[i] = follow ? pf_curl_field(ctx, i) : nullptr;
+    leave_curl = leave_curl && pf_nl_fused_supported(ctx);
+    for (int i = 0; i < 3; ++i) a.curl[i] = leave_curl ? pf_curl_field(ctx, i) : nullptr;
     a.mixed = ctx->cfg.precision == PF_PREC_MIXED;
     a.mpart = ctx->mpart;
     a.U = ctx->U;
@@ -785,8 +786,9 @@ static StepArgs make_step_args(const pf_ctx *ctx, int corrector) {
 bool pf_fused_step_ok(const pf_ctx *ctx) { return ctx->g.N <= STEP_MAX_N; }
 
 // One predictor (corrector=0) or corrector (corrector=1) vel_step.  The
-// predictor's u_ := u copy is a pointer swap of vel[0..2] and prev[0..2].
-int pf_vel_step_fused(pf_ctx *ctx, int corrector) {
+// predictor's u_ := u copy is a pointer swap of vel[0..2] and prev[0..2]; what
+// it was given to leave is noted for pf_next_nonlinear.
+int pf_vel_step_fused(pf_ctx *ctx, int corrector, bool leave_curl) {
     const Geo &g = ctx->g;
     if (!pf_fused_step_ok(ctx)) {
         pf_set_error("fused step supports N <= %d", STEP_MAX_N);
@@ -796,7 +798,8 @@ int pf_vel_step_fused(pf_ctx *ctx, int corrector) {
         for (int i = 0; i < 3; ++i) std::swap(ctx->vel[i].d, ctx->prev[i].d);
         ctx->parity ^= 1;
     }
-    const StepArgs a = make_step_args(ctx, corrector);
+    const StepArgs a = make_step_args(ctx, corrector, leave_curl);
+    ctx->curl_left = !corrector && a.curl[0];
     const int blocks = pf_step_tiles(g);
     int sms = 0;
     PF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
@@ -854,7 +857,7 @@ static int step_batch_fill(pf_step_batch *b, pf_ctx *const *pipes, int n) {
             for (int i = 0; i < n; ++i) {
                 pf_ctx *c = pipes[i];
                 if (s) for (int k = 0; k < 3; ++k) std::swap(c->vel[k].d, c->prev[k].d);
-                args.push_back(make_step_args(c, m));
+                args.push_back(make_step_args(c, m, true));
                 if (s) for (int k = 0; k < 3; ++k) std::swap(c->vel[k].d, c->prev[k].d);
             }
     std::vector<int> sizes;

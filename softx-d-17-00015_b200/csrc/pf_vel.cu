@@ -88,14 +88,19 @@ static int vel_step(pf_ctx *ctx) {
 
 static bool fused_step_ok(const pf_ctx *ctx) { return pf_fused_step_ok(ctx); }
 
-// velocity.f90:400-410
-extern "C" int pf_vel_predictor(pf_ctx *ctx) {
-    PF_ARG(ctx, "null ctx");
+// velocity.f90:400-410; leave_curl: pf_next_nonlinear follows
+static int predictor(pf_ctx *ctx, bool leave_curl) {
     PF_TRY(require_matrices(ctx));
-    if (fused_step_ok(ctx)) return pf_vel_step_fused(ctx, 0);
+    if (fused_step_ok(ctx)) return pf_vel_step_fused(ctx, 0, leave_curl);
+    ctx->curl_left = false;
     for (int i = 0; i < 6; ++i)
         PF_TRY(pf_launch_ew(ctx, EW_COPY, ctx->vel[i].d, nullptr, ctx->prev[i].d, nullptr, 0.0));
     return vel_step(ctx);
+}
+
+extern "C" int pf_vel_predictor(pf_ctx *ctx) {
+    PF_ARG(ctx, "null ctx");
+    return predictor(ctx, false);
 }
 
 // velocity.f90:416-432 (tim_measurecorr folded into one device reduction)
@@ -150,8 +155,9 @@ int pf_first_nonlinear(pf_ctx *ctx) {
     PF_TRY(pf_vel_imposesym(ctx));
     return transform_nonlinear(ctx, PF_NL_FRESH);
 }
-// the terms of the velocity a predictor has just made
-int pf_next_nonlinear(pf_ctx *ctx) { return transform_nonlinear(ctx, fused_step_ok(ctx) ? PF_NL_STEPPED : PF_NL_FRESH); }
+// the terms of the velocity a predictor has just made, from the curl it left if
+// it was given to leave one
+int pf_next_nonlinear(pf_ctx *ctx) { return transform_nonlinear(ctx, ctx->curl_left ? PF_NL_STEPPED : PF_NL_FRESH); }
 
 extern "C" int pf_vel_transform_nonlinear(pf_ctx *ctx) {
     PF_ARG(ctx, "null ctx");
@@ -315,7 +321,7 @@ extern "C" int pf_timestep(pf_ctx *ctx, int *ncorr) {
             // nothing on the device)
             PF_TRY(capture(ctx, p, &ctx->g_main[p], &ctx->g_main_n[p], [&]() {
                 PF_TRY(main_nonlinear(ctx, NL_FIRST));
-                PF_TRY(pf_vel_step_fused(ctx, 0));
+                PF_TRY(pf_vel_step_fused(ctx, 0, !pf_util_active(ctx)));
                 PF_TRY(main_nonlinear(ctx, NL_NEXT));
                 return pf_vel_step_fused(ctx, 1);
             }));
@@ -350,7 +356,7 @@ extern "C" int pf_timestep(pf_ctx *ctx, int *ncorr) {
             if (ctx->tim.new_dt) PF_TRY(pf_vel_matrices_impl(ctx));
         }
         if (pf_util_active(ctx)) PF_TRY(pf_util_run(ctx, 1));
-        PF_TRY(pf_vel_predictor(ctx));
+        PF_TRY(predictor(ctx, !pf_util_active(ctx)));
         ctx->tim.it = 1;
         while (ctx->tim.it != 0) {
             PF_TRY(main_nonlinear(ctx, nc == 0 ? NL_NEXT : NL_AGAIN));
@@ -373,7 +379,7 @@ extern "C" int pf_steporbit(pf_ctx *ctx, int nsteps) {
     PF_TRY(require_matrices(ctx));
     for (int s = 0; s < nsteps; ++s) {
         PF_TRY(pf_first_nonlinear(ctx));
-        PF_TRY(pf_vel_predictor(ctx));
+        PF_TRY(predictor(ctx, true));  // no hook here: the fused transforms follow with a plug-in set too
         PF_TRY(pf_next_nonlinear(ctx));
         PF_TRY(vel_corrector_async(ctx));
         PF_TRY(pf_vel_imposesym(ctx));
