@@ -577,7 +577,10 @@ template <typename C> struct NLTiles {
     int MC, ZC;
     size_t zsm, tsm;
 };
-static constexpr size_t NL_TILE_MAX_SMEM = 100 * 1024;  // largest tile a tuning may choose
+// Largest tile a tuning may choose.  A z tile counts by its rows as FFTRows
+// holds them, whatever the passes take for it (RowsIO: up to 108,288 bytes),
+// so that the choices a program has cached stay the ones that are accepted.
+static constexpr size_t NL_TILE_MAX_SMEM = 100 * 1024;
 
 template <typename C> static size_t theta_smem(int Th, int ZC) { return (size_t)rows_elems<C>(Th, 3 * ZC) * sizeof(C); }
 
@@ -613,8 +616,10 @@ int pf_nl_tiles_check(const pf_ctx *ctx, const pf_tuning *tu) {
            "pf_ctx_set_tuning: nl_mc >= 0, nl_zc even in 0..32");
     if (!pf_nl_fused_supported(ctx)) return PF_OK;
     const bool mixed = ctx->cfg.precision == PF_PREC_MIXED;
-    const size_t zsm = mixed ? nl_tiles<float2>(ctx->g, *tu).zsm : nl_tiles<double2>(ctx->g, *tu).zsm;
-    const size_t tsm = mixed ? nl_tiles<float2>(ctx->g, *tu).tsm : nl_tiles<double2>(ctx->g, *tu).tsm;
+    const Geo &g = ctx->g;
+    const size_t zsm = mixed ? rows_elems<float2>(g.Z, nl_tiles<float2>(g, *tu).MC) * sizeof(float2)
+                             : rows_elems<double2>(g.Z, nl_tiles<double2>(g, *tu).MC) * sizeof(double2);
+    const size_t tsm = mixed ? nl_tiles<float2>(g, *tu).tsm : nl_tiles<double2>(g, *tu).tsm;
     if (zsm > NL_TILE_MAX_SMEM || tsm > NL_TILE_MAX_SMEM) {
         pf_set_error("pf_ctx_set_tuning: transform tiles need %zu / %zu bytes of shared memory (cap %zu)", zsm, tsm,
                      NL_TILE_MAX_SMEM);
