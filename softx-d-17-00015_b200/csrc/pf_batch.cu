@@ -536,10 +536,13 @@ static int batch_corrector(pf_batch *b, const std::vector<int> &act) {
 }
 
 // Corrector control after a batched step (timestep.f90:214-253, main.f90:35-41)
-// from the scalars the step left in b->hsc; returns the passes taken.
+// from the scalars the step left in b->hsc; returns the passes taken.  A step
+// that could not finish (pf_step_status) is its own pipe's failure: no corrector
+// control on what it left, and *status stays PF_ERR_CUDA whatever the others report.
 static long long batch_after_step(pf_batch *b, int orbit, int *status) {
     long long passes = 0;
     std::vector<int> act;
+    bool stuck = false;
     for (int i = 0; i < b->n; ++i) {
         pf_ctx *c = b->pipes[i];
         c->tim.it = 1;
@@ -561,11 +564,11 @@ static long long batch_after_step(pf_batch *b, int orbit, int *status) {
             pf_ctx *c = b->pipes[i];
             const double err2 = bits_to_double(b->hsc[i].dterr2_bits);
             if (pf_step_status(b->hsc[i]) != PF_OK) {
-                *status = PF_ERR_CUDA;
-                if (!first) {
-                    c->tim.it = 0;
-                    continue;
-                }
+                stuck = true;
+                c->last_status = PF_ERR_CUDA;
+                c->last_error = pf_last_error();
+                c->tim.it = 0;
+                continue;
             }
             c->tim.dterr = std::max(c->tim.dterr, std::sqrt(err2));
             const int s = pf_tim_check_cgce(c);
@@ -574,7 +577,7 @@ static long long batch_after_step(pf_batch *b, int orbit, int *status) {
                     c->last_status = s;
                     c->last_error = pf_last_error();
                 }
-                if (!orbit) *status = s;
+                if (!orbit && *status != PF_ERR_CUDA) *status = s;
             }
             // the state went non-finite: the max of the corrections' bit patterns
             // is a NaN or Inf pattern (the reference would carry on with NaN)
@@ -587,6 +590,10 @@ static long long batch_after_step(pf_batch *b, int orbit, int *status) {
             if (c->tim.it != 0) again.push_back(i);
         }
         act.swap(again);
+    }
+    if (stuck) {
+        *status = PF_ERR_CUDA;
+        for (int i = 0; i < b->n; ++i) pf_step_status(b->hsc[i]);  // its message, not a later pipe's
     }
     for (pf_ctx *c : b->pipes) {
         c->tim.t = c->tim.t + c->tim.dt;
@@ -615,7 +622,7 @@ extern "C" int pf_batch_step(pf_batch *b, int nsteps, int orbit, long long *corr
                     const int s = pf_timestep(c, &nc);
                     c->last_status = s;
                     c->last_error = s != PF_OK ? pf_last_error() : "";
-                    if (s != PF_OK) status = s;
+                    if (s != PF_OK && status != PF_ERR_CUDA) status = s;
                     passes += nc;
                 }
             }
@@ -670,7 +677,9 @@ extern "C" int pf_batch_step(pf_batch *b, int nsteps, int orbit, long long *corr
                 } else {
                     int nc = 0;
                     const int s = pf_timestep(c, &nc);
-                    if (s != PF_OK) status = s;
+                    c->last_status = s;
+                    c->last_error = s != PF_OK ? pf_last_error() : "";
+                    if (s != PF_OK && status != PF_ERR_CUDA) status = s;
                     passes += nc;
                 }
             }

@@ -1,0 +1,111 @@
+"""A fused step whose factor copies never arrived is its own pipe's failure.
+
+The kernel reports it in the pipe's device scalars.  Here the report is written
+there from the host, as the kernel would leave it, through a few lines built
+against the library's own header: no copy is held back and nothing waits.
+"""
+import ctypes as C
+import subprocess
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+from _util import SMALL, device_pipe
+
+pytestmark = pytest.mark.gpu
+
+ROOT = Path(__file__).resolve().parents[1]
+PLANT = r"""
+#include "pf_internal.cuh"
+extern "C" int plant(pf_ctx *c) {
+    const int v = PF_STEP_STUCK;
+    cudaStreamSynchronize(c->stream);
+    return cudaMemcpy(&c->dsc->info, &v, sizeof(v), cudaMemcpyHostToDevice) == cudaSuccess ? 0 : 1;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def plant(tmp_path_factory):
+    d = tmp_path_factory.mktemp("plant")
+    (d / "plant.cu").write_text(PLANT)
+    so = d / "plant.so"
+    subprocess.run(["/usr/local/cuda/bin/nvcc", "-std=c++17", "-shared", "-Xcompiler", "-fPIC",
+                    f"-I{ROOT / 'softx-d-17-00015_b200' / 'csrc'}", f"-I{ROOT / 'include'}", str(d / "plant.cu"),
+                    "-o", str(so)], check=True)
+    fn = C.CDLL(str(so)).plant
+    fn.argtypes = [C.c_void_p]
+    return lambda ctx: fn(ctx) == 0
+
+
+def _state(cfgd, seed):
+    import pipeflow as P
+    p = device_pipe(cfgd)
+    P.seeded_state(p, seed, 1e-3)
+    st = p.get_state()
+    p.close()
+    return st
+
+
+def _same(a, b):
+    return all(np.array_equal(x[0], y[0]) and np.array_equal(x[1], y[1]) for x, y in zip(a, b))
+
+
+def _status(fn):
+    import pipeflow as P
+    with pytest.raises(P.PipeflowError) as e:
+        fn()
+    return e.value.status
+
+
+@pytest.mark.parametrize("last_aborts", [False, True])
+@pytest.mark.parametrize("mirror", [False, True], ids=["staged", "branches"])
+def test_a_batch_step_reports_it_whatever_the_other_pipes_report(plant, last_aborts, mirror):
+    import pipeflow as P
+    cfgs = [P.PipeConfig(**dict(SMALL[0], mirrorsym=mirror)) for _ in range(3)]
+    batch = P.Batch(cfgs)
+    batch.matrices()
+    for i, p in enumerate(batch.pipes):
+        P.seeded_state(p, 50 + i, 1e-3)
+    batch.step(1)
+    batch.step(1)
+    if last_aborts:  # the corrector control's "dt --> 0" of the pipe after it
+        t = batch.pipes[2].tim
+        t.dt, t.step = 1e-10, 31
+        batch.pipes[2].set_tim(t)
+    assert plant(batch.pipes[1].ctx)
+    dt, corr_dt = batch.pipes[1].tim.dt, batch.pipes[1].tim.corr_dt
+    assert _status(lambda: batch.step(1)) == P._lib.PF_ERR_CUDA
+    # the corrector control did not run on what the step left
+    assert batch.pipes[1].tim.it == 0 and batch.pipes[1].tim.corr_dt == corr_dt and batch.pipes[1].tim.dt == dt
+    batch.close()
+
+
+def test_a_served_request_gets_it_and_the_others_their_results(plant):
+    import pipeflow as P
+    cfgd = SMALL[0]
+    states = [_state(cfgd, 70 + i) for i in range(3)]
+    srv = P.Server(hbm_budget=20 * 10**9, orbit=False)
+    ids = [srv.submit(P.PipeConfig(**cfgd), 3, st) for st in states]
+    srv.step()
+    bh, ph = C.c_void_p(), C.c_void_p()
+    assert srv.lib.pf_serve_batch(srv.h, C.byref(bh)) == 0 and srv.lib.pf_batch_pipe(bh, 1, C.byref(ph)) == 0
+    assert plant(ph)
+    assert _status(srv.step) == P._lib.PF_ERR_CUDA
+    srv.step()
+    assert set(srv.finished()) == set(ids)
+    assert _status(lambda: srv.result(ids[1])) == P._lib.PF_ERR_CUDA
+    for i in (0, 2):
+        a = device_pipe(cfgd)
+        a.vel_matrices()
+        a.set_state(*states[i])
+        for _ in range(3):
+            a.timestep()
+        assert _same(srv.result(ids[i]), a.get_state())
+        a.close()
+    # its memory serves the next request
+    again = srv.submit(P.PipeConfig(**cfgd), 1, states[1])
+    srv.step()
+    srv.result(again)
+    srv.close()
