@@ -25,6 +25,9 @@ extern "C" int pf_vel_imposesym(pf_ctx *ctx) {
 
 extern "C" int pf_vel_matrices(pf_ctx *ctx) {
     PF_ARG(ctx, "null ctx");
+    // a fresh start for a pipe whose last step could not finish (not in
+    // pf_vel_matrices_impl, which a step calls between its own launches)
+    PF_CUDA(cudaMemsetAsync(&ctx->dsc->info, 0, sizeof(int), ctx->stream));
     return pf_vel_matrices_impl(ctx);
 }
 

@@ -109,3 +109,23 @@ def test_a_served_request_gets_it_and_the_others_their_results(plant):
     srv.step()
     srv.result(again)
     srv.close()
+
+
+def test_new_matrices_start_a_pipe_afresh(plant):
+    import pipeflow as P
+    a, b = device_pipe(SMALL[2]), device_pipe(SMALL[2])
+    st = _state(SMALL[2], 60)
+    for p in (a, b):
+        p.vel_matrices()
+        p.set_state(*st)
+    assert plant(a.ctx)
+    assert _status(a.timestep) == P._lib.PF_ERR_CUDA
+    assert _status(a.timestep) == P._lib.PF_ERR_CUDA  # the state is not to be trusted until then
+    a.vel_matrices()
+    a.set_state(*st)
+    a.set_tim(b.tim)
+    for p in (a, b):
+        p.timestep()
+    assert _same(a.get_state(), b.get_state())
+    a.close()
+    b.close()
