@@ -371,6 +371,20 @@ inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, int threads, 
     return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
+// Waits for the phase of the given parity of an mbarrier (a shared address);
+// false if it did not complete while `tries` lasted, and at once when they are
+// used up.  A try suspends for up to 4 us, so MBAR_TRIES are a second; they are
+// counted down over the waits that share them.
+static constexpr int MBAR_TRIES = 1 << 18;
+__device__ __forceinline__ bool mbar_wait(unsigned mbar, unsigned parity, int &tries) {
+    unsigned done;
+    do
+        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+                     : "=r"(done) : "r"(mbar), "r"(parity) : "memory");
+    while (!done && --tries > 0);
+    return done != 0;
+}
+
 // x / d for 0 <= x < 2^22 and d > 0, given inv = 1.0f / d: a float
 // reciprocal estimate corrected by one step (cheaper than a run-time integer
 // division inside index loops)

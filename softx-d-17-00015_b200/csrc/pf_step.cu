@@ -87,15 +87,6 @@ __device__ __forceinline__ void bulk_copy(unsigned dst, const void *src, unsigne
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst),
                  "l"(src), "r"(bytes), "r"(mbar) : "memory");
 }
-// Waits for the phase of the given parity, at most a second or so; false if
-// it did not complete.
-__device__ __forceinline__ bool mbar_wait(unsigned mbar, unsigned parity) {
-    unsigned done = 0;
-    for (int t = 0; t < (1 << 20) && !done; ++t)
-        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-                     : "=r"(done) : "r"(mbar), "r"(parity) : "memory");
-    return done != 0;
-}
 __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p)); }
 __device__ __forceinline__ void mbar_arrive(unsigned mbar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(mbar) : "memory");
@@ -112,18 +103,26 @@ static constexpr int GROUP = 1920;  // bytes for W = 8
 static constexpr int GF = KL + 1;   // forward columns of a group
 __host__ __device__ constexpr int group_back(bool wide) { return wide ? 3 : 5; }
 __host__ __device__ constexpr int group_bytes(int W) { return GROUP / 8 * W; }
+// a stream's mbarriers: a chunk has landed in its place, its place is free again
+struct StreamBars {
+    unsigned long long full[RING], empty[RING];
+    long long asked;  // chunks asked for so far
+};
+__device__ __forceinline__ unsigned bar_full(unsigned bars, int place) { return bars + place * 8; }
+__device__ __forceinline__ unsigned bar_empty(unsigned bars, int place) { return bars + (RING + place) * 8; }
 struct FactorStream {
     const double *ft;   // the tile
     int N, W, flags;
     int g, places;      // groups a chunk, chunks of the ring
-    unsigned ring, full, empty;  // shared addresses: the chunks, RING barriers each
+    unsigned ring, bars;  // shared addresses: the chunks, the StreamBars
 };
 // Ask for chunks from .. to-1 of the stream, each once its place is free; by
-// one lane.  False if a place never was.
+// one lane.  False if a place was not free within the second of MBAR_TRIES: no
+// more are asked for then.
 __device__ __noinline__ bool stream_fill(const FactorStream s, int from, int to) {
     if (s.g < 1) return false;  // a ring too small for a chunk
     const double *src = s.ft;
-    int q = 0, place = 0, turn = 0;
+    int q = 0, place = 0, turn = 0, tries = MBAR_TRIES;
 #pragma unroll 1
     for (int back = 0; back < 2; ++back) {
         const int cols = s.g * (back ? group_back(s.flags & 2) : GF);
@@ -133,8 +132,12 @@ __device__ __noinline__ bool stream_fill(const FactorStream s, int from, int to)
             const int words = min(cols, s.N - j0) * row;
             if (q >= to) return true;
             if (q >= from) {
-                if (turn > 0 && !mbar_wait(s.empty + place * 8, (turn - 1) & 1)) return false;
-                bulk_copy(s.ring + place * s.g * group_bytes(s.W), src, words * 8, s.full + place * 8);
+                // (a solve that has given up hands places back with their copies still on the way)
+                if (turn > 0 && !(mbar_wait(bar_empty(s.bars, place), (turn - 1) & 1, tries) &&
+                                  mbar_wait(bar_full(s.bars, place), (turn - 1) & 1, tries)))
+                    return false;
+                bulk_copy(s.ring + place * s.g * group_bytes(s.W), src, words * 8, bar_full(s.bars, place));
+                asm volatile("st.shared.u64 [%0], %1;\n" ::"r"(s.bars + 2 * RING * 8), "l"(q + 1ll) : "memory");
             }
             src += words;
             if (++place == s.places) {
@@ -149,7 +152,8 @@ __device__ __noinline__ bool stream_fill(const FactorStream s, int from, int to)
 // A group's factors are read into registers before any of its results is
 // stored, which would order the reads behind the chain.  f: the field's byte
 // offset into the block's dynamic shared memory.  Returns false if a copy
-// never came.
+// did not come within the second of MBAR_TRIES; it then waits for no other, and
+// what it leaves in the field is of no use.
 template <bool PIV, bool WIDE, int W>
 __device__ __noinline__ bool tile_solve(const FactorStream s, int f) {
     extern __shared__ __align__(128) unsigned char step_sm[];
@@ -161,12 +165,12 @@ __device__ __noinline__ bool tile_solve(const FactorStream s, int f) {
     const unsigned fl = base + f + lane * 8;
     int place = 0, left = 0;
     unsigned par = 0;
-    bool ok = true;
+    int tries = MBAR_TRIES;
     if (s.g < 1) return false;
     const double *col = rd;
     auto next = [&](int group) {  // the next group's factors
         if (left == 0) {
-            ok &= mbar_wait(s.full + place * 8, par);
+            mbar_wait(bar_full(s.bars, place), par, tries);
             col = rd + place * s.g * (group_bytes(W) / 8);
             left = s.g;
         } else {
@@ -181,7 +185,7 @@ __device__ __noinline__ bool tile_solve(const FactorStream s, int f) {
             left = 0;
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(s.empty + place * 8);
+            if (lane == 0) mbar_arrive(bar_empty(s.bars, place));
             if (++place == s.places) {
                 place = 0;
                 par ^= 1;
@@ -245,7 +249,7 @@ __device__ __noinline__ bool tile_solve(const FactorStream s, int f) {
         }
     }
     __syncwarp();
-    return ok;
+    return tries > 0;
 }
 
 // ------------------------------------------------------------------ tiles
@@ -314,7 +318,7 @@ static_assert(NBAND == 9, "rows of ten doubles");
 // `ld` bytes each if there is room for them (`apart`); else these share b3
 // and the pressure ring, once both are done with.
 struct StepHead {
-    unsigned long long bars[4][2][RING];  // LNp, LDp, LDm, LDz: full, empty
+    StreamBars bars[4];    // LNp, LDp, LDm, LDz
     double ainv[16][17];   // 4x4 inverse per slot
     double coef[8][16];    // aR(1..4), aI(1..4) per slot
     double flux;           // 2 int uz r dr of the mean mode
@@ -359,8 +363,11 @@ __device__ __forceinline__ void step_tile(const StepArgs &a, int tile, const Ste
     const bool live = tile_mode(g, tile, slot, nh, k, m);
     if (!live) nh = 0;
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 8 * RING; ++i)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(sbase + i * 8) : "memory");
+        for (int s = 0; s < 4; ++s) {
+            hd.bars[s].asked = 0;
+            for (int i = 0; i < 2 * RING; ++i)
+                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(sbase + s * (int)sizeof(StreamBars) + i * 8) : "memory");
+        }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     }
@@ -392,8 +399,7 @@ __device__ __forceinline__ void step_tile(const StepArgs &a, int tile, const Ste
         if (sys > 0) s.ring += (lay.apart ? lay.ppe : -N * 256) + (sys - 1) * lay.ld;
         s.places = bytes >= RING * group_bytes(W) ? RING : 2;
         s.g = bytes / (s.places * group_bytes(W));
-        s.full = (unsigned)__cvta_generic_to_shared(&hd.bars[sys][0][0]);
-        s.empty = (unsigned)__cvta_generic_to_shared(&hd.bars[sys][1][0]);
+        s.bars = sbase + sys * (int)sizeof(StreamBars);
         return s;
     };
     bool ok = true;
@@ -515,7 +521,7 @@ __device__ __forceinline__ void step_tile(const StepArgs &a, int tile, const Ste
     } else if (role == 3 && lane0) {
         ok &= stream_fill(stream(0), stream(0).places, 1 << 30);
     }
-    __syncthreads();
+    ok = !__syncthreads_or(!ok);
     // rhs - rt2pm(grad p), grad p = (dr p, i m/r p, i alpha k p); zero boundary rows
 #pragma unroll 1
     for (int n = ty; n < N; n += NR) {
@@ -537,7 +543,9 @@ __device__ __forceinline__ void step_tile(const StepArgs &a, int tile, const Ste
     // so far, may now take asynchronous copies
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     __syncthreads();
-    if (role < 3) {
+    if (!ok) {
+        // no more waits
+    } else if (role < 3) {
         const FactorStream s = stream(1 + role);
         const int f = fields + role * N * 256;
         if (s.flags == 0) ok &= tile_solve<false, false, W>(s, f);
@@ -547,8 +555,23 @@ __device__ __forceinline__ void step_tile(const StepArgs &a, int tile, const Ste
         const FactorStream s = stream(role - 2);
         ok &= stream_fill(s, lay.apart ? s.places : 0, 1 << 30);
     }
-    if (!ok) atomicCAS(&a.sc->info, 0, PF_STEP_STUCK);
-    __syncthreads();
+    if (__syncthreads_or(!ok)) {
+        // reported to the host; the copies still on their way must not land in
+        // the shared memory of a block after this one
+        if (threadIdx.x == 0) {
+            atomicCAS(&a.sc->info, 0, PF_STEP_STUCK);
+            int tries = MBAR_TRIES;
+#pragma unroll 1
+            for (int sys = 0; sys < 4; ++sys) {
+                const FactorStream s = stream(sys);
+                const int n = (int)*(volatile long long *)&hd.bars[sys].asked;
+#pragma unroll 1
+                for (int q = max(0, n - s.places); q < n; ++q)
+                    mbar_wait(bar_full(s.bars, q % s.places), q / s.places & 1, tries);
+            }
+        }
+        __syncthreads();
+    }
     if (threadIdx.x < 16 && live) {
         // vel_evalBC + a = -A^-1 B (velocity.f90:239-243, 262-298)
         const int e = (N - 1) * 16;

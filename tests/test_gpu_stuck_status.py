@@ -2,7 +2,8 @@
 
 The kernel reports it in the pipe's device scalars.  Here the report is written
 there from the host, as the kernel would leave it, through a few lines built
-against the library's own header: no copy is held back and nothing waits.
+against the library's own header: no copy is held back.  The wait itself is tried on
+a barrier that nothing arrives at.
 """
 import ctypes as C
 import subprocess
@@ -23,20 +24,46 @@ extern "C" int plant(pf_ctx *c) {
     cudaStreamSynchronize(c->stream);
     return cudaMemcpy(&c->dsc->info, &v, sizeof(v), cudaMemcpyHostToDevice) == cudaSuccess ? 0 : 1;
 }
+// a barrier that nothing arrives at
+static __global__ void k_wait(double *out) {
+    __shared__ __align__(8) unsigned long long bar;
+    const unsigned b = (unsigned)__cvta_generic_to_shared(&bar);
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b) : "memory");
+    int tries = MBAR_TRIES;
+    for (int i = 0; i < 2; ++i) {
+        unsigned long long t0, t1;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0)::"memory");
+        out[2 * i] = mbar_wait(b, 0, tries);
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1)::"memory");
+        out[2 * i + 1] = (double)(t1 - t0) * 1e-9;
+    }
+}
+extern "C" int wait_for_nothing(double *out) {
+    double *d = nullptr;
+    if (cudaMalloc((void **)&d, 32) != cudaSuccess) return 1;
+    k_wait<<<1, 1>>>(d);
+    const cudaError_t e = cudaMemcpy(out, d, 32, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return e == cudaSuccess ? 0 : 1;
+}
 """
 
 
 @pytest.fixture(scope="module")
-def plant(tmp_path_factory):
+def helper(tmp_path_factory):
     d = tmp_path_factory.mktemp("plant")
     (d / "plant.cu").write_text(PLANT)
     so = d / "plant.so"
-    subprocess.run(["/usr/local/cuda/bin/nvcc", "-std=c++17", "-shared", "-Xcompiler", "-fPIC",
-                    f"-I{ROOT / 'softx-d-17-00015_b200' / 'csrc'}", f"-I{ROOT / 'include'}", str(d / "plant.cu"),
+    subprocess.run(["/usr/local/cuda/bin/nvcc", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a",
+                    "-shared", "-Xcompiler", "-fPIC", f"-I{ROOT / 'softx-d-17-00015_b200' / 'csrc'}", f"-I{ROOT / 'include'}", str(d / "plant.cu"),
                     "-o", str(so)], check=True)
-    fn = C.CDLL(str(so)).plant
-    fn.argtypes = [C.c_void_p]
-    return lambda ctx: fn(ctx) == 0
+    return C.CDLL(str(so))
+
+
+@pytest.fixture
+def plant(helper):
+    helper.plant.argtypes = [C.c_void_p]
+    return lambda ctx: helper.plant(ctx) == 0
 
 
 def _state(cfgd, seed):
@@ -129,3 +156,10 @@ def test_new_matrices_start_a_pipe_afresh(plant):
     assert _same(a.get_state(), b.get_state())
     a.close()
     b.close()
+
+
+def test_a_wait_gives_up_after_a_second_and_the_ones_after_it_at_once(helper):
+    out = (C.c_double * 4)()
+    assert helper.wait_for_nothing(out) == 0
+    assert out[0] == 0.0 and 0.5 <= out[1] < 2.0
+    assert out[2] == 0.0 and out[3] < 1e-3
