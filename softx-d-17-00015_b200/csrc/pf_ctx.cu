@@ -146,6 +146,7 @@ static int ctx_init(pf_ctx *ctx, const pf_config *cfg, int device) {
     }
     if (device >= 0) PF_CUDA(cudaSetDevice(device));
     PF_CUDA(cudaGetDevice(&ctx->device));
+    PF_CUDA(cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device));
     PF_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
     ctx->own_stream = true;
     ctx->cfg = *cfg;

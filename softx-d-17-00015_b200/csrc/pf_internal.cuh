@@ -207,7 +207,7 @@ struct pf_lumesh {
 struct pf_ctx {
     pf_config cfg;
     Geo g;
-    int device;
+    int device, sms;
     cudaStream_t stream;
     bool own_stream;
     HostMesh hm;
@@ -351,9 +351,10 @@ template <typename T> __device__ __forceinline__ T pick3(T const (&p)[3], int i)
 // kernel reads or writes only after chain_wait, which returns when all of it
 // has finished and which every block calls.  Two steps of N=48 with 2985 modes
 // 566 -> 541 us, four of N=40 446 -> 414, of N=16 279 -> 267.  The transform
-// passes launched so gain nothing or lose (all of them chained as well: N=48
-// 590 us): several of their blocks share an SM, and blocks that start early
-// crowd the SMs that come free first.
+// passes are launched so where they are small (pf_nl.cu); larger ones gain
+// nothing or lose (all of them chained as well: N=48 590 us): several of their
+// blocks share an SM, and blocks that start early crowd the SMs that come free
+// first.
 __device__ __forceinline__ void chain_open() { asm volatile("griddepcontrol.launch_dependents;\n" ::); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 template <typename... P, typename... A>

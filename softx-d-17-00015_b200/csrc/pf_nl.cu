@@ -472,15 +472,20 @@ template <int L> struct NLOcc<float2, L> {
 
 template <int ZL, typename C>
 __global__ void __launch_bounds__(NL_THREADS, (NLOcc<C, ZL>::zinv)) k_nl_zinv(NLArgs a) {
+    chain_open();
+    chain_wait();
     nl_zinv_body<ZL, C>(a, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 template <int TL, typename C>
 __global__ void __launch_bounds__(NL_THREADS, (NLOcc<C, TL>::theta)) k_nl_theta(NLArgs a) {
+    chain_open();
+    chain_wait();
     nl_theta_body<TL, C>(a, blockIdx.x, blockIdx.y);
 }
 template <int ZL, typename C>
 __global__ void __launch_bounds__(NL_THREADS, (NLOcc<C, ZL>::zfwd)) k_nl_zfwd(NLArgs a) {
     chain_open();
+    chain_wait();
     nl_zfwd_body<ZL, C>(a, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 template <int ZL, int TL>
@@ -677,6 +682,17 @@ template <typename K> static int raise_smem(K kernel, size_t bytes, size_t &cur)
     return PF_OK;
 }
 
+// A pass of up to half as many blocks as SMs is set up while the launch before
+// it drains, which makes up for the launch that forms curl(u): N = 24 with 83
+// modes 20.6 -> 16.7 us the four, 18.4 when the z pass formed it.  With as many
+// blocks as SMs a step got slower (mixed, N = 32, 81 modes: 88 -> 100 us).
+static cudaError_t pass_launch(const pf_ctx *ctx, void (*k)(NLArgs), dim3 grid, size_t smem, const NLArgs &a) {
+    if ((long long)grid.x * grid.y * grid.z <= ctx->sms / 2)
+        return launch_chained(k, grid, NL_THREADS, smem, ctx->stream, a);
+    k<<<grid, NL_THREADS, smem, ctx->stream>>>(a);
+    return cudaSuccess;
+}
+
 template <typename C>
 static int launch_nl(pf_ctx *ctx, const NLArgs &a) {
     const Geo &g = ctx->g;
@@ -703,7 +719,7 @@ static int launch_nl(pf_ctx *ctx, const NLArgs &a) {
         static size_t set_ = 0;                                       \
         PF_TRY(raise_smem(k_nl_zinv<L, C>, t.zsm, set_));             \
         ProfScope ps_(ctx, PF_K_ZINV);                                \
-        k_nl_zinv<L, C><<<gz, NL_THREADS, t.zsm, ctx->stream>>>(a);   \
+        PF_CUDA(pass_launch(ctx, k_nl_zinv<L, C>, gz, t.zsm, a));     \
     } break;
         PF_NL_LENGTHS(PF_CASE)
 #undef PF_CASE
@@ -718,7 +734,7 @@ static int launch_nl(pf_ctx *ctx, const NLArgs &a) {
         static size_t set_ = 0;                                       \
         PF_TRY(raise_smem(k_nl_theta<L, C>, t.tsm, set_));            \
         ProfScope ps_(ctx, PF_K_THFWD);                               \
-        k_nl_theta<L, C><<<gt, NL_THREADS, t.tsm, ctx->stream>>>(a);  \
+        PF_CUDA(pass_launch(ctx, k_nl_theta<L, C>, gt, t.tsm, a));    \
     } break;
         PF_NL_LENGTHS(PF_CASE)
 #undef PF_CASE
@@ -733,7 +749,7 @@ static int launch_nl(pf_ctx *ctx, const NLArgs &a) {
         static size_t set_ = 0;                                       \
         PF_TRY(raise_smem(k_nl_zfwd<L, C>, t.zsm, set_));             \
         ProfScope ps_(ctx, PF_K_ZFWD);                                \
-        k_nl_zfwd<L, C><<<gf, NL_THREADS, t.zsm, ctx->stream>>>(a);   \
+        PF_CUDA(pass_launch(ctx, k_nl_zfwd<L, C>, gf, t.zsm, a));     \
     } break;
         PF_NL_LENGTHS(PF_CASE)
 #undef PF_CASE
@@ -744,11 +760,12 @@ static int launch_nl(pf_ctx *ctx, const NLArgs &a) {
     return PF_OK;
 }
 
-template <bool MIXED> __global__ void k_nl_prep(NLArgs a, int sym);
+template <bool MIXED> __global__ void k_nl_prep(NLArgs a, int rows, int sym);
 __global__ void k_nl_mean64_fin(NLArgs a, int stepped);
 static int prep_attrs();
-static size_t prep_smem(int N);
+static size_t prep_smem(int rows);
 static constexpr int PREP_MAX_N = 128;  // its two staged components fill 1 KB of shared memory a radial point
+static int prep_rows(int N, int chunks, int sms);
 
 // vel_transform + vel_nonlinear: curl(u) (PF_NL_STEPPED: left by the fused
 // predictor that made u), the three transform launches, and in mixed
@@ -765,9 +782,11 @@ int pf_launch_nl_fused(pf_ctx *ctx, int mode) {
         {
             ProfScope ps_(ctx, PF_K_STENCIL);
             PF_TRY(prep_attrs());
-            const int blocks = (ctx->g.H + 31) / 32, sym = mode == PF_NL_SYM;
-            if (mixed) k_nl_prep<true><<<blocks, PREP_THREADS, prep_smem(N), ctx->stream>>>(a, sym);
-            else k_nl_prep<false><<<blocks, PREP_THREADS, prep_smem(N), ctx->stream>>>(a, sym);
+            const int chunks = (ctx->g.H + 31) / 32, rows = prep_rows(N, chunks, ctx->sms), sym = mode == PF_NL_SYM;
+            const dim3 grid(chunks, (N + rows - 1) / rows);
+            const size_t sm = prep_smem(std::min(N, rows + 2 * KL));
+            if (mixed) k_nl_prep<true><<<grid, PREP_THREADS, sm, ctx->stream>>>(a, rows, sym);
+            else k_nl_prep<false><<<grid, PREP_THREADS, sm, ctx->stream>>>(a, rows, sym);
         }
         PF_LAUNCHED(ctx);
     }
@@ -782,10 +801,10 @@ int pf_launch_nl_fused(pf_ctx *ctx, int mode) {
 }
 
 // ----------------------------------------- curl(u) and the FP64 mean mode
-// One block per 32-mode chunk, u_t and u_z of those modes at every radial
-// point staged in shared memory (each value read from HBM once), one warp per
-// radial point at a time (lanes = modes): curl(u) (variables.f90:408-436) from
-// the staged rows, stored for the z pass.
+// One block per 32-mode chunk and run of radial points, u_t and u_z of those
+// modes there and KL rows beyond staged in shared memory, one warp per radial
+// point at a time (lanes = modes): curl(u) (variables.f90:408-436) from the
+// staged rows, stored for the z pass.
 //
 // With FP32 transforms the k=m=0 coefficient of u x curl(u) is replaced by
 // its exact FP64 value.  On the 3/2-dealiased grid no product of retained
@@ -795,48 +814,56 @@ int pf_launch_nl_fused(pf_ctx *ctx, int mode) {
 // (the c2r transform ignores Im f00): the chunk's sums go out as partials
 // here, and one warp per radial point adds the chunks' partials in a fixed
 // order afterwards.
-template <bool MIXED> __device__ __forceinline__ void nl_prep_body(const NLArgs &a, int chunk, int sym) {
-    extern __shared__ double2 msm[];  // [2][N][32]: u_t, u_z of this chunk's modes
+template <bool MIXED>
+__device__ __forceinline__ void nl_prep_body(const NLArgs &a, int chunk, int n0, int n1, int sym) {
+    extern __shared__ double2 msm[];  // [2][j1 - j0][32]: u_t, u_z of this chunk's modes at the rows read
     const Geo &g = a.g;
     const int N = g.N, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int j0 = max(0, n0 - KL), j1 = min(N, n1 + KL);
     const int nh = chunk * 32 + lane;
     const bool live = nh < g.H, mean = sym && nh == 0;
     const size_t Hp = g.Hp;
-    double2 *st = msm, *sz = msm + N * 32;
+    double2 *st = msm, *sz = msm + (j1 - j0) * 32;
 #pragma unroll 4
-    for (int n = warp; n < N; n += nw) {
+    for (int n = j0 + warp; n < j1; n += nw) {
         const size_t at = (size_t)n * Hp + nh;
         double2 t = live ? a.u[1][at] : make_double2(0.0, 0.0), z = live ? a.u[2][at] : make_double2(0.0, 0.0);
         if (mean) {  // var_imposesym of the mean mode (variables.f90:611-616)
             t.y = z.y = 0.0;
-            const_cast<double2 *>(a.u[0])[at] = make_double2(0.0, 0.0);
-            const_cast<double2 *>(a.u[1])[at] = t;
-            const_cast<double2 *>(a.u[2])[at] = z;
+            if (n >= n0 && n < n1) {  // what the blocks beside this one read of these rows stays as it is
+                const_cast<double2 *>(a.u[0])[at] = make_double2(0.0, 0.0);
+                const_cast<double2 *>(a.u[1])[at].y = 0.0;
+                const_cast<double2 *>(a.u[2])[at].y = 0.0;
+            }
         }
-        st[n * 32 + lane] = t;
-        sz[n * 32 + lane] = z;
+        st[(n - j0) * 32 + lane] = t;
+        sz[(n - j0) * 32 + lane] = z;
     }
     __syncthreads();
     int k = 0, m = 0;
     if (live) mode_km(nh, g.K, k, m);
     const double k1a1 = g.alpha * k;
     const double *__restrict__ drb = a.dm.dr;
-    for (int n = warp; n < N; n += nw) {
+    for (int n = n0 + warp; n < n1; n += nw) {
         double s[3] = {0.0, 0.0, 0.0};
         if (live) {
             const size_t at = (size_t)n * Hp + nh;
             const double2 ur = mean ? make_double2(0.0, 0.0) : a.u[0][at];
-            const double2 ut = st[n * 32 + lane], uz = sz[n * 32 + lane];
+            const double2 ut = st[(n - j0) * 32 + lane], uz = sz[(n - j0) * 32 + lane];
             const double rm1 = a.dm.rp[2 * N + n];
-            const int lo = max(0, n - KL), hi = min(N - 1, n + KL);
+            double w[NBAND];  // read together, then the sums
+#pragma unroll
+            for (int i = 0; i < NBAND; ++i) w[i] = drb[(NBAND - 1 - i) * N + min(max(n - KL + i, 0), N - 1)];
             double2 dz = make_double2(0.0, 0.0), dt = dz;
-            for (int j = lo; j <= hi; ++j) {  // d/dr of u_z and u_t (var_coll_meshmult)
-                const double w = drb[(KL + n - j) * N + j];
-                const double2 z = sz[j * 32 + lane], t = st[j * 32 + lane];
-                dz.x = fma(w, z.x, dz.x);
-                dz.y = fma(w, z.y, dz.y);
-                dt.x = fma(w, t.x, dt.x);
-                dt.y = fma(w, t.y, dt.y);
+#pragma unroll
+            for (int i = 0; i < NBAND; ++i) {  // d/dr of u_z and u_t (var_coll_meshmult)
+                const int j = n - KL + i;
+                if (j < 0 || j >= N) continue;
+                const double2 z = sz[(j - j0) * 32 + lane], t = st[(j - j0) * 32 + lane];
+                dz.x = fma(w[i], z.x, dz.x);
+                dz.y = fma(w[i], z.y, dz.y);
+                dt.x = fma(w[i], t.x, dt.x);
+                dt.y = fma(w[i], t.y, dt.y);
             }
             const Curl c = mode_curl(ur, ut, uz, dt, dz, rm1, rm1 * g.Mp * m, k1a1);
             if (MIXED) {
@@ -893,9 +920,18 @@ __device__ __forceinline__ void nl_mean64_fin_body(const NLArgs &a, int n, int s
     a.N[2][at] = make_double2(zr, (-a.dm.velUp[n]) * ur.y);
 }
 
-static size_t prep_smem(int N) { return (size_t)2 * N * 32 * sizeof(double2); }
-template <bool MIXED> __global__ void __launch_bounds__(PREP_THREADS) k_nl_prep(NLArgs a, int sym) {
-    nl_prep_body<MIXED>(a, blockIdx.x, sym);
+static size_t prep_smem(int rows) { return (size_t)2 * rows * 32 * sizeof(double2); }
+// Radial points a block of a lone pipe's launch takes: a multiple of its eight
+// warps, as few as still give two blocks an SM, since few chunks leave the GPU
+// empty (N = 128, 4 chunks, with the transforms: 44 us with all points in a
+// block, 28 with eight)
+static int prep_rows(int N, int chunks, int sms) {
+    const int runs = std::min((N + 7) / 8, std::max(1, 2 * sms / chunks));
+    return runs == 1 ? N : ((N + runs - 1) / runs + 7) / 8 * 8;
+}
+template <bool MIXED> __global__ void __launch_bounds__(PREP_THREADS) k_nl_prep(NLArgs a, int rows, int sym) {
+    chain_open();
+    nl_prep_body<MIXED>(a, blockIdx.x, blockIdx.y * rows, min(a.g.N, (blockIdx.y + 1) * rows), sym);
 }
 // one warp per radial point
 __global__ void __launch_bounds__(128) k_nl_mean64_fin(NLArgs a, int stepped) {
@@ -956,8 +992,8 @@ __global__ void __launch_bounds__(PREP_THREADS) k_nl_prep_batch(const NLArgs *__
     const int2 pb = blk[blockIdx.x];
     if (act && !act[pb.x]) return;
     const NLArgs a = args[pb.x];
-    if ((int)blockIdx.x < nfp64) nl_prep_body<false>(a, pb.y, sym);
-    else nl_prep_body<true>(a, pb.y, sym);
+    if ((int)blockIdx.x < nfp64) nl_prep_body<false>(a, pb.y, 0, a.g.N, sym);
+    else nl_prep_body<true>(a, pb.y, 0, a.g.N, sym);
 }
 __global__ void __launch_bounds__(128) k_nl_mean64_fin_batch(const NLArgs *__restrict__ args,
                                                             const int2 *__restrict__ blk, int stepped,

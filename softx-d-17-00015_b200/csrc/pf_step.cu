@@ -824,8 +824,6 @@ int pf_vel_step_fused(pf_ctx *ctx, int corrector, bool leave_curl) {
     const StepArgs a = make_step_args(ctx, corrector, leave_curl);
     ctx->curl_left = !corrector && a.curl[0];
     const int blocks = pf_step_tiles(g);
-    int sms = 0;
-    PF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
     {
         ProfScope ps_(ctx, PF_K_STEP);
 #define PF_CASE(NMAX, NT, MINB)                                             \
@@ -835,7 +833,7 @@ int pf_vel_step_fused(pf_ctx *ctx, int corrector, bool leave_curl) {
         PF_TRY(pf_raise_smem((const void *)k_step<NT, MINB>, sm));          \
         PF_CUDA(launch_chained(k_step<NT, MINB>, dim3(blocks), NT, sm, ctx->stream, a, lay)); \
     }
-        if (blocks <= sms) {  // a block to an SM: all its threads and shared memory for latency
+        if (blocks <= ctx->sms) {  // a block to an SM: all its threads and shared memory for latency
             const StepSmem lay = step_rings(g.N, 1, blocks);
             const size_t sm = step_smem(g.N, lay);
             PF_TRY(pf_raise_smem((const void *)k_step<256, 1>, sm));
