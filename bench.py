@@ -194,8 +194,10 @@ def read_traffic(kernel: str, workload: str):
 # coll field size S: the coll fields it must read and write once (factors,
 # twiddles and transform scratch are not algorithmic).  The fused step reads
 # the old velocity and N and writes the velocity and N_ (12S, predictor), and
-# also reads N_ and the last velocity in the corrector (18S): 15S on average.
-PER_LAUNCH_S = {"lusolve": 6, "ppe": 2, "stencil": 2, "ew": 2, "infl": 4, "zinv": 3, "thinv": 3, "thfwd": 3,
+# also reads N_ and the last velocity in the corrector (18S): 15S on average;
+# the curl(u) that the predictor leaves for the transforms is scratch (3S, in
+# mixed precision 1.5S).
+PER_LAUNCH_S = {"lusolve": 6, "stencil": 2, "ew": 2, "infl": 4, "zinv": 3, "thinv": 3, "thfwd": 3,
                 "zfwd": 3, "step": 15, "factor": 0}
 
 
@@ -492,8 +494,10 @@ def run_batched(args, torch, P, dist, world, rank, local):
     extra = {"corrector_iterations_per_step": nc, "algorithmic_bytes_per_batch_step": step_bytes,
              "stage_batched": staged, "worklist_stages": worklist, "autotune": tuned,
              "transform_roofline": {
-                 "scope": "one evaluation of the nonlinear terms of every pipe: FP64 mean-mode pass (and curl), "
-                          "z inverse, theta pass with u x curl(u), z forward (all transform launches)",
+                 "scope": "the transform launches of one evaluation of the nonlinear terms of every pipe: z inverse, "
+                          "theta pass with u x curl(u), z forward, reduction of the FP64 mean mode; curl(u) and the "
+                          "mean mode's sums come with the predictor (step) or, before a step and before further "
+                          "corrector passes, from a launch timed as stencil",
                  "avg_evaluation_us": chain_ms * 1e3, "share_of_step_kernels": chain_share,
                  "algorithmic_bytes": chain_bytes, "achieved_gbs": chain_bytes / (chain_ms / 1e3) / 1e9,
                  "frac_of_measured_hbm": chain_bytes / (chain_ms / 1e3) / 1e9 / peaks()[0],

@@ -525,7 +525,6 @@ static int batch_corrector(pf_batch *b, const std::vector<int> &act) {
     if (!b->h_act) PF_CUDA(cudaMallocHost((void **)&b->h_act, b->n * sizeof(int)));
     for (int i = 0; i < b->n; ++i) b->h_act[i] = 0;
     for (int i : act) b->h_act[i] = 1;
-    const int p = b->pipes[0]->parity;
     const size_t open0 = b->sprof.open.size();
     PF_TRY(staged_corrector(b, b->pipes[0]->parity, &b->launches));
     PF_CUDA(cudaStreamSynchronize(b->master));

@@ -1,12 +1,8 @@
-// Shared-memory mixed-radix Stockham FFT with the transform length known at
-// compile time: the radix sequence (4s, then 2, 3, 5, 7) and all index
-// arithmetic are constants, and each butterfly lives in registers.
+// Row transforms with the length known at compile time: every radix and all
+// index arithmetic are constants, and each butterfly lives in registers.
 //
-// B batches of length L sit contiguously (batch stride L) in `src`; `dst` is
-// the ping-pong buffer; tw[t] = exp(+2 pi i t / L).  SIGN=+1 is FFTW's
-// unnormalised backward transform, SIGN=-1 the forward one.  The Stockham
-// pass with radix R maps butterfly j (k = j mod Ns) to outputs
-// (j/Ns)*Ns*R + k + q*Ns after twiddling input q by W^(SIGN q k L/(Ns R)).
+// tw[t] = exp(+2 pi i t / L).  SIGN=+1 is FFTW's unnormalised backward
+// transform, SIGN=-1 the forward one.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -113,15 +109,6 @@ template <int SIGN, typename C> __device__ __forceinline__ C c_root(C a, int e, 
 __host__ __device__ constexpr int fft_first_radix(int L) {
     return L % 4 == 0 ? 4 : L % 2 == 0 ? 2 : L % 3 == 0 ? 3 : L % 5 == 0 ? 5 : L % 7 == 0 ? 7 : L;
 }
-__host__ __device__ constexpr bool fft_supported(int L) {
-    while (L > 1) {
-        const int r = fft_first_radix(L);
-        if (r > 7) return false;
-        L /= r;
-    }
-    return true;
-}
-
 template <int R, int SIGN, typename C>
 __device__ __forceinline__ void fft_dft(C (&v)[R]) {
     if constexpr (R == 2) {
@@ -156,48 +143,6 @@ __device__ __forceinline__ void fft_dft(C (&v)[R]) {
 #pragma unroll
         for (int q = 0; q < R; ++q) v[q] = o[q];
     }
-}
-
-template <int L, int R, int NS, int SIGN, typename C>
-__device__ __forceinline__ void fft_pass(const C *__restrict__ src, C *__restrict__ dst, int B, const C *tw) {
-    constexpr int NB = L / R;
-    constexpr int STRIDE = L / (NS * R);
-    for (int idx = threadIdx.x; idx < NB * B; idx += blockDim.x) {
-        const int b = idx / NB, j = idx - b * NB;
-        const int k = j % NS;
-        const C *sp = src + b * L;
-        C *dp = dst + b * L;
-        C v[R];
-#pragma unroll
-        for (int q = 0; q < R; ++q) {
-            C x = sp[j + q * NB];
-            if (NS > 1 && q > 0) x = c_mul(x, c_tw<SIGN>(tw[q * k * STRIDE]));
-            v[q] = x;
-        }
-        fft_dft<R, SIGN>(v);
-        const int base = (j / NS) * NS * R + k;
-#pragma unroll
-        for (int q = 0; q < R; ++q) dp[base + q * NS] = v[q];
-    }
-}
-
-// Runs all passes; returns the buffer that holds the result.  Every thread
-// of the block must call it (it synchronises between passes).
-template <int L, int REM, int NS, int SIGN, typename C>
-__device__ __forceinline__ C *fft_run(C *src, C *dst, int B, const C *tw) {
-    if constexpr (REM == 1) {
-        return src;
-    } else {
-        constexpr int R = fft_first_radix(REM);
-        fft_pass<L, R, NS, SIGN>(src, dst, B, tw);
-        __syncthreads();
-        return fft_run<L, REM / R, NS * R, SIGN>(dst, src, B, tw);
-    }
-}
-
-template <int L, int SIGN, typename C>
-__device__ __forceinline__ C *smem_fft_t(C *buf, C *tmp, int B, const C *tw) {
-    return fft_run<L, L, 1, SIGN>(buf, tmp, B, tw);
 }
 
 // ---------------------------------------------------------------------------
@@ -349,10 +294,13 @@ __device__ __forceinline__ void fft4_tables(C *tw, C *tw2, const C *__restrict__
 }
 
 // ---------------------------------------------------------------------------
-// Stockham passes of radix 8 or 6 where the length allows (else as above),
-// each butterfly an in-register codelet (rfft_run): a length-384 row takes
+// Stockham passes of radix 8 or 6 where the length allows (else 4, 2, 3, 5,
+// 7), each butterfly an in-register codelet (rfft_run): a length-384 row takes
 // three passes (8, 8, 6) instead of five (4, 4, 4, 2, 3), so three barriers
-// and shared-memory round trips instead of five.
+// and shared-memory round trips instead of five.  B rows of length L sit
+// contiguously in `src`, `dst` is the ping-pong buffer; the pass with radix R
+// maps butterfly j (k = j mod NS) to outputs (j/NS)*NS*R + k + q*NS after
+// twiddling input q by W^(SIGN q k L/(NS R)).
 __host__ __device__ constexpr int fft_big_radix(int L) {
     return L % 8 == 0 ? 8 : L % 6 == 0 ? 6 : fft_first_radix(L);
 }

@@ -27,6 +27,9 @@
 #define NBAND (2 * PF_KL + 1)   // rows of a mesh band
 #define NLU (3 * PF_KL + 1)     // rows of a lumesh band (LDAB)
 
+constexpr int STEP_MAX_N = 128; // radial points up to which a pipe takes the one-launch step
+constexpr int B200_SMS = 148;   // what the grids of grid-stride and host-only launches are sized for
+
 // ------------------------------------------------------------------ errors
 void pf_set_error(const char *fmt, ...);
 #define PF_CUDA(call)                                                        \

@@ -182,7 +182,7 @@ static int na_zinv(const double *re, const double *im, double2 *T, const double2
     // threads a row keeps busy; enough columns for a block, and blocks for the GPU
     const int per = FR::four ? FR::L2 : L / 8, nb = (N + NA_NR - 1) / NA_NR;
     int MC = std::min(M, std::max(1, 256 / (per * NA_NR)));
-    while (MC > 1 && (M + MC - 1) / MC * nb < 2 * 148) MC = (MC + 1) / 2;
+    while (MC > 1 && (M + MC - 1) / MC * nb < 2 * B200_SMS) MC = (MC + 1) / 2;
     const int threads = std::min(256, (MC * NA_NR * per + 31) / 32 * 32);
     const size_t sm = FR::smem_elems(MC * NA_NR) * sizeof(double2);
     PF_TRY(pf_raise_smem((const void *)k_na_zinv<L>, sm));

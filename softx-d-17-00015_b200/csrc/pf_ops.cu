@@ -45,7 +45,7 @@ int pf_launch_ew(pf_ctx *ctx, EwOp op, const double2 *a, const double2 *b, doubl
                  double2 *o2, double s) {
     const Geo &g = ctx->g;
     const long long total = (long long)g.N * g.Hp;
-    const unsigned grid = (unsigned)std::min<long long>(grid1(total, BLK), 148LL * 16);
+    const unsigned grid = (unsigned)std::min<long long>(grid1(total, BLK), 16LL * B200_SMS);
     {
         ProfScope ps_(ctx, PF_K_EW);
         k_ew<<<grid, BLK, 0, ctx->stream>>>((int)op, a, b, o1, o2, s, g.N, g.H, g.Hp);
@@ -406,7 +406,7 @@ int pf_launch_measurecorr(pf_ctx *ctx, const double2 *a0, const double2 *b0, con
     const Geo &g = ctx->g;
     unsigned long long *out = &ctx->dsc->dterr2_bits;
     if (reset) PF_CUDA(cudaMemsetAsync(out, 0, sizeof(unsigned long long), ctx->stream));
-    const unsigned grid = (unsigned)std::min<long long>(grid1((long long)g.N * g.Hp, BLK), 148LL * 8);
+    const unsigned grid = (unsigned)std::min<long long>(grid1((long long)g.N * g.Hp, BLK), 8LL * B200_SMS);
     {
         ProfScope ps_(ctx, PF_K_EW);
         k_measurecorr<<<grid, BLK, 0, ctx->stream>>>(a0, b0, a1, b1, a2, b2, out, g.N, g.H, g.Hp);

@@ -68,7 +68,7 @@ unsigned long long bytes_estimate(const pf_config &c) {
     g.K = c.K;
     g.M = c.M;
     b += 4 * (NLU * N * Hp * 8 + N * Hp);      // four factor sets, pivots
-    if (c.N <= 128) b += 4 * pf_tile_elems(g) * 8;  // their tiles (fused-step sizes)
+    if (c.N <= STEP_MAX_N) b += 4 * pf_tile_elems(g) * 8;  // their tiles (fused-step sizes)
     b += 6 * N * Hp * 8 + 16 * Hp * 8;         // influence vectors and 4x4 inverses
     b += 64 * N * 8 + 4 * (Z + Th) * 16;       // mesh, twiddles, small buffers
     return b;

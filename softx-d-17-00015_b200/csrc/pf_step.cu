@@ -328,7 +328,7 @@ static constexpr int STEP_HEAD = 3584;
 static_assert(sizeof(StepHead) <= STEP_HEAD, "block header");
 struct StepSmem {
     int ppe, ld, apart;
-    int far;  // the launch works on more than L2 holds
+    int far;  // the launch's own tiles work on more than L2 holds (a batch's other groups, beside it, not counted)
 };
 
 // 16 slots by NT/16 row groups; W = 16: a tile of m = 0.  Products that feed
@@ -743,8 +743,6 @@ __global__ void __launch_bounds__(NT, MINB) k_step_batch(const StepArgs *__restr
 }
 
 // ------------------------------------------------------------------ host
-static constexpr int STEP_MAX_N = 128;
-
 // (N limit, threads, resident blocks): shared memory, 1.2 KB a radial point
 // plus the rings, allows that many blocks
 #define PF_STEP_SHAPES(X) X(32, 192, 4) X(64, 256, 2) X(128, 256, 1)

@@ -337,7 +337,7 @@ static int nonnewtonian(pf_ctx *ctx) {
         PF_CUDA(cudaMemsetAsync(mm, 0, 2 * sizeof(unsigned long long), ctx->stream));
         {
             ProfScope ps_(ctx, PF_K_EW);
-            k_minmax<<<148, 256, 0, ctx->stream>>>(nu, np, mm, mm + 1);
+            k_minmax<<<B200_SMS, 256, 0, ctx->stream>>>(nu, np, mm, mm + 1);
         }
         PF_LAUNCHED(ctx);
         PF_CUDA(cudaMemcpyAsync(ctx->util_diag_d, mm, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToDevice,
@@ -436,7 +436,7 @@ static int les(pf_ctx *ctx) {
     PF_CUDA(cudaMemsetAsync(mm, 0, 2 * sizeof(unsigned long long), ctx->stream));
     {
         ProfScope ps_(ctx, PF_K_EW);
-        k_minmax<<<148, 256, 0, ctx->stream>>>(nu, np, mm, mm + 1);
+        k_minmax<<<B200_SMS, 256, 0, ctx->stream>>>(nu, np, mm, mm + 1);
     }
     PF_LAUNCHED(ctx);
     PF_CUDA(cudaMemcpyAsync(ctx->util_diag_d, mm, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToDevice,
