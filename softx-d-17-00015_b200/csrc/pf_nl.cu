@@ -760,7 +760,7 @@ static int launch_nl(pf_ctx *ctx, const NLArgs &a) {
     return PF_OK;
 }
 
-template <bool MIXED> __global__ void k_nl_prep(NLArgs a, int rows, int sym);
+template <bool MIXED, bool RUN> __global__ void k_nl_prep(NLArgs a, int rows, int sym);
 __global__ void k_nl_mean64_fin(NLArgs a, int stepped);
 static int prep_attrs();
 static size_t prep_smem(int rows);
@@ -785,8 +785,9 @@ int pf_launch_nl_fused(pf_ctx *ctx, int mode) {
             const int chunks = (ctx->g.H + 31) / 32, rows = prep_rows(N, chunks, ctx->sms), sym = mode == PF_NL_SYM;
             const dim3 grid(chunks, (N + rows - 1) / rows);
             const size_t sm = prep_smem(std::min(N, rows + 2 * KL));
-            if (mixed) k_nl_prep<true><<<grid, PREP_THREADS, sm, ctx->stream>>>(a, rows, sym);
-            else k_nl_prep<false><<<grid, PREP_THREADS, sm, ctx->stream>>>(a, rows, sym);
+            const auto k = mixed ? (rows < N ? k_nl_prep<true, true> : k_nl_prep<true, false>)
+                                 : (rows < N ? k_nl_prep<false, true> : k_nl_prep<false, false>);
+            k<<<grid, PREP_THREADS, sm, ctx->stream>>>(a, rows, sym);
         }
         PF_LAUNCHED(ctx);
     }
@@ -814,7 +815,10 @@ int pf_launch_nl_fused(pf_ctx *ctx, int mode) {
 // (the c2r transform ignores Im f00): the chunk's sums go out as partials
 // here, and one warp per radial point adds the chunks' partials in a fixed
 // order afterwards.
-template <bool MIXED>
+// RUN: a block takes a run of the radial points and waits for their weights once.
+// One for all has warps enough to hide them, and stores whole values (64 mixed
+// pipes: 131 us; in the form of the runs 143).
+template <bool MIXED, bool RUN>
 __device__ __forceinline__ void nl_prep_body(const NLArgs &a, int chunk, int n0, int n1, int sym) {
     extern __shared__ double2 msm[];  // [2][j1 - j0][32]: u_t, u_z of this chunk's modes at the rows read
     const Geo &g = a.g;
@@ -830,7 +834,11 @@ __device__ __forceinline__ void nl_prep_body(const NLArgs &a, int chunk, int n0,
         double2 t = live ? a.u[1][at] : make_double2(0.0, 0.0), z = live ? a.u[2][at] : make_double2(0.0, 0.0);
         if (mean) {  // var_imposesym of the mean mode (variables.f90:611-616)
             t.y = z.y = 0.0;
-            if (n >= n0 && n < n1) {  // what the blocks beside this one read of these rows stays as it is
+            if (!RUN) {
+                const_cast<double2 *>(a.u[0])[at] = make_double2(0.0, 0.0);
+                const_cast<double2 *>(a.u[1])[at] = t;
+                const_cast<double2 *>(a.u[2])[at] = z;
+            } else if (n >= n0 && n < n1) {  // what the blocks beside this one read of these rows stays as it is
                 const_cast<double2 *>(a.u[0])[at] = make_double2(0.0, 0.0);
                 const_cast<double2 *>(a.u[1])[at].y = 0.0;
                 const_cast<double2 *>(a.u[2])[at].y = 0.0;
@@ -851,19 +859,24 @@ __device__ __forceinline__ void nl_prep_body(const NLArgs &a, int chunk, int n0,
             const double2 ur = mean ? make_double2(0.0, 0.0) : a.u[0][at];
             const double2 ut = st[(n - j0) * 32 + lane], uz = sz[(n - j0) * 32 + lane];
             const double rm1 = a.dm.rp[2 * N + n];
-            double w[NBAND];  // read together, then the sums
-#pragma unroll
-            for (int i = 0; i < NBAND; ++i) w[i] = drb[(NBAND - 1 - i) * N + min(max(n - KL + i, 0), N - 1)];
             double2 dz = make_double2(0.0, 0.0), dt = dz;
-#pragma unroll
-            for (int i = 0; i < NBAND; ++i) {  // d/dr of u_z and u_t (var_coll_meshmult)
-                const int j = n - KL + i;
-                if (j < 0 || j >= N) continue;
+            auto term = [&](double w, int j) {  // d/dr of u_z and u_t (var_coll_meshmult)
                 const double2 z = sz[(j - j0) * 32 + lane], t = st[(j - j0) * 32 + lane];
-                dz.x = fma(w[i], z.x, dz.x);
-                dz.y = fma(w[i], z.y, dz.y);
-                dt.x = fma(w[i], t.x, dt.x);
-                dt.y = fma(w[i], t.y, dt.y);
+                dz.x = fma(w, z.x, dz.x);
+                dz.y = fma(w, z.y, dz.y);
+                dt.x = fma(w, t.x, dt.x);
+                dt.y = fma(w, t.y, dt.y);
+            };
+            if (RUN) {  // the weights read together, then the sums
+                double w[NBAND];
+#pragma unroll
+                for (int i = 0; i < NBAND; ++i) w[i] = drb[(NBAND - 1 - i) * N + min(max(n - KL + i, 0), N - 1)];
+#pragma unroll
+                for (int i = 0; i < NBAND; ++i)
+                    if (n - KL + i >= 0 && n - KL + i < N) term(w[i], n - KL + i);
+            } else {
+                const int hi = min(N - 1, n + KL);
+                for (int j = max(0, n - KL); j <= hi; ++j) term(drb[(KL + n - j) * N + j], j);
             }
             const Curl c = mode_curl(ur, ut, uz, dt, dz, rm1, rm1 * g.Mp * m, k1a1);
             if (MIXED) {
@@ -929,9 +942,10 @@ static int prep_rows(int N, int chunks, int sms) {
     const int runs = std::min((N + 7) / 8, std::max(1, 2 * sms / chunks));
     return runs == 1 ? N : ((N + runs - 1) / runs + 7) / 8 * 8;
 }
-template <bool MIXED> __global__ void __launch_bounds__(PREP_THREADS) k_nl_prep(NLArgs a, int rows, int sym) {
+template <bool MIXED, bool RUN>
+__global__ void __launch_bounds__(PREP_THREADS) k_nl_prep(NLArgs a, int rows, int sym) {
     chain_open();
-    nl_prep_body<MIXED>(a, blockIdx.x, blockIdx.y * rows, min(a.g.N, (blockIdx.y + 1) * rows), sym);
+    nl_prep_body<MIXED, RUN>(a, blockIdx.x, blockIdx.y * rows, min(a.g.N, (blockIdx.y + 1) * rows), sym);
 }
 // one warp per radial point
 __global__ void __launch_bounds__(128) k_nl_mean64_fin(NLArgs a, int stepped) {
@@ -992,8 +1006,8 @@ __global__ void __launch_bounds__(PREP_THREADS) k_nl_prep_batch(const NLArgs *__
     const int2 pb = blk[blockIdx.x];
     if (act && !act[pb.x]) return;
     const NLArgs a = args[pb.x];
-    if ((int)blockIdx.x < nfp64) nl_prep_body<false>(a, pb.y, 0, a.g.N, sym);
-    else nl_prep_body<true>(a, pb.y, 0, a.g.N, sym);
+    if ((int)blockIdx.x < nfp64) nl_prep_body<false, false>(a, pb.y, 0, a.g.N, sym);
+    else nl_prep_body<true, false>(a, pb.y, 0, a.g.N, sym);
 }
 __global__ void __launch_bounds__(128) k_nl_mean64_fin_batch(const NLArgs *__restrict__ args,
                                                             const int2 *__restrict__ blk, int stepped,
@@ -1086,8 +1100,8 @@ __global__ void __launch_bounds__(NL_THREADS, ST == 1 ? 6 : 5)
 
 // shared-memory limit of the prep kernels
 static int prep_attrs() {
-    PF_TRY(pf_raise_smem((const void *)k_nl_prep<true>, prep_smem(PREP_MAX_N)));
-    PF_TRY(pf_raise_smem((const void *)k_nl_prep<false>, prep_smem(PREP_MAX_N)));
+    for (const auto k : {k_nl_prep<true, true>, k_nl_prep<true, false>, k_nl_prep<false, true>, k_nl_prep<false, false>})
+        PF_TRY(pf_raise_smem((const void *)k, prep_smem(PREP_MAX_N)));
     return pf_raise_smem((const void *)k_nl_prep_batch, prep_smem(PREP_MAX_N));
 }
 
